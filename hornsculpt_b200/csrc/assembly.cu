@@ -15,6 +15,7 @@
 #include "autotune.hpp"
 #include "device_once.hpp"
 #include "device_types.cuh"
+#include "green_math.cuh"
 #include "host_mesh.hpp"
 #include "kernel_timer.hpp"
 
@@ -33,6 +34,7 @@ constexpr size_t kGatherColumnSmem = 200 * 1024;  // fused column gather: 3T com
 // (offsets 0, 6, 18, 34).
 constexpr int kRulePoints = 98;
 __constant__ double cRule[kRulePoints * 4];
+__constant__ double cRuleSquares[kRulePoints * 3];  // b1^2, b1 b2, b2^2
 __constant__ double cGauss20[40];
 
 template <int NP> __device__ constexpr int ruleOffset() {
@@ -103,147 +105,237 @@ __device__ __forceinline__ void pairRecordValue(int o, const Real *MG, const Rea
     }
 }
 
+// Both records of an unordered pair from its moments M = {MG, MP, MQ} (the
+// formulas of pairRecordValue). ps = plane stride in complex values; whether a
+// value was infinite or NaN is returned.
+__device__ __forceinline__ bool storePairRecords(const double (&M)[54], const DPanel &t, const DPanel &s, double k,
+                                                 double invk, double2 *fwd, double2 *rev, size_t ps) {
+    const double *MG = M, *MP = M + 18, *MQ = M + 36;
+    const double knn = k * (t.n[0] * s.n[0] + t.n[1] * s.n[1] + t.n[2] * s.n[2]);
+    double gre = 0, gim = 0;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        gre += MG[2 * c];
+        gim += MG[2 * c + 1];
+    }
+    gre *= invk;
+    gim *= invk;
+    unsigned largest = 0;  // of the high words: 0x7ff..... only for infinities and NaN
+    const auto value = [&](double re, double im) {
+        largest = max(largest, max(unsigned(__double2hiint(re)) & 0x7fffffffu, unsigned(__double2hiint(im)) & 0x7fffffffu));
+        return make_double2(re, im);
+    };
+    // element (i, j): test vertex i, trial vertex j; X = MP forward, MQ reverse
+    const auto element = [&](int i, int j, const double *X) {
+        const double curl = t.curl[3 * i] * s.curl[3 * j] + t.curl[3 * i + 1] * s.curl[3 * j + 1] +
+                            t.curl[3 * i + 2] * s.curl[3 * j + 2];
+        const int m = 2 * (3 * i + j);
+        return value(fma(gim, curl, fma(-knn, MG[m + 1], -X[m])), fma(-gre, curl, fma(knn, MG[m], -X[m + 1])));
+    };
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        #pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            fwd[j * ps + i] = element(i, j, MP);
+            rev[i * ps + j] = element(i, j, MQ);
+        }
+    }
+    // right-hand side moments of vertex a: sums over the other panel's vertices
+    const auto moment = [&](int a, int own, int other, const double *Y) {
+        double gr = 0, gi = 0, yr = 0, yi = 0;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const int m = own * a + other * b;
+            gr += MG[m];
+            gi += MG[m + 1];
+            yr += Y[m];
+            yi += Y[m + 1];
+        }
+        return value(fma(-yi, invk, -gr), fma(yr, invk, -gi));
+    };
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        fwd[3 * ps + a] = moment(a, 6, 2, MQ);
+        rev[3 * ps + a] = moment(a, 2, 6, MP);
+    }
+    return largest >= 0x7ff00000u;
+}
+
 // ---------------------------------------------------------------------------
-// Regular pairs: one unordered pair per NP threads, thread x owns test point x
-// and sweeps the NP trial points, contracting trial bases on the fly.
+// Regular pairs of the plain form: SPLIT threads per unordered pair, each
+// owning every SPLIT-th test point with all its trial points.
+//
+// Bound: the FP64 pipe (64 fma per SM and clock), so the kernel is built to
+// spend few FP64 instructions per sample and to keep the pipe fed from one
+// thread's own unrolled samples. Per sample it accumulates moments against
+// {1, b1, b2} of the trial barycentrics (b0 = 1 - b1 - b2 is taken once per
+// test point) of g and of u = g (1 + ikr) / r^2, with u's second moments:
+// the double-layer factor (x - y).n_trial is constant over the trial panel
+// and (x - y).n_test affine in b1, b2, so both layers follow from u's moments
+// once per test point. The 27 complex moments of the pair stay in registers
+// and the records are written straight from them, without shared-memory
+// exchanges or barriers between the steps of a pair. 128 threads at two CTAs
+// per SM: 255 registers per thread. Measured (1280 triangles, 32 frequencies):
+// 12 points 12.5 -> 7.25 ms, 6 points 11.0 -> 4.5 ms against one thread per
+// test point with the contraction in shared memory; ncu: FP64 pipe 66 % and
+// 61 % active, the rest fixed latencies that two warps per scheduler do not
+// cover.
+//
+// SPLIT = 1 for the 6- and 12-point rules, whose pairs number in the
+// millions on every mesh. The 16- and 64-point rules serve few pairs on small
+// meshes (256 and 4096 samples each); there 8 and 32 threads share a pair and
+// add their moments by shuffles.
 // ---------------------------------------------------------------------------
-// 128 threads: four CTAs (16 warps) per SM within the 128 registers a thread
-// may use at that occupancy (the register file is split between the four SM
-// sub-partitions, so 192-thread CTAs would stop at two per SM).
 constexpr int kPlainThreads = 128;
 
+template <int NP> __device__ constexpr int plainSplit() { return NP == 64 ? 32 : NP == 16 ? 8 : 1; }
+
 template <int NP>
-__global__ void __launch_bounds__(kPlainThreads, 4) regularPairsKernel(const DPanel *__restrict__ panels, uint32_t T,
+__global__ void __launch_bounds__(kPlainThreads, 2) regularPairsKernel(const DPanel *__restrict__ panels, uint32_t T,
                                                           const double *__restrict__ ks,
                                                           const uint2 *__restrict__ bins,
                                                           const uint32_t *__restrict__ binCounts, size_t binCapacity,
                                                           const uint64_t *__restrict__ binOffsets, int bin,
                                                           double *__restrict__ records, SlotMap map, int *error) {
-    constexpr int PPC = kPlainThreads / NP;  // pairs per CTA; the last NP-group of threads may idle
-    constexpr int RO = ruleOffset<NP>();
-    __shared__ double sS[kPlainThreads][18];
-    __shared__ double sM[PPC][54];
-    // per trial point of each pair: its offset from the trial panel's first
-    // vertex and that offset against the trial and test normals
-    __shared__ double sY[kPlainThreads][5];
+    constexpr int RO = ruleOffset<NP>(), SPLIT = plainSplit<NP>(), UNROLL = NP == 6 ? 6 : 4;
     const int f = blockIdx.y;
     const double k = ks[f], invk = 1.0 / k;
     const uint32_t count = binCounts[f * kBins + bin];
     const uint2 *list = bins + binStart(binOffsets, binCapacity, f, bin);
     double *rec = records + size_t(f) * map.planeSlots * kRecordDoubles;
-    const int l = threadIdx.x / NP, x = threadIdx.x % NP;
-    const double *yRow = &sY[l * NP][0];
+    const uint32_t part = threadIdx.x % SPLIT;
+    DistanceCheck distance;
+    bool nonFinite = false, escaped = false;
+    constexpr uint32_t PPC = kPlainThreads / SPLIT;
     for (uint32_t base = blockIdx.x * PPC; base < count; base += gridDim.x * PPC) {
-        const uint32_t p = base + l;
-        const bool mine = l < PPC && p < count;
-        uint2 pr = make_uint2(0, 0);
-        if (mine) {
-            // thread x places the pair's trial point x
-            pr = list[p];
-            const DPanel &S = panels[pr.y], &A = panels[pr.x];
-            const double b1 = cRule[4 * (RO + x) + 1], b2 = cRule[4 * (RO + x) + 2];
-            double e[3];
+        const uint32_t p = base + threadIdx.x / SPLIT;
+        if (SPLIT == 1 && p >= count)
+            break;
+        // threads that share pairs stay together for the shuffles: a group past the end repeats the last pair
+        const uint2 pr = list[SPLIT == 1 ? p : min(p, count - 1)];
+        const DPanel &A = panels[pr.x], &S = panels[pr.y];
+        const double se1[3] = {S.e1[0], S.e1[1], S.e1[2]}, se2[3] = {S.e2[0], S.e2[1], S.e2[2]};
+        double M[54];
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-                e[c] = S.e1[c] * b1 + S.e2[c] * b2;
-            sY[threadIdx.x][0] = e[0];
-            sY[threadIdx.x][1] = e[1];
-            sY[threadIdx.x][2] = e[2];
-            sY[threadIdx.x][3] = e[0] * S.n[0] + e[1] * S.n[1] + e[2] * S.n[2];
-            sY[threadIdx.x][4] = e[0] * A.n[0] + e[1] * A.n[1] + e[2] * A.n[2];
-        }
-        __syncthreads();
-        if (mine) {
-            const DPanel &A = panels[pr.x];
-            const DPanel &S = panels[pr.y];
+        for (int c = 0; c < 54; ++c)
+            M[c] = 0;
+#pragma unroll 1
+        for (int x = int(part); x < NP; x += SPLIT) {
             const double bx1 = cRule[4 * (RO + x) + 1], bx2 = cRule[4 * (RO + x) + 2];
             // test point x relative to the trial panel's first vertex
             const double P0 = (A.v0[0] - S.v0[0]) + (A.e1[0] * bx1 + A.e2[0] * bx2);
             const double P1 = (A.v0[1] - S.v0[1]) + (A.e1[1] * bx1 + A.e2[1] * bx2);
             const double P2 = (A.v0[2] - S.v0[2]) + (A.e1[2] * bx1 + A.e2[2] * bx2);
-            const double w0 = cRule[4 * (RO + x) + 3] * 4.0 * A.area * S.area * kInvFourPi;
-            // (x - y).n_s = P.n_s - e(y).n_s, (x - y).n_t = P.n_t - e(y).n_t
-            const double psP = P0 * S.n[0] + P1 * S.n[1] + P2 * S.n[2];
-            const double qtP = P0 * A.n[0] + P1 * A.n[1] + P2 * A.n[2];
-            double sp[6] = {0, 0, 0, 0, 0, 0}, sq[6] = {0, 0, 0, 0, 0, 0}, sg[6] = {0, 0, 0, 0, 0, 0};
-            bool bad = false;
-#pragma unroll(NP == 6 ? 6 : 4)
-            for (int y = 0; y < NP; ++y) {
-                const double b0 = cRule[4 * (RO + y)], b1 = cRule[4 * (RO + y) + 1], b2 = cRule[4 * (RO + y) + 2];
-                const double wy = cRule[4 * (RO + y) + 3];
-                const double *Y = yRow + 5 * y;
-                const double dx = P0 - Y[0], dy = P1 - Y[1], dz = P2 - Y[2];
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                bad |= !(r2 > 0) || !isfinite(r2);
-                const double rinv = rsqrt(r2);
-                const double r = r2 * rinv, kr = k * r;
-                double sn, cs;
-                sincos(kr, &sn, &cs);
-                const double sc = w0 * wy * rinv;
-                const double gr = cs * sc, gi = -sn * sc;
-                const double rr = gr - gi * kr, ri = gi + gr * kr;
-                const double rinv2 = rinv * rinv;
-                const double ps = (psP - Y[3]) * rinv2;
-                const double qt = (Y[4] - qtP) * rinv2;
-                const double Pr = rr * ps, Pi = ri * ps, Qr = rr * qt, Qi = ri * qt;
-                const double bb[3] = {b0, b1, b2};
+            double g[6], u[12];  // g against 1, b1, b2; u against 1, b1, b2, b1^2, b1 b2, b2^2
 #pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    sp[2 * j] += Pr * bb[j];
-                    sp[2 * j + 1] += Pi * bb[j];
-                    sq[2 * j] += Qr * bb[j];
-                    sq[2 * j + 1] += Qi * bb[j];
-                    sg[2 * j] += gr * bb[j];
-                    sg[2 * j + 1] += gi * bb[j];
+            for (int c = 0; c < 6; ++c)
+                g[c] = 0;
+#pragma unroll
+            for (int c = 0; c < 12; ++c)
+                u[c] = 0;
+#pragma unroll UNROLL
+            for (int y = 0; y < NP; ++y) {
+                const double b1 = cRule[4 * (RO + y) + 1], b2 = cRule[4 * (RO + y) + 2];
+                const double *bb = cRuleSquares + 3 * (RO + y);
+                const double dx = fma(-b2, se2[0], fma(-b1, se1[0], P0));
+                const double dy = fma(-b2, se2[1], fma(-b1, se1[1], P1));
+                const double dz = fma(-b2, se2[2], fma(-b1, se1[2], P2));
+                const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                distance.add(r2);
+                const double rinv = reciprocalRoot(r2);
+                const double kr = k * (r2 * rinv);
+                double sn, cs;
+                sinCos(kr, sn, cs);
+                const double sc = cRule[4 * (RO + y) + 3] * rinv;
+                const double gr = cs * sc, gi = -sn * sc;
+                const double rinv2 = rinv * rinv;
+                const double ur = fma(-gi, kr, gr) * rinv2, ui = fma(gr, kr, gi) * rinv2;
+                g[0] += gr;
+                g[1] += gi;
+                g[2] = fma(gr, b1, g[2]);
+                g[3] = fma(gi, b1, g[3]);
+                g[4] = fma(gr, b2, g[4]);
+                g[5] = fma(gi, b2, g[5]);
+                u[0] += ur;
+                u[1] += ui;
+                u[2] = fma(ur, b1, u[2]);
+                u[3] = fma(ui, b1, u[3]);
+                u[4] = fma(ur, b2, u[4]);
+                u[5] = fma(ui, b2, u[5]);
+                u[6] = fma(ur, bb[0], u[6]);
+                u[7] = fma(ui, bb[0], u[7]);
+                u[8] = fma(ur, bb[1], u[8]);
+                u[9] = fma(ui, bb[1], u[9]);
+                u[10] = fma(ur, bb[2], u[10]);
+                u[11] = fma(ui, bb[2], u[11]);
+            }
+            const double wx = cRule[4 * (RO + x) + 3];
+            const double row[3] = {wx, wx * bx1, wx * bx2};
+            // (x - y).n_trial: constant over the trial panel; -(x - y).n_test = q0 + t1 b1 + t2 b2
+            const double ps = P0 * S.n[0] + P1 * S.n[1] + P2 * S.n[2];
+            const double q0 = -(P0 * A.n[0] + P1 * A.n[1] + P2 * A.n[2]);
+            const double t1 = se1[0] * A.n[0] + se1[1] * A.n[1] + se1[2] * A.n[2];
+            const double t2 = se2[0] * A.n[0] + se2[1] * A.n[1] + se2[2] * A.n[2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double rp = row[i] * ps;
+#pragma unroll
+                for (int c = 0; c < 6; ++c) {
+                    M[6 * i + c] = fma(row[i], g[c], M[6 * i + c]);
+                    M[18 + 6 * i + c] = fma(rp, u[c], M[18 + 6 * i + c]);
                 }
             }
-            if (bad)
-                flagError(error, kErrDistance);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const double q[3] = {fma(t2, u[4 + c], fma(t1, u[2 + c], q0 * u[c])),
+                                     fma(t2, u[8 + c], fma(t1, u[6 + c], q0 * u[2 + c])),
+                                     fma(t2, u[10 + c], fma(t1, u[8 + c], q0 * u[4 + c]))};
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j)
+                        M[36 + 6 * i + 2 * j + c] = fma(row[i], q[j], M[36 + 6 * i + 2 * j + c]);
+            }
+        }
+        if (SPLIT > 1) {
+#pragma unroll
+            for (int h = SPLIT / 2; h >= 1; h >>= 1)
+#pragma unroll
+                for (int c = 0; c < 54; ++c)
+                    M[c] += __shfl_xor_sync(0xffffffffu, M[c], h);
+            if (part != 0 || p >= count)
+                continue;
+        }
+        // from (1, b1, b2) to (b0, b1, b2) on both sides, and the panels' Jacobians
+        const double w4 = 4.0 * A.area * S.area * kInvFourPi;
+#pragma unroll
+        for (int kind = 0; kind < 3; ++kind) {
+            double *m = M + 18 * kind;
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    m[6 * i + c] -= m[6 * i + 2 + c] + m[6 * i + 4 + c];
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                sS[threadIdx.x][c] = sg[c];
-                sS[threadIdx.x][6 + c] = sp[c];
-                sS[threadIdx.x][12 + c] = sq[c];
+                m[c] = (m[c] - (m[6 + c] + m[12 + c])) * w4;
+                m[6 + c] *= w4;
+                m[12 + c] *= w4;
             }
         }
-        __syncthreads();
-        // Test-side contraction: M[kind][i][j] = sum_x bt_i(x) S_kind,j(x).
-        for (int item = threadIdx.x; item < PPC * 27; item += kPlainThreads) {
-            const int pl = item / 27, e = item % 27, kind = e / 9, i = (e % 9) / 3, j = e % 3;
-            if (base + pl >= count)
-                continue;
-            double re = 0, im = 0;
-            for (int xx = 0; xx < NP; ++xx) {
-                const int th = pl * NP + xx;
-                const double bt = cRule[4 * (RO + xx) + i];
-                re += bt * sS[th][kind * 6 + 2 * j];
-                im += bt * sS[th][kind * 6 + 2 * j + 1];
-            }
-            sM[pl][kind * 18 + 2 * (3 * i + j)] = re;
-            sM[pl][kind * 18 + 2 * (3 * i + j) + 1] = im;
-        }
-        __syncthreads();
-        for (int item = threadIdx.x; item < PPC * 24; item += kPlainThreads) {
-            const int pl = item / 24, o = item % 24;
-            if (base + pl >= count)
-                continue;
-            const uint2 pr = list[base + pl];
-            double re, im;
-            pairRecordValue(o, &sM[pl][0], &sM[pl][18], &sM[pl][36], panels[pr.x], panels[pr.y], k, invk, re, im);
-            const size_t slot = o < 12 ? mapSlot(map, T, pr.x, pr.y) : mapSlot(map, T, pr.y, pr.x);
-            const int e = o < 12 ? o : o - 12;
-            if (!isfinite(re) || !isfinite(im))
-                flagError(error, kErrNonFinite);
-            if (slot == kNoSlot) {
-                flagError(error, kErrEscapedPlan);
-                continue;
-            }
-            double *dst = rec + mapOffset(map.planeSlots, slot, e);
-            dst[0] = re;
-            dst[1] = im;
-        }
-        __syncthreads();
+        const size_t fwd = mapSlot(map, T, pr.x, pr.y), rev = mapSlot(map, T, pr.y, pr.x);
+        if (fwd == kNoSlot || rev == kNoSlot)
+            escaped = true;
+        else
+            nonFinite |= storePairRecords(M, A, S, k, invk, reinterpret_cast<double2 *>(rec) + 3 * fwd,
+                                          reinterpret_cast<double2 *>(rec) + 3 * rev, map.planeSlots * 3);
     }
+    if (distance.bad())
+        flagError(error, kErrDistance);
+    if (nonFinite)
+        flagError(error, kErrNonFinite);
+    if (escaped)
+        flagError(error, kErrEscapedPlan);
 }
 
 // ---------------------------------------------------------------------------
@@ -1620,6 +1712,15 @@ void uploadRuleTablesNow(cudaStream_t stream) {
         }
     }
     cudaCheck(cudaMemcpyToSymbolAsync(cRule, table, sizeof(table), 0, cudaMemcpyHostToDevice, stream), "rule upload");
+    double squares[kRulePoints * 3];
+    for (int i = 0; i < kRulePoints; ++i) {
+        const double b1 = table[4 * i + 1], b2 = table[4 * i + 2];
+        squares[3 * i] = b1 * b1;
+        squares[3 * i + 1] = b1 * b2;
+        squares[3 * i + 2] = b2 * b2;
+    }
+    cudaCheck(cudaMemcpyToSymbolAsync(cRuleSquares, squares, sizeof(squares), 0, cudaMemcpyHostToDevice, stream),
+              "rule upload");
     static float tableF[kRulePoints * 8];
     for (int i = 0; i < kRulePoints; ++i) {
         const double b1 = table[4 * i + 1], b2 = table[4 * i + 2];
