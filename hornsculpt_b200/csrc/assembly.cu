@@ -399,12 +399,65 @@ __device__ __forceinline__ void mixedValues(double dx, double dy, double dz, flo
 // Rule table per point: b0, b1, b2, w, b1^2, 2 b1 b2, b2^2, 0.
 __constant__ float cRuleF[kRulePoints * 8];
 
+// Record stores of a warp's 32 unordered pairs, one plane and direction at a
+// time. A record plane entry is three complex values (48 B in FP64, 24 B in
+// FP32), so a lane writing its own pair's values would touch 32 different
+// sectors with every store and each sector two to four times. Here the lanes
+// put their values in shared memory and write them out in memory order: the
+// classification lists pairs in tiles of 8 test x 4 trial panels, so runs of 8
+// (forward) and 4 (reverse) entries are contiguous and most sectors are
+// written whole, once. On meshes whose record planes stay near the caches the
+// second-level cache merges the partial sectors and the detour costs more than
+// it saves, so DirectStore is the other form (launchRegular chooses).
+template <class V> struct PlaneStore {
+    V *stage;     // 96 entries of the warp
+    V *dst[3];    // this lane's targets in plane 0 (null: no record)
+    int src[3];   // and their places in `stage`
+    // base: this lane's entry in plane 0, null without a pair; reverse: the order of the reverse slots
+    __device__ __forceinline__ PlaneStore(V *warpStage, V *base, bool reverse) : stage(warpStage) {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int q = lane + 32 * c, t = q / 3, row = q % 3;
+            const int pair = reverse ? (t & 3) * 8 + (t >> 2) : t;
+            V *p = reinterpret_cast<V *>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(base), pair));
+            dst[c] = p ? p + row : nullptr;
+            src[c] = 3 * pair + row;
+        }
+    }
+    __device__ __forceinline__ void put(size_t offset, V v0, V v1, V v2) const {
+        const int lane = threadIdx.x & 31;
+        __syncwarp();  // the previous plane has been read
+        stage[3 * lane] = v0;
+        stage[3 * lane + 1] = v1;
+        stage[3 * lane + 2] = v2;
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            if (dst[c])
+                dst[c][offset] = stage[src[c]];
+    }
+};
+
+// The same interface for a lane that writes its own pair's entries.
+template <class V> struct DirectStore {
+    V *base;
+    __device__ __forceinline__ DirectStore(V *, V *entry, bool) : base(entry) {}
+    __device__ __forceinline__ void put(size_t offset, V v0, V v1, V v2) const {
+        base[offset] = v0;
+        base[offset + 1] = v1;
+        base[offset + 2] = v2;
+    }
+};
+
 // Both records of an unordered regular pair (forward: test A, trial S;
 // reverse: test S, trial A) from its FP32 moments (the layout and formulas of
-// pairRecordValue), stored straight into the record planes. ps = plane stride.
-__device__ __forceinline__ void storePairRecords(const float (&M)[54], const MixedPanel *__restrict__ pa,
-                                                 const MixedPanel *__restrict__ pb, float k, float invk, float *fwd,
-                                                 float *rev, size_t ps, bool &nonFinite) {
+// pairRecordValue). ps = plane stride in complex values; whether a value was
+// infinite or NaN is returned.
+template <class Store>
+__device__ __forceinline__ bool storePairRecords(const float (&M)[54], const MixedPanel *__restrict__ pa,
+                                                 const MixedPanel *__restrict__ pb, float k, float invk,
+                                                 const Store &fwd, const Store &rev, size_t ps) {
     const float *MG = M, *MP = M + 18, *MQ = M + 36;
     const float4 na = pa->n, nb = pb->n;
     const float knn = k * (na.x * nb.x + na.y * nb.y + na.z * nb.z);
@@ -418,47 +471,40 @@ __device__ __forceinline__ void storePairRecords(const float (&M)[54], const Mix
     gim *= invk;
     const float4 ca[3] = {pa->curl[0], pa->curl[1], pa->curl[2]}, cs[3] = {pb->curl[0], pb->curl[1], pb->curl[2]};
     float check = 0.f;
+    const auto value = [&](float re, float im) {
+        check += fabsf(re) + fabsf(im);
+        return make_float2(re, im);
+    };
+    // element (i, j): A's local vertex i, S's local vertex j; X = MP forward, MQ reverse
+    const auto element = [&](int i, int j, const float *X) {
+        const float curl = ca[i].x * cs[j].x + ca[i].y * cs[j].y + ca[i].z * cs[j].z;
+        const int m = 2 * (3 * i + j);
+        return value(fmaf(gim, curl, fmaf(-knn, MG[m + 1], -X[m])), fmaf(-gre, curl, fmaf(knn, MG[m], -X[m + 1])));
+    };
 #pragma unroll
-    for (int i = 0; i < 3; ++i)      // A's local vertex
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {  // S's local vertex
-            const float curl = ca[i].x * cs[j].x + ca[i].y * cs[j].y + ca[i].z * cs[j].z;
-            const int m = 2 * (3 * i + j);
-            // forward element (row i, col j); reverse element (row j, col i)
-            const float fr = fmaf(gim, curl, fmaf(-knn, MG[m + 1], -MP[m]));
-            const float fi = fmaf(-gre, curl, fmaf(knn, MG[m], -MP[m + 1]));
-            const float rr = fmaf(gim, curl, fmaf(-knn, MG[m + 1], -MQ[m]));
-            const float ri = fmaf(-gre, curl, fmaf(knn, MG[m], -MQ[m + 1]));
-            *reinterpret_cast<float2 *>(fwd + j * ps + 2 * i) = make_float2(fr, fi);
-            *reinterpret_cast<float2 *>(rev + i * ps + 2 * j) = make_float2(rr, ri);
-            check += fabsf(fr) + fabsf(fi) + fabsf(rr) + fabsf(ri);
-        }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        // forward rhs row a (A's vertex): sum over S's vertices; reverse rhs row a (S's vertex): over A's
-        float fgr = 0.f, fgi = 0.f, fyr = 0.f, fyi = 0.f, rgr = 0.f, rgi = 0.f, ryr = 0.f, ryi = 0.f;
+    for (int j = 0; j < 3; ++j) {
+        fwd.put(j * ps, element(0, j, MP), element(1, j, MP), element(2, j, MP));
+        rev.put(j * ps, element(j, 0, MQ), element(j, 1, MQ), element(j, 2, MQ));
+    }
+    // right-hand side moments of vertex a: sums over the other panel's vertices
+    const auto moment = [&](int a, int own, int other, const float *Y) {
+        float gr = 0.f, gi = 0.f, yr = 0.f, yi = 0.f;
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
-            const int mf = 2 * (3 * a + b), mr = 2 * (3 * b + a);
-            fgr += MG[mf];
-            fgi += MG[mf + 1];
-            fyr += MQ[mf];
-            fyi += MQ[mf + 1];
-            rgr += MG[mr];
-            rgi += MG[mr + 1];
-            ryr += MP[mr];
-            ryi += MP[mr + 1];
+            const int m = own * a + other * b;
+            gr += MG[m];
+            gi += MG[m + 1];
+            yr += Y[m];
+            yi += Y[m + 1];
         }
-        const float2 fv = make_float2(fmaf(-fyi, invk, -fgr), fmaf(fyr, invk, -fgi));
-        const float2 rv = make_float2(fmaf(-ryi, invk, -rgr), fmaf(ryr, invk, -rgi));
-        *reinterpret_cast<float2 *>(fwd + 3 * ps + 2 * a) = fv;
-        *reinterpret_cast<float2 *>(rev + 3 * ps + 2 * a) = rv;
-        check += fabsf(fv.x) + fabsf(fv.y) + fabsf(rv.x) + fabsf(rv.y);
-    }
-    nonFinite |= !isfinite(check);
+        return value(fmaf(-yi, invk, -gr), fmaf(yr, invk, -gi));
+    };
+    fwd.put(3 * ps, moment(0, 6, 2, MQ), moment(1, 6, 2, MQ), moment(2, 6, 2, MQ));
+    rev.put(3 * ps, moment(0, 2, 6, MP), moment(1, 2, 6, MP), moment(2, 2, 6, MP));
+    return !isfinite(check);
 }
 
-template <int NP>
+template <int NP, bool Staged>
 __global__ void __launch_bounds__(128, 4) regularMixedKernel(const MixedPanel *__restrict__ mpanels,
                                                              const Bounds *__restrict__ bounds, uint32_t T,
                                                              const double *__restrict__ ks,
@@ -476,11 +522,15 @@ __global__ void __launch_bounds__(128, 4) regularMixedKernel(const MixedPanel *_
     const float kf = float(k), invkf = float(1.0 / k);
     const uint32_t count = binCounts[f * kBins + bin];
     const uint2 *list = bins + binStart(binOffsets, binCapacity, f, bin);
-    float *rec = records + size_t(f) * T * T * kRecordDoubles;
-    const size_t planeStride = size_t(T) * T * 6;
+    float2 *rec = reinterpret_cast<float2 *>(records + size_t(f) * T * T * kRecordDoubles);
+    __shared__ float2 stage[4][Staged ? 96 : 1];
+    float2 *const warpStage = stage[threadIdx.x / 32];
+    using Store = std::conditional_t<Staged, PlaneStore<float2>, DirectStore<float2>>;
     bool bad = false, nonFinite = false;
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
-        const uint2 pr = list[p];
+    // staged: a warp takes 32 consecutive pairs, and lanes past the end repeat the last pair and store nothing
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; Staged ? (p & ~31u) < count : p < count;
+         p += gridDim.x * blockDim.x) {
+        const uint2 pr = list[Staged ? min(p, count - 1) : p];
         const MixedPanel &A = mpanels[pr.x], &S = mpanels[pr.y];
         const V3 ca = bounds[pr.x].center, cb = bounds[pr.y].center;
         // centre displacement, distance and phase (reduced to [-pi, pi]) in FP64
@@ -575,8 +625,11 @@ __global__ void __launch_bounds__(128, 4) regularMixedKernel(const MixedPanel *_
             }
         }
         bad |= !(r2min > 0.f);
-        storePairRecords(M, &A, &S, kf, invkf, rec + (size_t(pr.y) * T + pr.x) * 6,
-                         rec + (size_t(pr.x) * T + pr.y) * 6, planeStride, nonFinite);
+        nonFinite |= storePairRecords(
+            M, &A, &S, kf, invkf,
+            Store(warpStage, !Staged || p < count ? rec + (size_t(pr.y) * T + pr.x) * 3 : nullptr, false),
+            Store(warpStage, !Staged || p < count ? rec + (size_t(pr.x) * T + pr.y) * 3 : nullptr, true),
+            size_t(T) * T * 3);
     }
     if (bad)
         flagError(error, kErrDistance);
@@ -1631,9 +1684,12 @@ void launchRegular(const AssemblyGeometry &g, const double *ks, uint32_t B, cons
     const auto launch = [&](int c) {
         if (mixed) {
             const dim3 grid(unsigned(smCount() * kMixedCtas[c]), B);
-            regularMixedKernel<NP><<<grid, 128, 0, stream>>>(g.mixedPanels, g.bounds, g.T, ks, ws.bins, ws.binCounts,
-                                                             ws.binCapacity, ws.binOffsets, bin,
-                                                             static_cast<float *>(ws.records), error);
+            // The 6-point rule writes the most for its samples. Staged stores from 4096 triangles on: 8042
+            // triangles 13.5 -> 10.6 ms, 12 756 triangles 12.1 -> 10.6 ms; equal at 3604, slower at 1280
+            // (1.89 against 2.14 ms), and slower for the 12-point rule at every size (3.04 against 3.30 ms).
+            const auto kernel = NP == 6 && g.T >= 4096 ? regularMixedKernel<NP, NP == 6> : regularMixedKernel<NP, false>;
+            kernel<<<grid, 128, 0, stream>>>(g.mixedPanels, g.bounds, g.T, ks, ws.bins, ws.binCounts, ws.binCapacity,
+                                             ws.binOffsets, bin, static_cast<float *>(ws.records), error);
         } else {
             const dim3 grid(unsigned(smCount() * kPlainCtas[c]), B);
             regularPairsKernel<NP><<<grid, kPlainThreads, 0, stream>>>(g.panels, g.T, ks, ws.bins, ws.binCounts,
