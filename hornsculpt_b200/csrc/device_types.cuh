@@ -145,6 +145,12 @@ void uploadRuleTables(cudaStream_t stream);
 // coefficients a1 a2 b1 b2, weight, pad), then per radial node (r, r^3 w, 1/r, 1 - r).
 std::vector<float> buildSingularTable(unsigned order);
 
+// Touching-pair tuples of the plain form, FP64, in the same order: per tuple
+// twelve doubles (radial slopes of the test and trial bases, displacement
+// coefficients a1 a2 b1 b2, weight, pad), then six per radial node (r, r w,
+// r^2 w, r^3 w, r^4 w, pad).
+std::vector<double> buildSingularTuples(unsigned order);
+
 // Per-batch assembly of B frequencies. ks[B]; flux q[B][E][T] complex;
 // outputs A[B][N*N] (column-major) and rhs[B][E][N] complex. Workspace:
 // records [B][T*T][24], gathered columns C[B][N][3T] complex, per-panel rhs
@@ -170,7 +176,7 @@ size_t recordBytes(uint32_t T, bool mixed);
 bool gatherUsesColumns(uint32_t T);
 // mixed: FP32 samples and records (phases kept exact: centre phase in FP64 for
 // regular pairs, FP64 displacement and phase for near pairs), FP64 matrix.
-void assembleBatch(const AssemblyGeometry &geo, const double *ks, const double *gaussSingular, const double *flux,
+void assembleBatch(const AssemblyGeometry &geo, const double *ks, const double *singularTuples, const double *flux,
                    uint32_t E, uint32_t B, const AssemblyWorkspace &ws, double *A, double *rhs, int *error,
                    cudaStream_t stream, class KernelTimer *timer, bool mixed = false);
 
@@ -188,7 +194,7 @@ struct NearFieldLayout {
     const uint32_t *nearRow, *nearCol;
 };
 size_t nearFieldWorkspaceBytes(size_t pairSlots, uint64_t pairCount);
-void assembleNearField(const AssemblyGeometry &g, const double *k, const double *gaussSingular, const double *flux,
+void assembleNearField(const AssemblyGeometry &g, const double *k, const double *singularTuples, const double *flux,
                        uint32_t E, const NearFieldLayout &nf, void *workspace, double *vals, double *rhsNear,
                        int *error, cudaStream_t stream, class KernelTimer *timer);
 

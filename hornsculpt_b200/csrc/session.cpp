@@ -294,12 +294,6 @@ void Session::preparePlan(const hs_numerics &o, double maxK, const volatile int3
         }
         d.pad[0] = d.pad[1] = 0;
     }
-    const auto gauss = gaussLegendre01(o.singular_order);
-    std::vector<double> g(2 * gauss.size());
-    for (size_t i = 0; i < gauss.size(); ++i) {
-        g[2 * i] = gauss[i].x;
-        g[2 * i + 1] = gauss[i].w;
-    }
     const cudaStream_t s = stream();
     upload(dPairCode_, code, s);
     upload(dTouching_, touching, s);
@@ -332,7 +326,8 @@ void Session::preparePlan(const hs_numerics &o, double maxK, const volatile int3
             patches_ = dPatches_.as<Patch>();
         }
     }
-    upload(dGauss_, g, s);
+    const std::vector<double> tuples = buildSingularTuples(o.singular_order);
+    upload(dSingularTuples_, tuples, s);
     upload(dSingularTable_, buildSingularTable(o.singular_order), s);
     cuda(cudaStreamSynchronize(s), "CUDA synchronization");
     singularSamples_ = 0;
@@ -384,7 +379,7 @@ size_t fmmSolveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t re
 size_t Session::residentBytes() const {
     size_t bytes = 0;
     for (const DeviceBuffer *b : {&dPanels_, &dBounds_, &dMixedPanels_, &dIncOffsets_, &dIncPanel_, &dIncLocal_,
-                                  &dRowScale_, &dMass_, &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dGauss_,
+                                  &dRowScale_, &dMass_, &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dSingularTuples_,
                                   &dSingularTable_, &dRecords_, &dColumns_, &dPanelRhs_, &dBins_, &dBinCounts_, &dBinOffsets_, &dA_,
                                   &dLU_, &dRhs_, &dX_, &dCorr_, &dNorms_, &dPivots_, &dKs_, &dFlux_, &dObservers_,
                                   &dPartials_, &dField_, &dDegrees_, &dWork32_, &dGmres_, &dLuPack_, &dSolveScratch_})
@@ -447,7 +442,7 @@ void Session::ensureWorkspace(uint32_t B, uint32_t E, uint32_t O, bool mixed, ui
     dWork32_.ensure(B * E * N * 8);
     size_t bytes = 0;
     for (const DeviceBuffer *b : {&dPanels_, &dBounds_, &dMixedPanels_, &dIncOffsets_, &dIncPanel_, &dIncLocal_, &dRowScale_, &dMass_,
-                                  &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dGauss_, &dSingularTable_, &dRecords_, &dColumns_,
+                                  &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dSingularTuples_, &dSingularTable_, &dRecords_, &dColumns_,
                                   &dPanelRhs_, &dBins_, &dBinCounts_, &dBinOffsets_, &dA_, &dLU_, &dRhs_, &dX_, &dCorr_, &dNorms_,
                                   &dPivots_, &dKs_, &dFlux_, &dObservers_, &dPartials_, &dField_, &dDegrees_,
                                   &dWork32_, &dGmres_, &dLuPack_, &dSolveScratch_})
@@ -747,7 +742,7 @@ std::unique_ptr<Result> Session::solve(const hs_request &r, const volatile int32
                 const double *fluxB = dFlux_.as<double>() + size_t(b) * E * T * 2;
                 const size_t reals = size_t(E) * N * 2;
                 double *nearRhs = dNearRhs_.as<double>();
-                assembleNearField(geo, dKs_.as<double>() + b, dGauss_.as<double>(), fluxB, E, layout,
+                assembleNearField(geo, dKs_.as<double>() + b, dSingularTuples_.as<double>(), fluxB, E, layout,
                                   dNearWork_.as<void>(), fmmSystem_->nearValues(), nearRhs, dError_.as<int>(), s,
                                   &timer_);
                 if (inner)
@@ -1273,7 +1268,7 @@ void Session::denseChain(const AssemblyGeometry &geo, const AssemblyWorkspace &w
                          cudaStream_t s, KernelTimer *timer, unsigned eventFlags) {
     const uint32_t N = geo.N;
     PhaseEvents &ev = phaseEvents();
-    assembleBatch(geo, dKs_.as<double>(), dGauss_.as<double>(), dFlux_.as<double>(), E, B, ws, dA_.as<double>(),
+    assembleBatch(geo, dKs_.as<double>(), dSingularTuples_.as<double>(), dFlux_.as<double>(), E, B, ws, dA_.as<double>(),
                   dRhs_.as<double>(), dError_.as<int>(), s, timer, mixed);
     cuda(cudaEventRecordWithFlags(ev.assembled, s, eventFlags), "phase event");
     // LU of every matrix of the batch (FP64, or an FP32 copy in the mixed
@@ -1327,7 +1322,7 @@ void Session::runDenseChain(const AssemblyGeometry &geo, const AssemblyWorkspace
     uint64_t signature = generation_ * 0x9e3779b97f4a7c15ull;
     for (const DeviceBuffer *b :
          {&dPanels_, &dBounds_, &dMixedPanels_, &dIncOffsets_, &dIncPanel_, &dIncLocal_, &dRowScale_, &dError_,
-          &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dGauss_, &dSingularTable_, &dRecords_, &dColumns_,
+          &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dSingularTuples_, &dSingularTable_, &dRecords_, &dColumns_,
           &dPanelRhs_, &dBins_, &dBinCounts_, &dBinOffsets_, &dA_, &dLU_, &dRhs_, &dX_, &dPivots_, &dInfo_, &dKs_,
           &dFlux_, &dWork32_, &dLuPack_, &dSolveScratch_})
         signature = (signature ^ reinterpret_cast<uintptr_t>(b->as<void>())) * 0x100000001b3ull;
@@ -1428,7 +1423,7 @@ void Session::debugAssemble(const hs_numerics &o, double planK, double k, const 
     AssemblyWorkspace ws{dRecords_.as<void>(), dColumns_.as<void>(), dPanelRhs_.as<double>(), dBins_.as<uint2>(),
                          dBinCounts_.as<uint32_t>(), size_t(T) * (T - 1) / 2,
                          T > kExactBinsT ? dBinOffsets_.as<uint64_t>() : nullptr};
-    assembleBatch(geo, dKs_.as<double>(), dGauss_.as<double>(), dFlux_.as<double>(), 1, 1, ws, dA_.as<double>(),
+    assembleBatch(geo, dKs_.as<double>(), dSingularTuples_.as<double>(), dFlux_.as<double>(), 1, 1, ws, dA_.as<double>(),
                   dRhs_.as<double>(), dError_.as<int>(), s, &timer_, o.precision == HS_PRECISION_MIXED);
     checkDeviceError("CUDA Galerkin assembly");
     cuda(cudaMemcpyAsync(matrix, dA_.as<void>(), size_t(N) * N * 16, cudaMemcpyDeviceToHost, s), "matrix download");
@@ -1480,7 +1475,7 @@ void Session::ensureFmmWorkspace(const hs_numerics &o, uint32_t E, uint32_t O, d
     dDegrees_.ensure(4);
     size_t bytes = 0;
     for (const DeviceBuffer *b : {&dPanels_, &dBounds_, &dMixedPanels_, &dIncOffsets_, &dIncPanel_, &dIncLocal_, &dRowScale_,
-                                  &dMass_, &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dGauss_, &dSingularTable_,
+                                  &dMass_, &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dSingularTuples_, &dSingularTable_,
                                   &dNearWork_, &dPanelRow_, &dPanelCol_, &dPanelPairs_, &dRhs_, &dX_, &dCorr_, &dNorms_,
                                   &dKs_, &dFlux_, &dObservers_, &dPartials_, &dField_, &dDegrees_})
         bytes += b->bytes();
@@ -1552,7 +1547,7 @@ void Session::directAuditSystem(const AssemblyGeometry &geo, double k, const dou
     AssemblyWorkspace ws{dRecords_.as<void>(), dColumns_.as<void>(), dPanelRhs_.as<double>(), dBins_.as<uint2>(),
                          dBinCounts_.as<uint32_t>(), size_t(T) * (T - 1) / 2,
                          T > kExactBinsT ? dBinOffsets_.as<uint64_t>() : nullptr};
-    assembleBatch(geo, dKs_.as<double>() + directAuditFrequency_, dGauss_.as<double>(), flux, E, 1, ws,
+    assembleBatch(geo, dKs_.as<double>() + directAuditFrequency_, dSingularTuples_.as<double>(), flux, E, 1, ws,
                   dA_.as<double>(), dAuditB_.as<double>(), dError_.as<int>(), stream(), nullptr, false);
     A = dA_.as<double>();
     b = dAuditB_.as<double>();

@@ -167,7 +167,7 @@ class Session {
     double planMs_ = 0;
     uint32_t planner_ = HS_PLANNER_DEVICE;
     DevicePlanStats planStats_;
-    DeviceBuffer dPairCode_, dTouching_, dNearPairs_, dPatches_, dGauss_, dSingularTable_;
+    DeviceBuffer dPairCode_, dTouching_, dNearPairs_, dPatches_, dSingularTuples_, dSingularTable_;
     // patches as the kernels see them: dPatches_, or the device alias of mapped
     // pinned host memory (residency)
     const Patch *patches_ = nullptr;
