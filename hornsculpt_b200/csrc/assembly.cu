@@ -1701,16 +1701,6 @@ __global__ void rhsVertexKernel(const double *__restrict__ panelRhs, const uint3
     dst[1] = im * rowScale[a];
 }
 
-int smCount() {
-    static PerDeviceValue<int> count;
-    return count.get([]() {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, currentDevice()) != cudaSuccess || n <= 0)
-            n = 148;
-        return n;
-    });
-}
-
 template <int NP>
 void launchRegular(const AssemblyGeometry &g, const double *ks, uint32_t B, const AssemblyWorkspace &ws, int bin,
                    int *error, cudaStream_t stream, KernelTimer *timer, bool mixed, const SlotMap &map) {

@@ -54,6 +54,10 @@ template <class R> __device__ __forceinline__ void csub(C2<R> &v, C2<R> a, C2<R>
     v.x -= a.x * b.x - a.y * b.y;
     v.y -= a.x * b.y + a.y * b.x;
 }
+template <> __device__ __forceinline__ void csub<double>(double2 &v, double2 a, double2 b) {  // four FP64 instructions, not six
+    v.x = fma(a.y, b.y, fma(-a.x, b.x, v.x));
+    v.y = fma(-a.y, b.x, fma(-a.x, b.y, v.y));
+}
 
 // Panel factorisation of columns [k0, k0+jb) over rows [k0, N) of one matrix.
 template <class R>
@@ -136,158 +140,12 @@ __global__ void __launch_bounds__(512) panelKernel(R *LU, uint32_t N, uint32_t k
     }
 }
 
-// Panel factorisation with the panel resident in shared memory (rows
-// [k0, N) x jb columns). Rows stay in place: step j selects the pivot among
-// the rows not yet selected (largest |re|+|im|, lowest row on ties), every
-// thread eliminates column j from its own rows and takes its candidate for
-// column j+1 in the same pass, so a column costs one barrier. The selection
-// order is turned into the LAPACK interchange sequence at the end and the
-// panel is written back in interchanged order.
-template <class R>
-__global__ void __launch_bounds__(1024) panelSmemKernel(R *LU, uint32_t N, uint32_t k0, uint32_t jb, int *pivots,
-                                                        int *info) {
-    extern __shared__ __align__(16) unsigned char rawSmem[];
-    const uint32_t rows = N - k0;
-    C2<R> *P = reinterpret_cast<C2<R> *>(rawSmem);                 // [jb][rows]
-    int *arrangement = reinterpret_cast<int *>(P + size_t(jb) * rows);  // position -> local row
-    int *where = arrangement + rows;                                 // local row -> position
-    uint32_t taken = 0;  // bit r: this thread's r-th row (threadIdx.x + r * blockDim.x) is a pivot row
-    __shared__ R sBest[2][32];
-    __shared__ int sRow[2][32];
-    __shared__ int sSel[kPanel];
-    R *M = LU + size_t(blockIdx.x) * N * N * 2;
-    int *piv = pivots + size_t(blockIdx.x) * N;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    // stage the panel: a batch of independent column loads in flight per thread
-    constexpr int kLoad = sizeof(R) == 8 ? 4 : 8;
-    for (uint32_t i = threadIdx.x; i < rows; i += blockDim.x) {
-        for (uint32_t q0 = 0; q0 < jb; q0 += kLoad) {
-            C2<R> v[kLoad];
-#pragma unroll
-            for (int t = 0; t < kLoad; ++t)
-                if (q0 + t < jb)
-                    v[t] = ld2(M + 2 * (size_t(k0 + q0 + t) * N + k0 + i));
-#pragma unroll
-            for (int t = 0; t < kLoad; ++t)
-                if (q0 + t < jb)
-                    P[size_t(q0 + t) * rows + i] = v[t];
-        }
-        arrangement[i] = int(i);
-        where[i] = int(i);
-    }
-    __syncthreads();
-    // candidates for column 0
-    R best = -1;
-    int bestRow = int(rows);
-    for (uint32_t i = threadIdx.x; i < rows; i += blockDim.x) {
-        const C2<R> v = P[i];
-        R a = fabs(v.x) + fabs(v.y);
-        if (!(a >= R(0)))
-            a = 0;  // a NaN row competes as zero, so a pivot row always exists
-        if (a > best) {
-            best = a;
-            bestRow = int(i);
-        }
-    }
-    for (uint32_t j = 0; j < jb; ++j) {
-        const int buf = j & 1;
-        for (int off = 16; off > 0; off >>= 1) {
-            const R ob = __shfl_down_sync(0xffffffffu, best, off);
-            const int oi = __shfl_down_sync(0xffffffffu, bestRow, off);
-            if (ob > best || (ob == best && oi < bestRow)) {
-                best = ob;
-                bestRow = oi;
-            }
-        }
-        if (lane == 0) {
-            sBest[buf][warp] = best;
-            sRow[buf][warp] = bestRow;
-        }
-        __syncthreads();
-        // every warp reduces the warp candidates by shuffles (same result in every warp)
-        R pb = lane < warps ? sBest[buf][lane] : R(-1);
-        int p = lane < warps ? sRow[buf][lane] : int(rows);
-        for (int off = 16; off > 0; off >>= 1) {
-            const R ob = __shfl_xor_sync(0xffffffffu, pb, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, p, off);
-            if (ob > pb || (ob == pb && oi < p)) {
-                pb = ob;
-                p = oi;
-            }
-        }
-        if (threadIdx.x == 0) {
-            sSel[j] = p;
-            if (!(pb > 0) && *info == 0)
-                atomicCAS(info, 0, int(k0 + j) + 1);
-        }
-        const C2<R> d = P[size_t(j) * rows + p];
-        const R den = d.x * d.x + d.y * d.y;
-        const R rden = den > 0 ? R(1) / den : R(0);
-        const C2<R> inv = mk<R>(d.x * rden, -d.y * rden);
-        best = -1;
-        bestRow = int(rows);
-        uint32_t r = 0;
-        for (uint32_t i = threadIdx.x; i < rows; i += blockDim.x, ++r) {
-            if (int(i) == p)
-                taken |= 1u << r;
-            if (taken >> r & 1u)
-                continue;
-            const C2<R> l = cmul<R>(P[size_t(j) * rows + i], inv);
-            P[size_t(j) * rows + i] = l;
-            // eliminate in chunks of columns: loads first, then updates and stores
-            constexpr int kChunk = sizeof(R) == 8 ? 4 : 8;
-            C2<R> next = mk<R>(0, 0);
-            for (uint32_t q0 = j + 1; q0 < jb; q0 += kChunk) {
-                C2<R> v[kChunk], pv[kChunk];
-#pragma unroll
-                for (int t = 0; t < kChunk; ++t)
-                    if (q0 + t < jb) {
-                        v[t] = P[size_t(q0 + t) * rows + i];
-                        pv[t] = P[size_t(q0 + t) * rows + p];
-                    }
-#pragma unroll
-                for (int t = 0; t < kChunk; ++t)
-                    if (q0 + t < jb) {
-                        csub<R>(v[t], l, pv[t]);
-                        P[size_t(q0 + t) * rows + i] = v[t];
-                    }
-                if (q0 == j + 1)
-                    next = v[0];
-            }
-            if (j + 1 < jb) {
-                R a = fabs(next.x) + fabs(next.y);
-                if (!(a >= R(0)))
-                    a = 0;
-                if (a > best) {
-                    best = a;
-                    bestRow = int(i);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    // selection order -> interchange sequence (row k0+j swapped with row piv[k0+j])
-    if (threadIdx.x == 0)
-        for (uint32_t j = 0; j < jb; ++j) {
-            const int r = sSel[j], pj = where[r], rj = arrangement[j];
-            piv[k0 + j] = int(k0) + pj;
-            arrangement[j] = r;
-            arrangement[pj] = rj;
-            where[r] = int(j);
-            where[rj] = pj;
-        }
-    __syncthreads();
-    for (uint32_t q = 0; q < jb; ++q)
-        for (uint32_t i = threadIdx.x; i < rows; i += blockDim.x)
-            st2(M + 2 * (size_t(k0 + q) * N + k0 + i), P[size_t(q) * rows + arrangement[i]]);
-}
-
 // Panel factorisation for tall panels, spread over a thread-block cluster:
 // CTA r of the cluster owns panel rows [r * rowsPerBlock, ...). The first
 // `cap` of them live in shared memory, one per thread; the rest (at most
 // kGlobalSlots per thread) stay in place in global memory and are eliminated
 // there by their thread. Pivot choice, tie rule and interchange sequence are
-// those of panelSmemKernel. Per column: each warp's best candidate goes to its
+// those of panelRegKernel. Per column: each warp's best candidate goes to its
 // CTA's shared memory (double-buffered by column parity); one cluster barrier;
 // every warp reduces the candidates of all CTAs through distributed shared
 // memory; one warp per CTA copies the pivot row from the CTA that holds it
@@ -300,7 +158,6 @@ __global__ void __launch_bounds__(1024) panelSmemKernel(R *LU, uint32_t N, uint3
 // their final positions. A final cluster barrier keeps every CTA's shared
 // memory alive until all remote reads are done.
 template <class R> constexpr uint32_t kClusterRows = sizeof(R) == 8 ? 384 : 768;
-constexpr uint32_t kMaxCluster = 16;
 constexpr int kGlobalSlots = 4;
 
 template <class R> struct ClusterPanelShared {
@@ -314,7 +171,7 @@ template <class R> struct ClusterPanelShared {
     int mapCount;
 };
 
-template <class R, int Slots>
+template <class R>
 __global__ void __launch_bounds__(1024) panelClusterKernel(R *LU, uint32_t N, uint32_t k0, uint32_t jb,
                                                            uint32_t rowsPerBlock, uint32_t cap, int *pivots,
                                                            int *info) {
@@ -351,11 +208,11 @@ __global__ void __launch_bounds__(1024) panelClusterKernel(R *LU, uint32_t N, ui
         const R a = fabs(z.x) + fabs(z.y);
         return a >= R(0) ? a : R(0);  // a NaN row competes as zero, so a pivot row always exists
     };
-    bool taken[1 + Slots];
+    bool taken[1 + kGlobalSlots];
     R best = R(-1);
     int bestRow = int(rows);
 #pragma unroll
-    for (int s = 0; s <= Slots; ++s) {
+    for (int s = 0; s <= kGlobalSlots; ++s) {
         taken[s] = !owns(s);
         if (!taken[s]) {
             const uint32_t g = rowBegin + local(s);
@@ -437,7 +294,7 @@ __global__ void __launch_bounds__(1024) panelClusterKernel(R *LU, uint32_t N, ui
         best = -1;
         bestRow = int(rows);
 #pragma unroll
-        for (int s = 0; s <= Slots; ++s) {
+        for (int s = 0; s <= kGlobalSlots; ++s) {
             if (taken[s])
                 continue;
             const uint32_t g = rowBegin + local(s);
@@ -577,7 +434,7 @@ __global__ void __launch_bounds__(1024) panelClusterKernel(R *LU, uint32_t N, ui
     };
     // pivots kept in global memory move to their positions (< jb; those rows are in CTA 0's shared memory)
 #pragma unroll
-    for (int s = 1; s <= Slots; ++s)
+    for (int s = 1; s <= kGlobalSlots; ++s)
         if (owns(s)) {
             const uint32_t g = rowBegin + local(s), pos = finalPosition(g);
             if (pos != g)
@@ -593,228 +450,430 @@ __global__ void __launch_bounds__(1024) panelClusterKernel(R *LU, uint32_t N, ui
     cluster.sync();  // keep rank 0's map alive until every CTA has read it
 }
 
-template <class R> size_t panelSmemBytes(uint32_t rows, uint32_t jb) {
-    return size_t(rows) * jb * sizeof(C2<R>) + size_t(rows) * 8;
+// Panel factorisation in registers: the panel's rows are spread over a cluster
+// of at most kMaxCluster CTAs (one for small matrices), one row per thread, two
+// in FP32 where one does not reach (panelShape). Pivot rule: largest
+// |re| + |im|, the lowest row on ties, a NaN row competes as zero; rows stay in
+// place until the end, where the selection order becomes the LAPACK
+// interchange sequence.
+//
+// Bound: the chain of 32 columns, each a maximum over all rows, the pivot row's
+// way to every thread and the elimination. So:
+//   * The panel is factored in two halves of 16 columns. A row's 16 values stay
+//     in registers and the elimination reads nothing but the pivot row
+//     (elimination in shared memory moved every remaining entry twice per
+//     column). Before the right half, its 16 pivot rows are solved with the
+//     left half's multipliers and every other row gets the left half's update
+//     in one pass. Each entry sees the operations of a 32-column right-looking
+//     elimination in the same order.
+//   * A column costs one block barrier and one cluster barrier: warps find their
+//     best row with integer reductions on the magnitude's bits (while the other
+//     columns' updates are still in flight), and its lane publishes the row;
+//     after the block barrier every warp finds the CTA's winner, and the warps
+//     push it to the CTAs of the cluster; after the cluster barrier each CTA has
+//     all candidates in its own shared memory. Candidate slots alternate with
+//     the column's parity: a slot is written again only after the barrier of
+//     the next column, which its readers have passed.
+//   * Register indices must be constants, and 16 unrolled columns are too long
+//     for the instruction cache, so the loop body handles kPanelUnroll columns
+//     and rotates the rows by that many: at column j of a half, a[r][c] holds
+//     its column j + c for c < 16 - j, and the finished columns after them.
+// The pushes of a column precede its cluster barrier and nothing is read
+// remotely after the last one, so a CTA may exit on its own.
+//
+// Measured, all panels of a solve, against panels in shared memory (one CTA or
+// cluster) and 32-column register panels of one CTA. FP64: N = 258 0.56 -> 0.32
+// ms, N = 642 x 32 1.78 -> 1.00, N = 2562 x 2 8.9 -> 4.6, N = 6380 28.1 -> 13.6.
+// FP32: N = 642 x 32 1.00 -> 0.82, N = 4023 x 3 13.2 -> 6.4, N = 6380 22.3 ->
+// 11.0. Of a column's 1.7 us at 15 CTAs about 0.7 are the push and the cluster
+// barrier, 0.3 the reductions within the CTA, 0.3 the candidate, 0.2 the updates.
+constexpr int kHalf = 16;
+constexpr int kPanelUnroll = 2;
+constexpr uint32_t kPanelThreads = 512;  // at most
+constexpr int kPanelWarps = int(kPanelThreads / 32);
+constexpr uint32_t kMaxCluster = 16;
+// Row moves of one panel: entry q < 32 the panel row that goes to position q,
+// entry 32 + r the position of panel row r when it is no pivot row and moves (else -1).
+constexpr int kMoves = 2 * kPanel;
+
+// Order-preserving key of a magnitude (non-negative), zero for "no row".
+struct PivotKey {
+    unsigned hi = 0, lo = 0;
+};
+__device__ __forceinline__ PivotKey pivotKey(double m) {
+    return {unsigned(__double2hiint(m)) + 1u, unsigned(__double2loint(m))};
 }
-constexpr size_t kPanelSmemLimit = 220 * 1024;
+__device__ __forceinline__ PivotKey pivotKey(float m) { return {__float_as_uint(m) + 1u, 0u}; }
+__device__ __forceinline__ bool zeroKey(PivotKey k) { return k.hi <= 1u && k.lo == 0u; }
 
-// FP32 panel factorisation with the panel in registers, for full 32-column
-// panels of at most kRegPanelRows rows: thread t owns panel rows
-// t + r * blockDim.x (r < kRegRowsPerThread), 32 complex values each, so the
-// elimination reads nothing but the pivot row. Pivot rule, tie rule and
-// interchange sequence are those of panelSmemKernel, and every entry of a
-// row that is not yet a pivot row is updated by the same operations in the
-// same order (a pivot row's multiplier is zero, which leaves finite values
-// unchanged).
-//
-// Per column, each warp reduces its candidates by shuffles and the lane that
-// holds the warp's best row writes that row's remaining columns to the
-// warp's slot in shared memory; after the column's one barrier every warp
-// reduces the warp candidates, reads the pivot row from the winning warp's
-// slot and eliminates its own rows. Slots and candidates alternate with the
-// column's parity: a warp writes the slot of column j + 2 only after the
-// barrier of column j + 1, which every reader of column j has passed.
-//
-// Register indices must be constants, and a fully unrolled 32-column body is
-// too long for the instruction cache (an earlier build stalled on
-// instruction fetch for most of its cycles). So each row is rotated instead:
-// at column j, a[r][c] holds column j + c for c < 32 - j and the finished
-// columns j + c - 32 after them. The loop body handles kRegUnroll columns
-// with constant indices (updates of the entries c >= 32 - j are predicated
-// off) and rotates the rows by kRegUnroll at its end; after the 32 columns
-// every row is back in column order.
-// Eight warps, so that each SM sub-partition holds two and a thread may use
-// 255 registers: 64 per row.
-constexpr int kRegRowsPerThread = 3;
-constexpr int kRegUnroll = 2;
-constexpr uint32_t kRegPanelThreads = 256;
-constexpr uint32_t kRegPanelRows = kRegRowsPerThread * kRegPanelThreads;
-constexpr int kRegPanelWarps = int(kRegPanelThreads / 32);
+// The largest key of the warp and the lowest row that has it; true in the lanes that hold it.
+template <class R> __device__ __forceinline__ bool warpPivot(PivotKey &key, int &row) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, key.hi);
+    bool mine = key.hi == hi;
+    unsigned lo = 0;
+    if constexpr (sizeof(R) == 8) {
+        lo = __reduce_max_sync(0xffffffffu, mine ? key.lo : 0u);
+        mine = mine && key.lo == lo;
+    }
+    const int lowest = __reduce_min_sync(0xffffffffu, mine ? row : 0x7fffffff);
+    mine = mine && row == lowest;
+    key = {hi, lo};
+    row = lowest;
+    return mine;
+}
 
-__global__ void __launch_bounds__(kRegPanelThreads, 1) panelRegKernel(float *LU, uint32_t N, uint32_t k0, int *pivots,
-                                                                      int *info) {
-    constexpr int RT = kRegRowsPerThread, U = kRegUnroll;
-    static_assert(kPanel % U == 0, "the column groups must tile the panel");
-    __shared__ __align__(16) float2 sCand[2][kRegPanelWarps][kPanel];
-    __shared__ float sBest[2][kRegPanelWarps];
-    __shared__ int sRow[2][kRegPanelWarps];
-    __shared__ int sSel[kPanel];
-    __shared__ int arrangement[kRegPanelRows], where[kRegPanelRows];
-    const uint32_t rows = N - k0, T = blockDim.x;
-    float *M = LU + size_t(blockIdx.x) * N * N * 2;
-    int *piv = pivots + size_t(blockIdx.x) * N;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = int(T >> 5);
-    int row[RT];
-    bool have[RT], taken[RT];
-    float2 a[RT][kPanel];
+template <class R> struct PanelShared {
+    __align__(16) C2<R> warpRow[2][kPanelWarps][kHalf];  // per warp: its candidate's remaining columns
+    __align__(16) C2<R> ctaRow[2][kMaxCluster][kHalf];   // per CTA of the cluster, pushed by it
+    __align__(16) C2<R> own[kHalf][kPanel];              // left pivot rows of this CTA: multipliers, right half
+    __align__(16) C2<R> top[kHalf][kPanel];              // all left pivot rows, then their solved right half
+    int4 warpKey[2][kPanelWarps];
+    int4 ctaKey[2][kMaxCluster];  // (hi, lo, row, 0)
+    int sel[kPanel], position[kPanel];
+};
+
+template <class R, int RT>
+__global__ void __launch_bounds__(kPanelThreads, 1) panelRegKernel(R *LU, uint32_t N, uint32_t k0, uint32_t jb,
+                                                                   uint32_t perBlock, int *pivots, int *moves,
+                                                                   int *info) {
+    namespace cg = cooperative_groups;
+    constexpr int U = kPanelUnroll;
+    static_assert(kHalf % U == 0 && kPanel == 2 * kHalf, "the column groups must tile the halves");
+    extern __shared__ __align__(16) unsigned char rawSmem[];
+    C2<R> *left = reinterpret_cast<C2<R> *>(rawSmem);  // [kHalf][perBlock]: the finished left half
+    __shared__ PanelShared<R> sh;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), C = cluster.num_blocks();
+    // a CTA's shared memory may be written by the others only once it runs: arrive
+    // here, wait before the first push
+    if (C > 1)
+        cluster.barrier_arrive();
+    const uint32_t rows = N - k0, rowBegin = rank * perBlock;
+    const uint32_t myRows = rowBegin < rows ? min(perBlock, rows - rowBegin) : 0u;
+    R *M = LU + size_t(blockIdx.y) * N * N * 2 + 2 * (size_t(k0) * N + k0);  // entry (0, 0) of the panel
+    const size_t stride = size_t(N) * 2;
+    const uint32_t threads = blockDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = int(threads >> 5);
+    const C2<R> zero = mk<R>(0, 0);
+    int row[RT], taken[RT];  // panel row (-1: none); its pivot index, -1 for none, kPanel without a row
 #pragma unroll
     for (int r = 0; r < RT; ++r) {
-        row[r] = int(threadIdx.x + r * T);
-        have[r] = uint32_t(row[r]) < rows;
-        taken[r] = !have[r];
+        const uint32_t local = threadIdx.x + r * threads;
+        row[r] = local < myRows ? int(rowBegin + local) : -1;  // never equal to a pivot of another CTA
+        taken[r] = local < myRows ? -1 : kPanel;
     }
-#pragma unroll
-    for (int q = 0; q < kPanel; ++q) {
-        const float *col = M + 2 * (size_t(k0 + q) * N + k0);
-#pragma unroll
-        for (int r = 0; r < RT; ++r)
-            a[r][q] = have[r] ? ld2<float>(col + 2 * row[r]) : make_float2(0.f, 0.f);
-    }
-    for (uint32_t i = threadIdx.x; i < rows; i += T) {
-        arrangement[i] = int(i);
-        where[i] = int(i);
-    }
-    const auto magnitude = [](float2 z) {
-        const float m = fabsf(z.x) + fabsf(z.y);
-        return m >= 0.f ? m : 0.f;  // a NaN row competes as zero, so a pivot row always exists
+    const auto magnitude = [](C2<R> z) {
+        const R m = fabs(z.x) + fabs(z.y);
+        return m >= R(0) ? m : R(0);
     };
+    C2<R> a[RT][kHalf];
 #pragma unroll 1
-    for (int j0 = 0; j0 < kPanel; j0 += U) {
+    for (int h = 0; h < 2; ++h) {
+        const int h0 = h * kHalf, width = min(kHalf, int(jb) - h0);
+        if (width <= 0)
+            break;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            // column j = j0 + u sits at index u of the rotated rows; its remaining
-            // columns at indices u .. u + left - 1
-            const int j = j0 + u, buf = j & 1, left = kPanel - j;
-            float best = -1.f;
-            int bestRow = int(rows), bestSlot = -1;
+        for (int c = 0; c < kHalf; ++c)
 #pragma unroll
             for (int r = 0; r < RT; ++r)
-                if (!taken[r]) {
-                    const float m = magnitude(a[r][u]);
+                a[r][c] = taken[r] != kPanel && c < width ? ld2(M + (h0 + c) * stride + 2 * row[r]) : zero;
+        if (h == 0 && C > 1)
+            cluster.barrier_wait();
+        if (h == 1) {  // the left half's update: solved values for its pivot rows, 16 products for the others
+#pragma unroll 1
+            for (int j = 0; j < kHalf; ++j) {
+                C2<R> l[RT];
+#pragma unroll
+                for (int r = 0; r < RT; ++r)
+                    l[r] = taken[r] < 0 ? left[size_t(j) * perBlock + threadIdx.x + r * threads] : zero;
+#pragma unroll
+                for (int c = 0; c < kHalf; ++c) {
+                    const C2<R> u = sh.top[j][kHalf + c];
+#pragma unroll
+                    for (int r = 0; r < RT; ++r)
+                        csub<R>(a[r][c], l[r], u);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+                if (taken[r] >= 0 && taken[r] < kPanel)
+#pragma unroll
+                    for (int c = 0; c < kHalf; ++c)
+                        a[r][c] = sh.top[taken[r]][kHalf + c];
+        }
+        // this warp's best row for the entries at index c; the row's lane returns true
+        const auto candidate = [&](int c, PivotKey &key, int &bestRow, int &slot) {
+            R best = R(-1);
+            bestRow = 0x7fffffff;
+            slot = -1;
+#pragma unroll
+            for (int r = 0; r < RT; ++r)
+                if (taken[r] < 0) {
+                    const R m = magnitude(a[r][c]);
                     if (m > best) {  // rows ascend with r: ties keep the lower row
                         best = m;
                         bestRow = row[r];
-                        bestSlot = r;
+                        slot = r;
                     }
                 }
-            const int myRow = bestRow;
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-                const int oi = __shfl_xor_sync(0xffffffffu, bestRow, off);
-                if (ob > best || (ob == best && oi < bestRow)) {
-                    best = ob;
-                    bestRow = oi;
-                }
-            }
-            // the warp's candidate row (slot entry c = column j + c; entries past the
-            // panel's end are never read)
-            if (bestSlot >= 0 && myRow == bestRow) {
-                float4 *dst = reinterpret_cast<float4 *>(&sCand[buf][warp][0]);
+            key = slot >= 0 ? pivotKey(best) : PivotKey{};
+            return warpPivot<R>(key, bestRow) && slot >= 0;
+        };
+        PivotKey key;
+        int bestRow, slot;
+        bool mine = candidate(0, key, bestRow, slot);
+#pragma unroll 1
+        for (int j0 = 0; j0 < kHalf; j0 += U) {
 #pragma unroll
-                for (int c = 0; c < kPanel; c += 2) {
-                    float2 x0 = a[0][(u + c) % kPanel], x1 = a[0][(u + c + 1) % kPanel];
+            for (int u = 0; u < U; ++u) {
+                // column j of the half sits at index u of the rotated rows
+                const int j = j0 + u, remaining = kHalf - j, buf = j & 1;
+                if (j >= width)
+                    break;  // the same for the whole cluster
+                if (mine) {
 #pragma unroll
-                    for (int r = 1; r < RT; ++r)
-                        if (bestSlot == r) {
-                            x0 = a[r][(u + c) % kPanel];
-                            x1 = a[r][(u + c + 1) % kPanel];
-                        }
-                    dst[c / 2] = make_float4(x0.x, x0.y, x1.x, x1.y);
+                    for (int c = 0; c < kHalf; ++c) {
+                        if (c >= remaining)
+                            break;
+                        C2<R> v = a[0][(u + c) % kHalf];
+#pragma unroll
+                        for (int r = 1; r < RT; ++r)
+                            if (slot == r)
+                                v = a[r][(u + c) % kHalf];
+                        sh.warpRow[buf][warp][c] = v;
+                    }
+                }
+                if (lane == 0)
+                    sh.warpKey[buf][warp] = make_int4(int(key.hi), int(key.lo), bestRow, 0);
+                __syncthreads();
+                int4 found = lane < warps ? sh.warpKey[buf][lane] : make_int4(0, 0, 0x7fffffff, 0);
+                key = {unsigned(found.x), unsigned(found.y)};
+                int p = found.z;
+                int winner = __ffs(__ballot_sync(0xffffffffu, warpPivot<R>(key, p))) - 1;
+                const C2<R> *pivotRow = sh.warpRow[buf][winner];
+                if (C > 1) {
+                    for (uint32_t to = warp; to < C; to += warps) {
+                        PanelShared<R> *other = cluster.map_shared_rank(&sh, int(to));
+                        if (lane < kHalf)
+                            other->ctaRow[buf][rank][lane] = pivotRow[lane];
+                        else if (lane == kHalf)
+                            other->ctaKey[buf][rank] = make_int4(int(key.hi), int(key.lo), p, 0);
+                    }
+                    cluster.sync();
+                    found = uint32_t(lane) < C ? sh.ctaKey[buf][lane] : make_int4(0, 0, 0x7fffffff, 0);
+                    key = {unsigned(found.x), unsigned(found.y)};
+                    p = found.z;
+                    winner = __ffs(__ballot_sync(0xffffffffu, warpPivot<R>(key, p))) - 1;
+                    pivotRow = sh.ctaRow[buf][winner];
+                }
+                if (threadIdx.x == 0) {
+                    sh.sel[h0 + j] = p;
+                    if (rank == 0 && zeroKey(key) && *info == 0)
+                        atomicCAS(info, 0, int(k0) + h0 + j + 1);
+                }
+                const C2<R> d = pivotRow[0];
+                const R den = d.x * d.x + d.y * d.y;
+                const R rden = den > R(0) ? R(1) / den : R(0);
+                const C2<R> inv = mk<R>(d.x * rden, -d.y * rden);
+                C2<R> l[RT];
+#pragma unroll
+                for (int r = 0; r < RT; ++r) {
+                    if (row[r] == p)
+                        taken[r] = h0 + j;
+                    const C2<R> m = cmul<R>(a[r][u], inv);
+                    l[r] = taken[r] >= 0 ? zero : m;  // a pivot row keeps its values
+                    a[r][u] = taken[r] >= 0 ? a[r][u] : m;
+                }
+                // the next column first: its candidate's reductions overlap the other columns' updates
+                if (remaining > 1)
+#pragma unroll
+                    for (int r = 0; r < RT; ++r)
+                        csub<R>(a[r][(u + 1) % kHalf], l[r], pivotRow[1]);
+                mine = candidate((u + 1) % kHalf, key, bestRow, slot);
+#pragma unroll
+                for (int c = 2; c < kHalf; ++c) {
+                    if (c >= remaining)  // finished columns
+                        break;
+                    const C2<R> pv = pivotRow[c];
+#pragma unroll
+                    for (int r = 0; r < RT; ++r)
+                        csub<R>(a[r][(u + c) % kHalf], l[r], pv);
                 }
             }
-            if (lane == 0) {
-                sBest[buf][warp] = best;
-                sRow[buf][warp] = bestRow;
-            }
-            __syncthreads();
-            // every warp reduces the warp candidates by shuffles (same result in every warp)
-            float pb = lane < warps ? sBest[buf][lane] : -1.f;
-            int p = lane < warps ? sRow[buf][lane] : int(rows), pw = lane;
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, pb, off);
-                const int oi = __shfl_xor_sync(0xffffffffu, p, off), ow = __shfl_xor_sync(0xffffffffu, pw, off);
-                if (ob > pb || (ob == pb && oi < p)) {
-                    pb = ob;
-                    p = oi;
-                    pw = ow;
-                }
-            }
-            if (threadIdx.x == 0) {
-                sSel[j] = p;
-                if (!(pb > 0.f) && *info == 0)
-                    atomicCAS(info, 0, int(k0) + j + 1);
-            }
-            const float2 *prow = sCand[buf][pw];
-            const float2 d = prow[0];
-            const float den = d.x * d.x + d.y * d.y;
-            const float rden = den > 0.f ? 1.f / den : 0.f;
-            const float2 inv = make_float2(d.x * rden, -d.y * rden);
-            // a row already chosen as a pivot row keeps its values: its multiplier is zero
-            float2 l[RT];
+            // rotate every row left by U
 #pragma unroll
             for (int r = 0; r < RT; ++r) {
-                taken[r] |= p == row[r];
-                const float2 m = cmul<float>(a[r][u], inv);
-                l[r] = taken[r] ? make_float2(0.f, 0.f) : m;
-                a[r][u] = taken[r] ? a[r][u] : m;
-            }
+                C2<R> t[U];
 #pragma unroll
-            for (int c = 1; c < kPanel; ++c) {
-                if (c >= left)  // finished columns
-                    break;
-                const float2 pv = prow[c];
+                for (int c = 0; c < U; ++c)
+                    t[c] = a[r][c];
 #pragma unroll
-                for (int r = 0; r < RT; ++r)
-                    csub<float>(a[r][(u + c) % kPanel], l[r], pv);
+                for (int c = 0; c + U < kHalf; ++c)
+                    a[r][c] = a[r][c + U];
+#pragma unroll
+                for (int c = 0; c < U; ++c)
+                    a[r][kHalf - U + c] = t[c];
             }
         }
-        // rotate every row left by U: index c takes column j0 + U + c
-        float2 t[RT][U];
+        if (h == 0 && int(jb) > kHalf) {
+            // put the left half aside; its pivot rows, with their right half, to every CTA
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
+            for (int r = 0; r < RT; ++r)
+                if (taken[r] != kPanel) {
 #pragma unroll
-            for (int c = 0; c < U; ++c)
-                t[r][c] = a[r][c];
+                    for (int c = 0; c < kHalf; ++c)
+                        left[size_t(c) * perBlock + threadIdx.x + r * threads] = a[r][c];
+                    if (taken[r] >= 0)
 #pragma unroll
-            for (int c = 0; c + U < kPanel; ++c)
-                a[r][c] = a[r][c + U];
+                        for (int c = 0; c < kHalf; ++c) {
+                            sh.own[taken[r]][c] = a[r][c];
+                            sh.own[taken[r]][kHalf + c] =
+                                kHalf + c < int(jb) ? ld2(M + (kHalf + c) * stride + 2 * row[r]) : zero;
+                        }
+                }
+            cluster.sync();
+            for (uint32_t e = threadIdx.x; e < uint32_t(kHalf * kPanel); e += threads) {
+                const uint32_t q = e / kPanel, c = e % kPanel;
+                sh.top[q][c] = cluster.map_shared_rank(&sh, int(uint32_t(sh.sel[q]) / perBlock))->own[q][c];
+            }
+            __syncthreads();
+            if (warp < kHalf / 2) {  // U12 = L11^-1 A12: a half warp per column, lane = pivot row
+                const int i = lane & (kHalf - 1), c = kHalf + 2 * warp + (lane >> 4);
+                C2<R> x = sh.top[i][c];
 #pragma unroll
-            for (int c = 0; c < U; ++c)
-                a[r][kPanel - U + c] = t[r][c];
+                for (int j = 0; j + 1 < kHalf; ++j) {
+                    const int from = (lane & kHalf) | j;
+                    const C2<R> xj = mk<R>(__shfl_sync(0xffffffffu, x.x, from), __shfl_sync(0xffffffffu, x.y, from));
+                    if (i > j)
+                        csub<R>(x, sh.top[i][j], xj);
+                }
+                __syncwarp();
+                sh.top[i][c] = x;
+            }
+            __syncthreads();
         }
     }
     __syncthreads();
-    // selection order -> interchange sequence (row k0+j swapped with row piv[k0+j])
-    if (threadIdx.x == 0)
-        for (int j = 0; j < kPanel; ++j) {
-            const int r = sSel[j], pj = where[r], rj = arrangement[j];
-            piv[k0 + j] = int(k0) + pj;
-            arrangement[j] = r;
-            arrangement[pj] = rj;
-            where[r] = j;
-            where[rj] = pj;
+    // Selection order -> interchanges (row k0 + j swapped with row piv[k0 + j]) and final positions:
+    // lane q holds the row now at position q and the position of panel row q.
+    if (warp == 0) {
+        int at = lane, where = lane;
+        bool selected = false;
+        for (int j = 0; j < int(jb); ++j) {
+            const int s = sh.sel[j], here = __shfl_sync(0xffffffffu, at, j);
+            const int from = __shfl_sync(0xffffffffu, where, s & 31);
+            const int pj = s < kPanel ? from : s;
+            if (rank == 0 && lane == 0)
+                pivots[size_t(blockIdx.y) * N + k0 + j] = int(k0) + pj;
+            if (lane == pj)
+                at = here;
+            if (lane == j)
+                at = s;
+            if (lane == here)
+                where = pj;
+            if (lane == s) {
+                where = j;
+                selected = true;
+            }
         }
+        sh.position[lane] = where;
+        if (rank == 0) {
+            int *mv = moves + size_t(blockIdx.y) * kMoves;
+            mv[lane] = lane < int(jb) ? sh.sel[lane] : -1;
+            mv[kPanel + lane] = selected || where == lane ? -1 : where;
+        }
+    }
     __syncthreads();
-    // row r of this thread goes to position where[row]; one running pointer per row
-    float *out[RT];
+    const int h0 = int(jb) > kHalf ? kHalf : 0;
 #pragma unroll
-    for (int r = 0; r < RT; ++r)
-        out[r] = M + 2 * (size_t(k0) * N + k0 + (have[r] ? where[row[r]] : 0));
-    const size_t stride = size_t(N) * 2;
+    for (int r = 0; r < RT; ++r) {
+        if (taken[r] == kPanel)
+            continue;
+        const int pos = taken[r] >= 0 ? taken[r] : row[r] < kPanel ? sh.position[row[r]] : row[r];
+        R *out = M + 2 * pos;
+        if (h0)
 #pragma unroll
-    for (int q = 0; q < kPanel; ++q)
+            for (int c = 0; c < kHalf; ++c)
+                st2(out + c * stride, left[size_t(c) * perBlock + threadIdx.x + r * threads]);
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
-            if (have[r])
-                st2<float>(out[r], a[r][q]);
-            out[r] += stride;
-        }
+        for (int c = 0; c < kHalf; ++c)
+            if (h0 + c < int(jb))
+                st2(out + (h0 + c) * stride, a[r][c]);
+    }
 }
 
-// Row interchanges of the panel applied to columns outside it.
-template <class R> __global__ void swapKernel(R *LU, uint32_t N, uint32_t k0, uint32_t jb, const int *pivots) {
-    const uint32_t col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= N || (col >= k0 && col < k0 + jb))
-        return;
-    R *M = LU + size_t(blockIdx.y) * N * N * 2 + 2 * size_t(col) * N;
-    const int *piv = pivots + size_t(blockIdx.y) * N;
-    for (uint32_t c = k0; c < k0 + jb; ++c) {
-        const int p = piv[c];
-        if (p != int(c)) {
-            const C2<R> a = ld2(M + 2 * c), b = ld2(M + 2 * p);
-            st2(M + 2 * c, b);
-            st2(M + 2 * p, a);
+// Moves of one panel for the panels that do not come from panelRegKernel: from
+// the interchange sequence, one warp per matrix (see kMoves).
+__global__ void panelMovesKernel(const int *pivots, uint32_t N, uint32_t k0, uint32_t jb, int *moves) {
+    __shared__ int rowAt[kMoves], position[kMoves];  // the rows and positions the interchanges touch
+    const int *piv = pivots + size_t(blockIdx.x) * N;
+    int *mv = moves + size_t(blockIdx.x) * kMoves;
+    const int lane = threadIdx.x;
+    // slots 0..31 are positions 0..31, slot 32 + j the position of interchange j's partner if it is below them
+    rowAt[lane] = lane;
+    position[lane] = lane;
+    const int partner = lane < int(jb) ? piv[k0 + lane] - int(k0) : -1;
+    rowAt[kPanel + lane] = position[kPanel + lane] = partner >= kPanel ? partner : -1;
+    mv[lane] = mv[kPanel + lane] = -1;
+    __syncwarp();
+    if (lane == 0)
+        for (int j = 0; j < int(jb); ++j) {
+            const int q = piv[k0 + j] - int(k0);
+            int slot = q;
+            if (q >= kPanel) {  // the first slot of that position carries its row
+                slot = kPanel;
+                while (position[slot] != q)
+                    ++slot;
+            }
+            const int t = rowAt[j];
+            rowAt[j] = rowAt[slot];
+            rowAt[slot] = t;
         }
+    __syncwarp();
+    if (lane < int(jb))
+        mv[lane] = rowAt[lane];
+    __syncwarp();
+    // rows of the first 32 that ended below: a position's first slot holds its row
+    const int slot = kPanel + lane, at = position[slot];
+    bool first = at >= 0;
+    for (int q = kPanel; q < slot; ++q)
+        first = first && position[q] != at;
+    if (first && rowAt[slot] < kPanel)
+        mv[kPanel + rowAt[slot]] = at;
+}
+
+// Row interchanges of the panel applied to the columns outside it: a warp takes
+// kSwapColumns columns, reads the (at most 64) entries that move and writes them
+// to their places. All reads are in flight together; following the
+// interchanges one after the other took a memory latency for each
+// (N = 6380: 1.74 -> 1.31 ms over a factorisation's 200 panels).
+constexpr int kSwapColumns = 4;
+template <class R>
+__global__ void __launch_bounds__(256) swapKernel(R *LU, uint32_t N, uint32_t k0, uint32_t jb, const int *moves) {
+    const int lane = threadIdx.x & 31;
+    const int *mv = moves + size_t(blockIdx.y) * kMoves;
+    const int from = mv[lane], to = mv[kPanel + lane];  // row `from` to position lane, row lane to position `to`
+    const bool in = from >= 0 && from != lane, out = to >= 0;
+    const uint32_t first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kSwapColumns;
+    R *M = LU + size_t(blockIdx.y) * N * N * 2 + 2 * (size_t(first) * N + k0);
+    C2<R> vIn[kSwapColumns], vOut[kSwapColumns];
+    bool active[kSwapColumns];
+#pragma unroll
+    for (int c = 0; c < kSwapColumns; ++c) {
+        const uint32_t col = first + c;
+        active[c] = col < N && (col < k0 || col >= k0 + jb);
+        if (active[c] && in)
+            vIn[c] = ld2(M + 2 * (size_t(c) * N + from));
+        if (active[c] && out)
+            vOut[c] = ld2(M + 2 * (size_t(c) * N + lane));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < kSwapColumns; ++c) {
+        if (active[c] && in)
+            st2(M + 2 * (size_t(c) * N + lane), vIn[c]);
+        if (active[c] && out)
+            st2(M + 2 * (size_t(c) * N + to), vOut[c]);
     }
 }
 
@@ -1608,46 +1667,69 @@ __global__ void toFloatKernel(const double *in, float *out, size_t count) {
         out[i] = float(in[i]);
 }
 
-// Largest cluster the panel kernel may use on this device: 16 CTAs (opt-in)
-// when the device can schedule such a cluster with full panel shared memory,
-// else the portable 8, else none.
+template <class R> constexpr size_t panelRegSmem(uint32_t perBlock) { return size_t(kHalf) * perBlock * sizeof(C2<R>); }
+template <class R> constexpr size_t kClusterSmem = size_t(kPanel) * kClusterRows<R> * sizeof(C2<R>);
+
+cudaLaunchConfig_t clusterConfig(uint32_t C, uint32_t B, uint32_t threads, size_t smem, cudaStream_t stream,
+                                 cudaLaunchAttribute &attr) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C, B);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = C;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Shape of a panelRegKernel launch. Small CTAs shorten every step of a column
+// (256 threads against 512: 11.0 against 11.7 ms FP32 and 13.6 against 14.8 ms
+// FP64 at N = 6380, 0.82 against 0.89 at N = 642 x 32), as long as a cluster
+// holds the panel and the batch's CTAs fit the device at once.
+struct PanelShape {
+    uint32_t threads, rowsPerThread;
+};
+template <class R> PanelShape panelShape(uint32_t rows, uint32_t B, uint32_t limit) {
+    const uint32_t sms = uint32_t(smCount());
+    PanelShape shape{256, 1};
+    const auto ctas = [&]() { return (rows + shape.threads * shape.rowsPerThread - 1) / (shape.threads * shape.rowsPerThread); };
+    if (ctas() > limit || B * ctas() > sms)
+        shape.threads = 512;
+    if (sizeof(R) == 4 && (ctas() > limit || B * ctas() > sms))
+        shape.rowsPerThread = 2;
+    return shape;
+}
+template <class R> uint32_t panelRegRows(uint32_t limit) { return limit * kPanelThreads * (sizeof(R) == 4 ? 2u : 1u); }
+
+// Largest cluster the panel kernels may use on this device: 16 CTAs (opt-in)
+// when the device can schedule such clusters with full shared memory, else the
+// portable 8, else one CTA.
 template <class R> uint32_t clusterLimitNow() {
-    const size_t smem = size_t(kPanel) * kClusterRows<R> * sizeof(C2<R>);
-    int limit = 0;
-    for (const void *kernel : {reinterpret_cast<const void *>(panelClusterKernel<R, 0>),
-                               reinterpret_cast<const void *>(panelClusterKernel<R, kGlobalSlots>)})
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
-            cudaGetLastError();
-            return 0;
-        }
-    for (uint32_t c : {kMaxCluster, 8u}) {
-        if (c > 8 && (cudaFuncSetAttribute(panelClusterKernel<R, 0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                          cudaSuccess ||
-                      cudaFuncSetAttribute(panelClusterKernel<R, kGlobalSlots>,
-                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
-            cudaGetLastError();
-            continue;
-        }
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(c, 1);
-        cfg.blockDim = dim3(1024);  // the largest launch: rows kept in global memory as well
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = c;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+    const auto fits = [](auto kernel, uint32_t c, uint32_t threads, size_t smem) {
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = clusterConfig(c, 1, threads, smem, nullptr, attr);
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, panelClusterKernel<R, kGlobalSlots>, &cfg) == cudaSuccess &&
-            clusters > 0) {
-            limit = int(c);
-            break;
-        }
-        cudaGetLastError();
+        const bool ok =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) == cudaSuccess &&
+            (c <= 8 || cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+        if (!ok)
+            cudaGetLastError();
+        return ok;
+    };
+    for (uint32_t c : {kMaxCluster, 8u, 1u}) {
+        bool ok = fits(panelRegKernel<R, 1>, c, kPanelThreads, panelRegSmem<R>(kPanelThreads)) &&
+                  (c == 1 || fits(panelClusterKernel<R>, c, 1024, kClusterSmem<R>));
+        if constexpr (sizeof(R) == 4)
+            ok = ok && fits(panelRegKernel<R, 2>, c, kPanelThreads, panelRegSmem<R>(2 * kPanelThreads));
+        if (ok)
+            return c;
     }
-    return uint32_t(limit);
+    throw std::runtime_error("LU panel kernel does not fit this device.");
 }
 template <class R> uint32_t clusterLimit() {
     static PerDeviceValue<uint32_t> limit;
@@ -1665,13 +1747,11 @@ template <class R> void factor(R *LU, uint32_t N, uint32_t B, int *pivots, int *
                                KernelTimer *timer, float *pack) {
     check(cudaMemsetAsync(info, 0, sizeof(int), stream), "LU info reset");
     const size_t gemmSmem = 2 * kPanel * 64 * sizeof(C2<R>);
+    int *moves = pivots + 2 * size_t(B) * N;
     static PerDeviceOnce attributes;
     attributes.run([&]() {
         check(cudaFuncSetAttribute(gemmKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemmSmem)),
               "gemm smem attribute");
-        check(cudaFuncSetAttribute(panelSmemKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(kPanelSmemLimit)),
-              "panel smem attribute");
         if constexpr (sizeof(R) == 4) {
             check(cudaFuncSetAttribute(trailingTensorKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem)),
                   "tensor update smem attribute");
@@ -1686,48 +1766,39 @@ template <class R> void factor(R *LU, uint32_t N, uint32_t B, int *pivots, int *
             const uint32_t jb = std::min(uint32_t(kPanel), end - k0);
             {
                 TimedScope s(timer, "lu_panel", stream);
-                const size_t bytes = panelSmemBytes<R>(N - k0, jb);
-                const uint32_t rows = N - k0;
-                const uint32_t limit = clusterLimit<R>();
-                if (sizeof(R) == 4 && jb == uint32_t(kPanel) && rows <= kRegPanelRows) {
-                    const uint32_t threads =
-                        std::max(32u, ((rows + kRegRowsPerThread - 1) / kRegRowsPerThread + 31) / 32 * 32);
-                    panelRegKernel<<<B, threads, 0, stream>>>(reinterpret_cast<float *>(LU), N, k0, pivots, info);
-                } else if (bytes > kPanelSmemLimit && rows <= limit * (kClusterRows<R> + kGlobalSlots * 1024u)) {
-                    // as few CTAs as hold the panel in shared memory, else the whole cluster with the
-                    // rows beyond kClusterRows per CTA kept in global memory
-                    const uint32_t C = std::min(limit, (rows + kClusterRows<R> - 1) / kClusterRows<R>);
-                    const uint32_t perBlock = (rows + C - 1) / C;
-                    const uint32_t cap = std::min(perBlock, kClusterRows<R>);
-                    cudaLaunchConfig_t cfg{};
-                    cfg.gridDim = dim3(C, B);
-                    cfg.blockDim = dim3(perBlock <= cap ? (perBlock + 31) / 32 * 32 : 1024u);
-                    cfg.dynamicSmemBytes = size_t(jb) * cap * sizeof(C2<R>);
-                    cfg.stream = stream;
-                    cudaLaunchAttribute attr[1];
-                    attr[0].id = cudaLaunchAttributeClusterDimension;
-                    attr[0].val.clusterDim.x = C;
-                    attr[0].val.clusterDim.y = 1;
-                    attr[0].val.clusterDim.z = 1;
-                    cfg.attrs = attr;
-                    cfg.numAttrs = 1;
-                    if (perBlock <= cap)
-                        check(cudaLaunchKernelEx(&cfg, panelClusterKernel<R, 0>, LU, N, k0, jb, perBlock, cap, pivots,
+                const uint32_t rows = N - k0, limit = clusterLimit<R>();
+                if (rows <= panelRegRows<R>(limit)) {  // rows in registers
+                    const PanelShape shape = panelShape<R>(rows, B, limit);
+                    const uint32_t perCta = shape.threads * shape.rowsPerThread;
+                    const uint32_t C = (rows + perCta - 1) / perCta, perBlock = (rows + C - 1) / C;
+                    cudaLaunchAttribute attr;
+                    const cudaLaunchConfig_t cfg =
+                        clusterConfig(C, B, shape.threads, panelRegSmem<R>(perBlock), stream, attr);
+                    if constexpr (sizeof(R) == 4) {
+                        const auto kernel = shape.rowsPerThread == 2 ? panelRegKernel<R, 2> : panelRegKernel<R, 1>;
+                        check(cudaLaunchKernelEx(&cfg, kernel, LU, N, k0, jb, perBlock, pivots, moves, info),
+                              "panel launch");
+                    } else
+                        check(cudaLaunchKernelEx(&cfg, panelRegKernel<R, 1>, LU, N, k0, jb, perBlock, pivots, moves,
                                                  info),
+                              "panel launch");
+                } else {
+                    const uint32_t perBlock = (rows + limit - 1) / limit, cap = std::min(perBlock, kClusterRows<R>);
+                    if (limit > 1 && rows <= limit * (kClusterRows<R> + kGlobalSlots * 1024u)) {
+                        cudaLaunchAttribute attr;
+                        const cudaLaunchConfig_t cfg =
+                            clusterConfig(limit, B, 1024, size_t(jb) * cap * sizeof(C2<R>), stream, attr);
+                        check(cudaLaunchKernelEx(&cfg, panelClusterKernel<R>, LU, N, k0, jb, perBlock, cap, pivots, info),
                               "cluster panel launch");
-                    else
-                        check(cudaLaunchKernelEx(&cfg, panelClusterKernel<R, kGlobalSlots>, LU, N, k0, jb, perBlock, cap,
-                                                 pivots, info),
-                              "cluster panel launch");
-                } else if (bytes <= kPanelSmemLimit)
-                    panelSmemKernel<R><<<B, std::min(1024u, (N - k0 + 31) / 32 * 32), bytes, stream>>>(
-                        LU, N, k0, jb, pivots, info);
-                else
-                    panelKernel<R><<<B, 512, 0, stream>>>(LU, N, k0, jb, pivots, info);
+                    } else
+                        panelKernel<R><<<B, 512, 0, stream>>>(LU, N, k0, jb, pivots, info);
+                    panelMovesKernel<<<B, 32, 0, stream>>>(pivots, N, k0, jb, moves);
+                }
             }
             {
                 TimedScope s(timer, "lu_swap", stream);
-                swapKernel<R><<<dim3((N + 127) / 128, B), 128, 0, stream>>>(LU, N, k0, jb, pivots);
+                constexpr uint32_t columns = 8 * kSwapColumns;
+                swapKernel<R><<<dim3((N + columns - 1) / columns, B), 256, 0, stream>>>(LU, N, k0, jb, moves);
             }
             const uint32_t cols = end - k0 - jb;  // columns of the outer block right of the panel
             if (cols) {
@@ -1902,7 +1973,7 @@ void debugLuFactor(bool fp32, uint32_t N, uint32_t B, const double *matrices, do
     check(cudaStreamSynchronize(stream), "LU hook");
 }
 
-size_t luWorkspaceBytes(uint32_t N, uint32_t B) { return 2 * size_t(B) * N * sizeof(int); }
+size_t luWorkspaceBytes(uint32_t N, uint32_t B) { return size_t(B) * (2 * size_t(N) + kMoves) * sizeof(int); }
 size_t luPackBytes(uint32_t N, uint32_t B) { return size_t(B) * packFloats(N) * sizeof(float); }
 
 }  // namespace hsb

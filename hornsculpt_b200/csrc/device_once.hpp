@@ -80,4 +80,15 @@ class PerDeviceHighWater {
     size_t level_[256] = {};
 };
 
+// Multiprocessors of the current device.
+inline int smCount() {
+    static PerDeviceValue<int> count;
+    return count.get([]() {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, currentDevice()) != cudaSuccess || n <= 0)
+            n = 148;
+        return n;
+    });
+}
+
 }  // namespace hsb
