@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(256) trsmKernel(R *LU, uint32_t N, uint32_t k0
     }
 }
 
-// A22 -= L21 * U12 with 64x64 output tiles, K = jb <= 32, over rows
+// FP32: A22 -= L21 * U12 with 64x64 output tiles, K = jb <= 32, over rows
 // [k0 + jb, N) and columns [k0 + jb, cEnd).
 template <class R>
 __global__ void __launch_bounds__(256) gemmKernel(R *LU, uint32_t N, uint32_t k0, uint32_t jb, uint32_t cEnd) {
@@ -976,6 +976,140 @@ __global__ void __launch_bounds__(256) gemmKernel(R *LU, uint32_t N, uint32_t k0
             if (r < N && c < cEnd)
                 st2(M + 2 * (size_t(c) * N + r), mk<R>(old[i][j].x - acc[i][j].x, old[i][j].y - acc[i][j].y));
         }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 update C -= L U (complex, K = kPanel or kOuter64 columns of L) on the
+// FP64 matrix instruction (mma.sync m8n8k4; tcgen05 has no FP64 kind).
+//
+// Bound: at K = 96 a 64 x 64 tile is 1.57 M fused operations against 128 KB of
+// C and 192 KB of operands, so the FP64 pipe (24.6 k cycles per tile on one SM)
+// leads the memory by more than a factor of two; at K = 32 they tie, which is why
+// the factorisation has two levels. A warp owns 4 x 4 (or 2 x 2) blocks of 8 x 8
+// outputs, real and imaginary accumulators in registers, starting from C
+// itself. Operands come in stages of 16 columns by cp.async into two buffers,
+// as complex pairs: one 16-byte load gives a fragment's real and imaginary part,
+// and 8 loads feed 64 matrix instructions. Leading dimensions of 2 (L) and 4 (U)
+// modulo 8 entries make both fragment reads free of bank conflicts. Three CTAs
+// per SM: a tile's loads of C and its stores overlap the others' products (two
+// left the matrix pipe at 51 %, waiting for C).
+//
+// Tile 64 x 64, or 32 x 32 where 64 x 64 tiles would leave SMs idle.
+// Measured, all updates of a factorisation, against one level of K = 32 updates
+// with FP64 fused multiply-adds: N = 6380 65.2 -> 25.3 ms (outer block 64: 28.0;
+// two CTAs per SM: 39.2), N = 2562 x 2 9.2 -> 4.0, N = 642 x 32 2.56 -> 1.11,
+// N = 258 0.137 -> 0.077
+// ---------------------------------------------------------------------------
+constexpr int kStageK = 16;
+constexpr int kOuter64 = 96;  // outer block width of the FP64 factorisation
+
+__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+// 16 bytes from global to shared memory, zeros when `valid` is false
+__device__ __forceinline__ void copyEntry(double2 *dst, const double *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(valid ? 16 : 0));
+}
+
+template <int TILE>
+constexpr size_t kGemm64Smem = 2 * (kStageK * (TILE + 2) + TILE * (kStageK + 4)) * sizeof(double2);  // 73 KB at 64
+
+// Rows [r0, N), columns [c0, cEnd), inner columns [k0, k0 + K): C(r, c) -= sum_k M(r, k) M(k, c). K is a
+// multiple of kStageK.
+template <int TILE>
+__global__ void __launch_bounds__(128, TILE == 64 ? 3 : 4) gemm64Kernel(double *LU, uint32_t N, uint32_t k0, uint32_t K,
+                                                                       uint32_t r0, uint32_t c0, uint32_t cEnd) {
+    constexpr int LDA = TILE + 2, LDB = kStageK + 4, W = TILE / 16;  // W x W blocks of 8 x 8 per warp
+    extern __shared__ __align__(16) unsigned char rawSmem[];
+    double2 *const sA = reinterpret_cast<double2 *>(rawSmem);  // two buffers [k][row]
+    double2 *const sB = sA + 2 * kStageK * LDA;                // two buffers [column][k]
+    double *M = LU + size_t(blockIdx.z) * N * N * 2;
+    const uint32_t row0 = r0 + blockIdx.x * TILE, col0 = c0 + blockIdx.y * TILE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wr = (warp & 1) * (TILE / 2), wc = (warp >> 1) * (TILE / 2);  // the warp's corner in the tile
+    const auto stage = [&](int buffer, uint32_t k) {
+        for (int e = threadIdx.x; e < kStageK * TILE; e += 128) {
+            const int kk = e / TILE, x = e % TILE;
+            const bool inside = row0 + x < N;
+            copyEntry(sA + buffer * kStageK * LDA + kk * LDA + x, M + 2 * (size_t(k + kk) * N + (inside ? row0 + x : 0)), inside);
+        }
+        for (int e = threadIdx.x; e < kStageK * TILE; e += 128) {
+            const int c = e / kStageK, kk = e % kStageK;
+            const bool inside = col0 + c < cEnd;
+            copyEntry(sB + buffer * TILE * LDB + c * LDB + kk, M + 2 * (size_t(inside ? col0 + c : 0) * N + k + kk), inside);
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+    stage(0, k0);
+    // accumulators: block (i, j) holds rows wr + 8i + lane / 4, columns wc + 8j + 2 (lane % 4) + {0, 1}
+    double re[W][W][2], im[W][W][2];
+    const uint32_t row = row0 + wr + lane / 4, col = col0 + wc + 2 * (lane % 4);
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t r = row + 8 * i, c = col + 8 * j + h;
+                const double2 v = r < N && c < cEnd ? ld2(M + 2 * (size_t(c) * N + r)) : make_double2(0, 0);
+                re[i][j][h] = v.x;
+                im[i][j][h] = v.y;
+            }
+    const int stages = int(K) / kStageK;
+    for (int s = 0; s < stages; ++s) {
+        if (s + 1 < stages) {
+            stage((s + 1) & 1, k0 + (s + 1) * kStageK);
+            asm volatile("cp.async.wait_group 1;");
+        } else
+            asm volatile("cp.async.wait_group 0;");
+        __syncthreads();
+        const double2 *A = sA + (s & 1) * kStageK * LDA + (lane % 4) * LDA + wr + lane / 4;
+        const double2 *B = sB + (s & 1) * TILE * LDB + (wc + lane / 4) * LDB + lane % 4;
+#pragma unroll
+        for (int kk = 0; kk < kStageK; kk += 4) {
+            double2 a[W], b[W];
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                a[i] = A[kk * LDA + 8 * i];
+                b[i] = B[8 * i * LDB + kk];
+            }
+            // four sweeps over the blocks: consecutive instructions have different accumulators
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    mma884(re[i][j], -a[i].x, b[j].x);
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    mma884(im[i][j], -a[i].x, b[j].y);
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    mma884(re[i][j], a[i].y, b[j].y);
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    mma884(im[i][j], -a[i].y, b[j].x);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t r = row + 8 * i, c = col + 8 * j + h;
+                if (r < N && c < cEnd)
+                    st2(M + 2 * (size_t(c) * N + r), make_double2(re[i][j][h], im[i][j][h]));
+            }
 }
 
 // ---------------------------------------------------------------------------
@@ -1260,47 +1394,47 @@ __global__ void __launch_bounds__(kTcThreads, 1) trailingTensorKernel(float *LU,
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NB));
 }
 
-// U12 = L11^{-1} A12 for the outer block (L11: the kOuter x kOuter unit lower
-// triangle at (K0, K0)), over the trailing columns [K0 + kOuter, N). L11 is
+// U12 = L11^{-1} A12 for the outer block (L11: the OUTER x OUTER unit lower
+// triangle at (K0, K0)), over the trailing columns [K0 + OUTER, N). L11 is
 // staged in shared memory column by column (coalesced); a warp solves one
-// column at a time with lane l holding rows l, l + 32, l + 64, l + 96 in
-// registers and the solved unknown broadcast by shuffle.
+// column at a time with lane l holding rows l, l + 32, ... in registers and the
+// solved unknown broadcast by shuffle. FP32 at OUTER = 128, FP64 at 96.
 constexpr int kTrsmColumns = 64, kTrsmThreads = 512;
-constexpr size_t kTrsmSmem = size_t(kOuter) * kOuter * sizeof(float2);  // 128 KB
+template <class R> constexpr int kOuterOf = sizeof(R) == 4 ? kOuter : kOuter64;
+template <class R> constexpr size_t kTrsmSmem = size_t(kOuterOf<R>) * kOuterOf<R> * sizeof(C2<R>);  // 128 KB, 144 KB
 
-__global__ void __launch_bounds__(kTrsmThreads, 1) trsmBlockKernel(float *LU, uint32_t N, uint32_t K0) {
-    extern __shared__ __align__(16) float2 Lc[];  // [column m][row]
-    float *M = LU + size_t(blockIdx.y) * N * N * 2;
-    for (uint32_t e = threadIdx.x; e < uint32_t(kOuter * kOuter); e += blockDim.x) {
-        const uint32_t r = e % kOuter, m = e / kOuter;
-        Lc[e] = *reinterpret_cast<const float2 *>(M + 2 * (size_t(K0 + m) * N + K0 + r));
+template <class R>
+__global__ void __launch_bounds__(kTrsmThreads, 1) trsmBlockKernel(R *LU, uint32_t N, uint32_t K0, uint32_t columns) {
+    constexpr int OUTER = kOuterOf<R>, S = OUTER / 32;
+    extern __shared__ __align__(16) unsigned char rawSmem[];
+    C2<R> *Lc = reinterpret_cast<C2<R> *>(rawSmem);  // [column m][row]
+    R *M = LU + size_t(blockIdx.y) * N * N * 2;
+    for (uint32_t e = threadIdx.x; e < uint32_t(OUTER * OUTER); e += blockDim.x) {
+        const uint32_t r = e % OUTER, m = e / OUTER;
+        Lc[e] = ld2(M + 2 * (size_t(K0 + m) * N + K0 + r));
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t c0 = K0 + kOuter + blockIdx.x * kTrsmColumns;
-    for (uint32_t c = c0 + warp; c < min(N, c0 + kTrsmColumns); c += kTrsmThreads / 32) {
-        float2 *col = reinterpret_cast<float2 *>(M + 2 * (size_t(c) * N + K0));
-        float2 v[4];
+    const uint32_t c0 = K0 + OUTER + blockIdx.x * columns;
+    for (uint32_t c = c0 + warp; c < min(N, c0 + columns); c += blockDim.x / 32) {
+        C2<R> *col = reinterpret_cast<C2<R> *>(M + 2 * (size_t(c) * N + K0));
+        C2<R> v[S];
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
+        for (int s = 0; s < S; ++s)
             v[s] = col[lane + 32 * s];
 #pragma unroll
-        for (int sb = 0; sb < 4; ++sb)
+        for (int sb = 0; sb < S; ++sb)
 #pragma unroll 8
             for (int mm = 0; mm < 32; ++mm) {
                 const int m = 32 * sb + mm;
-                const float2 x =
-                    make_float2(__shfl_sync(0xffffffffu, v[sb].x, mm), __shfl_sync(0xffffffffu, v[sb].y, mm));
+                const C2<R> x = mk<R>(__shfl_sync(0xffffffffu, v[sb].x, mm), __shfl_sync(0xffffffffu, v[sb].y, mm));
 #pragma unroll
-                for (int s = sb; s < 4; ++s)
-                    if (lane + 32 * s > m) {
-                        const float2 a = Lc[m * kOuter + lane + 32 * s];
-                        v[s].x -= a.x * x.x - a.y * x.y;
-                        v[s].y -= a.x * x.y + a.y * x.x;
-                    }
+                for (int s = sb; s < S; ++s)
+                    if (lane + 32 * s > m)
+                        csub<R>(v[s], Lc[m * OUTER + lane + 32 * s], x);
             }
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
+        for (int s = 0; s < S; ++s)
             col[lane + 32 * s] = v[s];
     }
 }
@@ -1736,13 +1870,28 @@ template <class R> uint32_t clusterLimit() {
     return limit.get([]() { return clusterLimitNow<R>(); });
 }
 
-// Right-looking LU with partial pivoting, 32-wide panels. FP64 runs one
-// level: every panel updates the whole trailing matrix (K = 32). FP32 runs two
-// levels: panels update only the rest of their kOuter-wide outer block, then
-// the outer block's U12 is solved (trsmBlockKernel) and the trailing matrix is
-// updated once with K = kOuter on the tensor cores (trailingTensorKernel).
-// Pivot choices follow the same rule in both; only the order of the update
-// sums differs.
+// C -= L U of the FP64 factorisation over rows and columns from `from` on, up to column cEnd.
+void launchGemm64(double *LU, uint32_t N, uint32_t B, uint32_t k0, uint32_t K, uint32_t cEnd, cudaStream_t stream) {
+    const uint32_t from = k0 + K, rows = N - from, cols = cEnd - from;
+    const auto tiles = [&](uint32_t t) { return dim3((rows + t - 1) / t, (cols + t - 1) / t, B); };
+    const dim3 wide = tiles(64);
+    if (size_t(wide.x) * wide.y * B >= size_t(smCount()))
+        gemm64Kernel<64><<<wide, 128, kGemm64Smem<64>, stream>>>(LU, N, k0, K, from, from, cEnd);
+    else
+        gemm64Kernel<32><<<tiles(32), 128, kGemm64Smem<32>, stream>>>(LU, N, k0, K, from, from, cEnd);
+}
+
+// Columns per CTA of trsmBlockKernel: kTrsmColumns, or one per warp where that would leave most SMs idle.
+template <class R> uint32_t trsmColumns(uint32_t rest, uint32_t B) {
+    const uint32_t wide = uint32_t(kTrsmColumns);
+    return size_t((rest + wide - 1) / wide) * B >= size_t(smCount()) ? wide : kTrsmThreads / 32;
+}
+
+// Right-looking LU with partial pivoting, 32-wide panels, two levels: panels
+// update only the rest of their outer block (FP32: kOuter columns, FP64:
+// kOuter64), then the outer block's U12 is solved (trsmBlockKernel) and the
+// trailing matrix is updated once with K = the block's width, in FP32 on the
+// tensor cores (trailingTensorKernel), in FP64 by gemm64Kernel.
 template <class R> void factor(R *LU, uint32_t N, uint32_t B, int *pivots, int *info, cudaStream_t stream,
                                KernelTimer *timer, float *pack) {
     check(cudaMemsetAsync(info, 0, sizeof(int), stream), "LU info reset");
@@ -1750,16 +1899,20 @@ template <class R> void factor(R *LU, uint32_t N, uint32_t B, int *pivots, int *
     int *moves = pivots + 2 * size_t(B) * N;
     static PerDeviceOnce attributes;
     attributes.run([&]() {
-        check(cudaFuncSetAttribute(gemmKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemmSmem)),
-              "gemm smem attribute");
+        check(cudaFuncSetAttribute(trsmBlockKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTrsmSmem<R>)),
+              "block trsm smem attribute");
         if constexpr (sizeof(R) == 4) {
+            check(cudaFuncSetAttribute(gemmKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemmSmem)),
+                  "gemm smem attribute");
             check(cudaFuncSetAttribute(trailingTensorKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem)),
                   "tensor update smem attribute");
-            check(cudaFuncSetAttribute(trsmBlockKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTrsmSmem)),
-                  "block trsm smem attribute");
+        } else {
+            check(cudaFuncSetAttribute(gemm64Kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(kGemm64Smem<64>)),
+                  "gemm smem attribute");
         }
     });
-    const uint32_t outer = sizeof(R) == 4 ? uint32_t(kOuter) : N;
+    constexpr uint32_t outer = uint32_t(kOuterOf<R>);
     for (uint32_t K0 = 0; K0 < N; K0 += outer) {
         const uint32_t end = std::min(N, K0 + outer);
         for (uint32_t k0 = K0; k0 < end; k0 += kPanel) {
@@ -1807,32 +1960,39 @@ template <class R> void factor(R *LU, uint32_t N, uint32_t B, int *pivots, int *
                     trsmKernel<R><<<dim3((cols + kPanel - 1) / kPanel, B), 256, 0, stream>>>(LU, N, k0, jb, end);
                 }
                 TimedScope s(timer, "lu_gemm", stream);
-                const uint32_t rows = N - k0 - jb;
-                gemmKernel<R><<<dim3((rows + 63) / 64, (cols + 63) / 64, B), 256, gemmSmem, stream>>>(LU, N, k0, jb,
-                                                                                                      end);
+                if constexpr (sizeof(R) == 4) {
+                    const uint32_t rows = N - k0 - jb;
+                    gemmKernel<R><<<dim3((rows + 63) / 64, (cols + 63) / 64, B), 256, gemmSmem, stream>>>(LU, N, k0, jb,
+                                                                                                          end);
+                } else
+                    launchGemm64(LU, N, B, k0, jb, end, stream);
             }
             check(cudaGetLastError(), "LU launch");
         }
-        if constexpr (sizeof(R) == 4) {
-            if (end < N) {
-                const uint32_t rest = N - end;
-                {
-                    TimedScope s(timer, "lu_trsm_outer", stream);
-                    trsmBlockKernel<<<dim3((rest + kTrsmColumns - 1) / kTrsmColumns, B), kTrsmThreads, kTrsmSmem,
-                                      stream>>>(LU, N, K0);
-                }
-                const uint32_t rowTiles = (rest + kTcRows - 1) / kTcRows, colTiles = (rest + kTcCols - 1) / kTcCols;
-                const size_t packStride = packFloats(N);
-                {
-                    TimedScope s(timer, "lu_pack", stream);
-                    packKernel<<<dim3(rowTiles + colTiles, kTcSteps, B), 256, 0, stream>>>(LU, N, K0, pack, packStride);
-                }
-                TimedScope s(timer, "lu_gemm_tensor", stream);
-                trailingTensorKernel<<<dim3(rowTiles, colTiles, B), kTcThreads, kTcSmem, stream>>>(LU, N, K0, pack,
-                                                                                                    packStride, info);
-                check(cudaGetLastError(), "LU outer update launch");
-            }
+        if (end == N)
+            break;
+        const uint32_t rest = N - end;
+        {
+            TimedScope s(timer, "lu_trsm_outer", stream);
+            const uint32_t columns = trsmColumns<R>(rest, B);
+            trsmBlockKernel<R><<<dim3((rest + columns - 1) / columns, B), kTrsmThreads, kTrsmSmem<R>, stream>>>(
+                LU, N, K0, columns);
         }
+        if constexpr (sizeof(R) == 4) {
+            const uint32_t rowTiles = (rest + kTcRows - 1) / kTcRows, colTiles = (rest + kTcCols - 1) / kTcCols;
+            const size_t packStride = packFloats(N);
+            {
+                TimedScope s(timer, "lu_pack", stream);
+                packKernel<<<dim3(rowTiles + colTiles, kTcSteps, B), 256, 0, stream>>>(LU, N, K0, pack, packStride);
+            }
+            TimedScope s(timer, "lu_gemm_tensor", stream);
+            trailingTensorKernel<<<dim3(rowTiles, colTiles, B), kTcThreads, kTcSmem, stream>>>(LU, N, K0, pack,
+                                                                                                packStride, info);
+        } else {
+            TimedScope s(timer, "lu_gemm", stream);
+            launchGemm64(LU, N, B, K0, outer, N, stream);
+        }
+        check(cudaGetLastError(), "LU outer update launch");
     }
 }
 
