@@ -1439,114 +1439,76 @@ __global__ void __launch_bounds__(kTrsmThreads, 1) trsmBlockKernel(R *LU, uint32
     }
 }
 
-// Forward / back substitution of one right-hand side per CTA, with the
-// vector staged in shared memory. Blocks of 32 unknowns: warp 0 loads the
-// 32x32 diagonal block into registers (independent coalesced loads, lane =
-// row) and solves it with shuffles; then every thread updates its rows with
-// the block's 32 columns.
-template <class R>
-__global__ void __launch_bounds__(sizeof(R) == 8 ? 256 : 512) solveKernel(const R *LU, const int *pivots, uint32_t N, uint32_t E, R *X) {
-    extern __shared__ __align__(16) unsigned char rawSmem[];
-    C2<R> *x = reinterpret_cast<C2<R> *>(rawSmem);
-    const uint32_t e = blockIdx.x, f = blockIdx.y;
-    const R *M = LU + size_t(f) * N * N * 2;
-    // the factorisation's row interchanges, composed into one permutation
-    // (stored after the batch's interchange sequences): a parallel gather
-    const int *perm = pivots + (size_t(gridDim.y) + f) * N;
-    R *out = X + (size_t(f) * E + e) * N * 2;
-    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x)
-        x[i] = ld2(out + 2 * perm[i]);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const C2<R> zero = mk<R>(0, 0);
-    // forward: unit lower triangle
-    for (uint32_t k = 0; k < N; k += 32) {
-        const uint32_t kb = min(32u, N - k);
-        if (warp == 0) {
-            C2<R> L[32];
-#pragma unroll
-            for (int m = 0; m < 32; ++m)
-                L[m] = (m < int(kb) && lane < int(kb)) ? ld2(M + 2 * (size_t(k + m) * N + k + lane)) : zero;
-            C2<R> mine = lane < int(kb) ? x[k + lane] : zero;
-#pragma unroll
-            for (int m = 0; m < 32; ++m) {
-                const C2<R> xm = mk<R>(__shfl_sync(0xffffffffu, mine.x, m), __shfl_sync(0xffffffffu, mine.y, m));
-                if (lane > m)
-                    csub<R>(mine, L[m], xm);
-            }
-            if (lane < int(kb))
-                x[k + lane] = mine;
-        }
-        __syncthreads();
-        if (kb == 32) {
-            for (uint32_t i = k + 32 + threadIdx.x; i < N; i += blockDim.x) {
-                C2<R> v = x[i];
-#pragma unroll
-                for (int m = 0; m < 32; ++m)
-                    csub<R>(v, ld2(M + 2 * (size_t(k + m) * N + i)), x[k + m]);
-                x[i] = v;
-            }
-        }
-        __syncthreads();
-    }
-    // backward: upper triangle with its diagonal
-    const uint32_t blocks = (N + 31) / 32;
-    for (uint32_t bi = blocks; bi-- > 0;) {
-        const uint32_t k = bi * 32, kb = min(32u, N - k);
-        if (warp == 0) {
-            C2<R> U[32];
-#pragma unroll
-            for (int m = 0; m < 32; ++m)
-                U[m] = (m < int(kb) && lane < int(kb)) ? ld2(M + 2 * (size_t(k + m) * N + k + lane)) : zero;
-            C2<R> mine = lane < int(kb) ? x[k + lane] : zero;
-#pragma unroll
-            for (int m = 31; m >= 0; --m) {
-                if (m < int(kb)) {
-                    if (lane == m) {
-                        const C2<R> d = U[m];
-                        const R den = d.x * d.x + d.y * d.y;
-                        mine = mk<R>((mine.x * d.x + mine.y * d.y) / den, (mine.y * d.x - mine.x * d.y) / den);
-                    }
-                    const C2<R> xm = mk<R>(__shfl_sync(0xffffffffu, mine.x, m), __shfl_sync(0xffffffffu, mine.y, m));
-                    if (lane < m)
-                        csub<R>(mine, U[m], xm);
-                }
-            }
-            if (lane < int(kb))
-                x[k + lane] = mine;
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) {
-            C2<R> v = x[i];
-            if (kb == 32) {
-#pragma unroll
-                for (int m = 0; m < 32; ++m)
-                    csub<R>(v, ld2(M + 2 * (size_t(k + m) * N + i)), x[k + m]);
-            } else {
-                for (uint32_t m = 0; m < kb; ++m)
-                    csub<R>(v, ld2(M + 2 * (size_t(k + m) * N + i)), x[k + m]);
-            }
-            x[i] = v;
-        }
-        __syncthreads();
-    }
-    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x)
-        st2(out + 2 * i, x[i]);
+// Blocked triangular solves. The row interchanges of a factorisation are
+// composed once into a permutation (permutationKernel, stored after the
+// interchanges), so a solve starts with a parallel gather of the right-hand
+// side into a work vector. The 32 x 32 diagonal blocks of both triangles are
+// inverted once per factorisation (diagonalInverseKernel, stored after the
+// permutations). Forward and backward substitution then run in blocks of
+// kTriBlock unknowns, one launch per block: CTA 0 brings the next block's rows
+// up to date with the block solved last and solves the next diagonal block; the
+// other CTAs apply the block solved last to every remaining row. The backward
+// sweep writes each solved block to the output vector.
+//
+// Bound: the chain of blocks. Everything CTA 0 needs is in flight from its
+// first instruction (the diagonal block by cp.async, 32 column loads per
+// thread), a 32 x 32 sub-block is one matrix-vector product with its inverse
+// instead of 32 dependent steps of shuffles (and divisions, backward), and
+// partial sums stay in the thread that owns their row and columns until their
+// sub-block is next. Measured per solve against shuffled sub-blocks loaded when
+// their turn came (one CTA per system up to N = 1024): FP32 N = 6380 3.2 -> 1.0
+// ms, N = 4023 x 3 2.1 -> 0.65, N = 642 x 32 0.25 -> 0.125; FP64 N = 6380
+// 4.2 -> 1.5, N = 2562 x 2 1.7 -> 0.62, N = 258 0.117 -> 0.065.
+constexpr uint32_t kTriBlock = 128, kSub = 32;
+constexpr uint32_t kTriThreads = 512;                  // 128 rows x 4 column groups
+constexpr uint32_t kTriGroups = kTriThreads / kTriBlock;
+constexpr uint32_t kTriSubs = kTriBlock / kSub;
+// shared memory of CTA 0: the sub-blocks of one triangle of the diagonal block (inverses on the diagonal)
+template <class R> constexpr size_t kTriSmem = size_t(kTriSubs * (kTriSubs + 1) / 2) * kSub * kSub * sizeof(C2<R>);
+
+// Complex entries of the inverses of one triangle of one matrix, and where they start in the pivot buffer.
+__host__ __device__ inline size_t inverseEntries(uint32_t N) { return size_t((N + kSub - 1) / kSub) * kSub * kSub; }
+__host__ __device__ inline size_t inverseOffset(uint32_t N, uint32_t B) {  // in ints, 16-byte aligned
+    return (size_t(B) * (2 * size_t(N) + kMoves) + 3) / 4 * 4;
+}
+template <class R> __host__ __device__ const C2<R> *inverses(const int *pivots, uint32_t N, uint32_t B, uint32_t f, bool lower) {
+    return reinterpret_cast<const C2<R> *>(pivots + inverseOffset(N, B)) + (2 * size_t(f) + (lower ? 0 : 1)) * inverseEntries(N);
 }
 
-// Blocked triangular solves for many CTAs. The row interchanges of a
-// factorisation are composed once into a permutation (permutationKernel,
-// stored after the interchanges), so a solve starts with a parallel gather of
-// the right-hand side into a work vector. Forward and backward substitution
-// then run in blocks of kTriBlock unknowns, one launch per block: CTA 0 brings
-// the next block's rows up to date with the block solved last and solves the
-// next diagonal block (32 x 32 sub-blocks in warp 0's registers, as in
-// solveKernel); the other CTAs apply the block solved last to every remaining
-// row (64 rows x 4 column groups of 32 per CTA, coalesced column reads, the four
-// partial sums added in a fixed order). The backward sweep writes each solved
-// block to the output vector.
-constexpr uint32_t kTriBlock = 128, kTriRows = 64;
-constexpr uint32_t kSmallSolve = 1024;  // up to this N the one-CTA-per-system kernel is faster
+// Inverses of the 32 x 32 diagonal blocks (blockIdx.x) of both triangles
+// (blockIdx.z) of each matrix: lane c solves for column c of the inverse,
+// rows stored contiguously. Rows past N are those of the identity.
+template <class R>
+__global__ void __launch_bounds__(32) diagonalInverseKernel(const R *LU, uint32_t N, int *pivots, uint32_t B) {
+    __shared__ C2<R> D[kSub][kSub + 1];  // [row][column]
+    const uint32_t f = blockIdx.y, k = blockIdx.x * kSub;
+    const bool lower = blockIdx.z == 0;
+    const int lane = threadIdx.x;
+    const R *M = LU + size_t(f) * N * N * 2;
+    for (int c = 0; c < int(kSub); ++c)
+        D[lane][c] = k + lane < N && k + c < N ? ld2(M + 2 * (size_t(k + c) * N + k + lane)) : mk<R>(lane == c ? 1 : 0, 0);
+    __syncwarp();
+    if (!lower) {  // reciprocal diagonal
+        const C2<R> d = D[lane][lane];
+        const R den = d.x * d.x + d.y * d.y;
+        D[lane][lane] = mk<R>(d.x / den, -d.y / den);
+        __syncwarp();
+    }
+    C2<R> x[kSub];
+#pragma unroll
+    for (int q = 0; q < int(kSub); ++q) {
+        const int i = lower ? q : int(kSub) - 1 - q;
+        C2<R> v = mk<R>(i == lane ? 1 : 0, 0);
+#pragma unroll
+        for (int p = 0; p < q; ++p)
+            csub<R>(v, D[i][lower ? p : int(kSub) - 1 - p], x[p]);
+        x[q] = lower ? v : cmul<R>(v, D[i][i]);
+    }
+    C2<R> *out = const_cast<C2<R> *>(inverses<R>(pivots, N, B, f, lower)) + size_t(blockIdx.x) * kSub * kSub;
+#pragma unroll
+    for (int q = 0; q < int(kSub); ++q)
+        out[(lower ? q : int(kSub) - 1 - q) * kSub + lane] = x[q];
+}
 
 __global__ void permutationKernel(const int *pivots, uint32_t N, int *perm) {
     extern __shared__ int p[];  // [N] the permutation, [N] the interchange sequence
@@ -1579,54 +1541,94 @@ template <class R> __global__ void gatherRhsKernel(const R *x, const int *perm, 
     st2(work + 2 * (v + i), ld2(x + 2 * (v + perm[size_t(f) * N + i])));
 }
 
+// v + a * b, and v = sum of the products of one thread
+template <class R> __device__ __forceinline__ void cadd(C2<R> &v, C2<R> a, C2<R> b) {
+    v.x = fma(-a.y, b.y, fma(a.x, b.x, v.x));
+    v.y = fma(a.y, b.x, fma(a.x, b.y, v.y));
+}
+// one complex value from global to shared memory without a register
+template <class R> __device__ __forceinline__ void copyAsync(C2<R> *dst, const R *src) {
+    const uint32_t to = uint32_t(__cvta_generic_to_shared(dst));
+    if constexpr (sizeof(R) == 8)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src));
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(src));
+}
+
 // One step of a sweep. Known block: unknowns [c0, c0 + cw) (cw = 0 on the first step); next block
 // [n0, n0 + nw). Forward (Lower): unit lower triangle, updated rows [n0 + nw, N). Backward: upper
 // triangle with its diagonal, updated rows [0, n0).
 template <class R, bool Lower>
-__global__ void __launch_bounds__(256) triStepKernel(const R *LU, uint32_t N, uint32_t E, R *work, R *out, uint32_t c0,
-                                                     uint32_t cw, uint32_t n0, uint32_t nw) {
+__global__ void __launch_bounds__(kTriThreads) triStepKernel(const R *LU, const int *pivots, uint32_t N, uint32_t E,
+                                                             R *work, R *out, uint32_t c0, uint32_t cw, uint32_t n0,
+                                                             uint32_t nw) {
+    extern __shared__ __align__(16) unsigned char rawSmem[];
     __shared__ C2<R> y[kTriBlock];
-    __shared__ C2<R> part[4][kTriBlock];
-    __shared__ C2<R> v[kTriBlock];
+    __shared__ C2<R> part[kTriGroups][kTriBlock];
     const uint32_t e = blockIdx.y, f = blockIdx.z, tid = threadIdx.x;
+    const uint32_t i = tid % kTriBlock, g = tid / kTriBlock;  // this thread's row and column group
     const R *M = LU + size_t(f) * N * N * 2;
     R *w = work + (size_t(f) * E + e) * N * 2;
     const C2<R> zero = mk<R>(0, 0);
-    for (uint32_t i = tid; i < cw; i += blockDim.x)
-        y[i] = ld2(w + 2 * (c0 + i));
-    __syncthreads();
-    if (blockIdx.x > 0) {  // rows outside the next block
-        const uint32_t i = tid % kTriRows, g = tid / kTriRows;
-        const uint32_t r = (Lower ? n0 + nw : 0) + (blockIdx.x - 1) * kTriRows + i;
-        const uint32_t rEnd = Lower ? N : n0;
-        C2<R> acc = zero;
-        if (r < rEnd) {
-            if (cw == kTriBlock) {  // full block: the 32 column loads in flight together
-                C2<R> a[32];
-#pragma unroll
-                for (int c = 0; c < 32; ++c)
-                    a[c] = ld2(M + 2 * (size_t(c0 + 32 * g + c) * N + r));
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const C2<R> b = y[32 * g + c];
-                    acc.x += a[c].x * b.x - a[c].y * b.y;
-                    acc.y += a[c].x * b.y + a[c].y * b.x;
+    const bool solver = blockIdx.x == 0;
+    const uint32_t r = solver ? n0 + i : (Lower ? n0 + nw : 0) + (blockIdx.x - 1) * kTriBlock + i;
+    const bool mine = solver ? i < nw : r < (Lower ? N : n0);
+    // sub-block (p, q) of the diagonal block, p >= q forward, p <= q backward, in steps of the sweep:
+    // step index s = p forward, last - p backward
+    C2<R> *const D = reinterpret_cast<C2<R> *>(rawSmem);
+    const uint32_t subs = (nw + kSub - 1) / kSub;
+    const auto subBlock = [&](uint32_t row, uint32_t column) {  // by sweep order, column <= row
+        return D + (row * (row + 1) / 2 + column) * kSub * kSub;
+    };
+    const auto subAt = [&](uint32_t s) { return Lower ? s : subs - 1 - s; };  // sub-block solved in step s
+    if (solver) {
+        const C2<R> *inverse = inverses<R>(pivots, N, gridDim.z, f, Lower) + size_t(n0 / kSub) * kSub * kSub;
+        for (uint32_t a = 0; a < subs; ++a)
+            for (uint32_t b = 0; b <= a; ++b) {
+                C2<R> *block = subBlock(a, b);
+                if (a == b) {  // [row][column]
+                    for (uint32_t x = tid; x < kSub * kSub; x += kTriThreads)
+                        copyAsync<R>(block + x, reinterpret_cast<const R *>(inverse + size_t(subAt(a)) * kSub * kSub + x));
+                    continue;
                 }
-            } else {
-                const uint32_t cEnd = min(cw, 32 * g + 32);
-                for (uint32_t c = 32 * g; c < cEnd; ++c) {
-                    const C2<R> a = ld2(M + 2 * (size_t(c0 + c) * N + r)), b = y[c];
-                    acc.x += a.x * b.x - a.y * b.y;
-                    acc.y += a.x * b.y + a.y * b.x;
+                for (uint32_t x = tid; x < kSub * kSub; x += kTriThreads) {  // [column][row]
+                    const uint32_t row = kSub * subAt(a) + x % kSub, column = kSub * subAt(b) + x / kSub;
+                    if (row < nw && column < nw)
+                        copyAsync<R>(block + x, M + 2 * (size_t(n0 + column) * N + n0 + row));
+                    else
+                        block[x] = zero;
                 }
             }
+        asm volatile("cp.async.commit_group;");
+    }
+    // this row's products with the block solved last: 32 column loads in flight (FP64: 16)
+    C2<R> acc = zero;
+    if (cw) {
+        constexpr uint32_t kLoads = sizeof(R) == 8 ? kSub / 2 : kSub;
+        C2<R> a[kLoads];
+        const uint32_t first = kSub * g;
+#pragma unroll
+        for (uint32_t h = 0; h < kSub; h += kLoads) {
+#pragma unroll
+            for (uint32_t c = 0; c < kLoads; ++c)
+                a[c] = mine && first + h + c < cw ? ld2(M + 2 * (size_t(c0 + first + h + c) * N + r)) : zero;
+            if (h == 0) {
+                for (uint32_t x = tid; x < kTriBlock; x += kTriThreads)
+                    y[x] = x < cw ? ld2(w + 2 * (c0 + x)) : zero;
+                __syncthreads();
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < kLoads; ++c)
+                cadd<R>(acc, a[c], y[first + h + c]);
         }
+    }
+    if (!solver) {
         part[g][i] = acc;
         __syncthreads();
-        if (g == 0 && r < rEnd) {
+        if (g == 0 && mine) {
             C2<R> t = ld2(w + 2 * r);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (uint32_t q = 0; q < kTriGroups; ++q) {
                 t.x -= part[q][i].x;
                 t.y -= part[q][i].y;
             }
@@ -1634,88 +1636,55 @@ __global__ void __launch_bounds__(256) triStepKernel(const R *LU, uint32_t N, ui
         }
         return;
     }
-    // CTA 0: the next block's rows, then its diagonal block
-    {
-        const uint32_t i = tid % kTriBlock, g = tid / kTriBlock;  // 2 groups of 64 columns
-        C2<R> acc = zero;
-        if (i < nw) {
-            const uint32_t cEnd = min(cw, 64 * g + 64);
-            for (uint32_t c = 64 * g; c < cEnd; c += 16) {  // 16 column loads in flight together
-                C2<R> a[16];
+    // The next block: its right-hand side in y, solved in place sub-block by sub-block.
+    __syncthreads();  // y has been read
+    if (tid < kTriBlock)
+        y[tid] = tid < nw ? ld2(w + 2 * (n0 + tid)) : zero;
+    asm volatile("cp.async.wait_group 0;");
+    for (uint32_t s = 0; s < subs; ++s) {
+        const uint32_t sub = subAt(s);
+        if (i / kSub == sub)
+            part[g][i] = acc;
+        __syncthreads();
+        // x = inverse * (y - partial sums): 16 threads per row, two columns each
+        const uint32_t row = tid / 16, c = 2 * (tid % 16);
+        const C2<R> *block = subBlock(s, s) + row * kSub + c;
+        C2<R> x = zero;
 #pragma unroll
-                for (int q = 0; q < 16; ++q)
-                    a[q] = c + q < cEnd ? ld2(M + 2 * (size_t(c0 + c + q) * N + n0 + i)) : zero;
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t at = kSub * sub + c + h;
+            C2<R> t = y[at];
 #pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const C2<R> b = c + q < cEnd ? y[c + q] : zero;
-                    acc.x += a[q].x * b.x - a[q].y * b.y;
-                    acc.y += a[q].x * b.y + a[q].y * b.x;
-                }
+            for (uint32_t q = 0; q < kTriGroups; ++q) {
+                t.x -= part[q][at].x;
+                t.y -= part[q][at].y;
+            }
+            cadd<R>(x, block[h], t);
+        }
+#pragma unroll
+        for (int h = 8; h >= 1; h >>= 1) {
+            x.x += __shfl_xor_sync(0xffffffffu, x.x, h);
+            x.y += __shfl_xor_sync(0xffffffffu, x.y, h);
+        }
+        __syncthreads();  // y of this sub-block has been read
+        if (c == 0)
+            y[kSub * sub + row] = x;
+        __syncthreads();
+        // its products into the rows still to be solved: 8 columns per thread
+        const uint32_t ahead = Lower ? i / kSub : subs - 1 - i / kSub;  // this row's step
+        if (i < kSub * subs && ahead > s) {
+            const C2<R> *product = subBlock(ahead, s) + i % kSub;
+#pragma unroll
+            for (uint32_t q = 0; q < kSub / kTriGroups; ++q) {
+                const uint32_t column = g * (kSub / kTriGroups) + q;
+                cadd<R>(acc, product[column * kSub], y[kSub * sub + column]);
             }
         }
-        part[g][i] = acc;
-        __syncthreads();
-        if (tid < nw) {
-            C2<R> t = ld2(w + 2 * (n0 + tid));
-            t.x -= part[0][tid].x + part[1][tid].x;
-            t.y -= part[0][tid].y + part[1][tid].y;
-            v[tid] = t;
-        }
-        __syncthreads();
-    }
-    const int lane = tid & 31, warp = tid >> 5;
-    const uint32_t subs = (nw + 31) / 32;
-    for (uint32_t q = 0; q < subs; ++q) {
-        const uint32_t sb = Lower ? q : subs - 1 - q;  // sub-block order
-        const uint32_t k = 32 * sb, kb = min(32u, nw - k);
-        if (warp == 0) {
-            C2<R> L[32];
-#pragma unroll
-            for (int m = 0; m < 32; ++m)
-                L[m] = (m < int(kb) && lane < int(kb)) ? ld2(M + 2 * (size_t(n0 + k + m) * N + n0 + k + lane)) : zero;
-            C2<R> mine = lane < int(kb) ? v[k + lane] : zero;
-            if (Lower) {
-#pragma unroll
-                for (int m = 0; m < 32; ++m) {
-                    const C2<R> xm = mk<R>(__shfl_sync(0xffffffffu, mine.x, m), __shfl_sync(0xffffffffu, mine.y, m));
-                    if (lane > m)
-                        csub<R>(mine, L[m], xm);
-                }
-            } else {
-#pragma unroll
-                for (int m = 31; m >= 0; --m) {
-                    if (m < int(kb)) {
-                        if (lane == m) {
-                            const C2<R> d = L[m];
-                            const R den = d.x * d.x + d.y * d.y;
-                            mine = mk<R>((mine.x * d.x + mine.y * d.y) / den, (mine.y * d.x - mine.x * d.y) / den);
-                        }
-                        const C2<R> xm =
-                            mk<R>(__shfl_sync(0xffffffffu, mine.x, m), __shfl_sync(0xffffffffu, mine.y, m));
-                        if (lane < m)
-                            csub<R>(mine, L[m], xm);
-                    }
-                }
-            }
-            if (lane < int(kb))
-                v[k + lane] = mine;
-        }
-        __syncthreads();
-        // the rest of the block: rows after (forward) or before (backward) the sub-block
-        const uint32_t rBegin = Lower ? k + kb : 0, rEnd = Lower ? nw : k;
-        for (uint32_t r = rBegin + tid; r < rEnd; r += blockDim.x) {
-            C2<R> t = v[r];
-#pragma unroll 8
-            for (uint32_t m = 0; m < kb; ++m)
-                csub<R>(t, ld2(M + 2 * (size_t(n0 + k + m) * N + n0 + r)), v[k + m]);
-            v[r] = t;
-        }
-        __syncthreads();
     }
     if (tid < nw) {
-        st2(w + 2 * (n0 + tid), v[tid]);
+        st2(w + 2 * (n0 + tid), y[tid]);
         if (!Lower)
-            st2(out + 2 * ((size_t(f) * E + e) * N + n0 + tid), v[tid]);
+            st2(out + 2 * ((size_t(f) * E + e) * N + n0 + tid), y[tid]);
     }
 }
 
@@ -1999,47 +1968,46 @@ template <class R> void factor(R *LU, uint32_t N, uint32_t B, int *pivots, int *
 template <class R> void solve(const R *LU, const int *pivots, uint32_t N, uint32_t B, uint32_t E, R *x,
                               void *scratch, cudaStream_t stream, KernelTimer *timer) {
     TimedScope s(timer, "lu_solve", stream);
-    const size_t smem = size_t(N) * sizeof(C2<R>);
-    if (N <= kSmallSolve) {  // one CTA per system: the vector in shared memory, no launch per block
-        static PerDeviceHighWater attr;
-        if (smem > 48 * 1024 && attr.raise(smem))
-            check(cudaFuncSetAttribute(solveKernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-                  "solve smem attribute");
-        solveKernel<R><<<dim3(E, B), sizeof(R) == 8 ? 256 : 512, smem, stream>>>(LU, pivots, N, E, x);
-        check(cudaGetLastError(), "triangular solve launch");
-        return;
-    }
+    static PerDeviceOnce attributes;
+    attributes.run([]() {
+        check(cudaFuncSetAttribute(triStepKernel<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTriSmem<R>)),
+              "solve smem attribute");
+        check(cudaFuncSetAttribute(triStepKernel<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTriSmem<R>)),
+              "solve smem attribute");
+    });
     const int *perm = pivots + size_t(B) * N;
     R *work = static_cast<R *>(scratch);
     gatherRhsKernel<R><<<dim3((N + 255) / 256, E, B), 256, 0, stream>>>(x, perm, N, E, work);
     const uint32_t blocks = (N + kTriBlock - 1) / kTriBlock;
+    const auto grid = [&](uint32_t rows) { return dim3(1 + (rows + kTriBlock - 1) / kTriBlock, E, B); };
     // forward: block b is solved in step b with the rows updated by block b - 1
     for (uint32_t b = 0; b < blocks; ++b) {
         const uint32_t n0 = b * kTriBlock, nw = std::min(kTriBlock, N - n0);
         const uint32_t c0 = b ? n0 - kTriBlock : 0, cw = b ? kTriBlock : 0;
-        const uint32_t rows = N - n0 - nw;
-        triStepKernel<R, true><<<dim3(1 + (rows + kTriRows - 1) / kTriRows, E, B), 256, 0, stream>>>(
-            LU, N, E, work, x, c0, cw, n0, nw);
+        triStepKernel<R, true><<<grid(b ? N - n0 - nw : 0), kTriThreads, kTriSmem<R>, stream>>>(LU, pivots, N, E, work, x,
+                                                                                                c0, cw, n0, nw);
     }
     // backward: from the last block up
     for (uint32_t q = 0; q < blocks; ++q) {
         const uint32_t b = blocks - 1 - q;
         const uint32_t n0 = b * kTriBlock, nw = std::min(kTriBlock, N - n0);
         const uint32_t c0 = q ? n0 + kTriBlock : 0, cw = q ? std::min(kTriBlock, N - c0) : 0;
-        triStepKernel<R, false><<<dim3(1 + (n0 + kTriRows - 1) / kTriRows, E, B), 256, 0, stream>>>(
-            LU, N, E, work, x, c0, cw, n0, nw);
+        triStepKernel<R, false><<<grid(q ? n0 : 0), kTriThreads, kTriSmem<R>, stream>>>(LU, pivots, N, E, work, x, c0, cw,
+                                                                                        n0, nw);
     }
     check(cudaGetLastError(), "triangular solve launch");
 }
 
-template <class R> void permutation(const int *pivots, uint32_t N, uint32_t B, cudaStream_t stream) {
+// What the solves need of a factorisation: the composed permutations and the inverted diagonal blocks.
+template <class R> void prepareSolves(const R *LU, int *pivots, uint32_t N, uint32_t B, cudaStream_t stream) {
     const size_t smem = 2 * size_t(N) * sizeof(int);
     static PerDeviceHighWater attr;
     if (smem > 48 * 1024 && attr.raise(smem))
         check(cudaFuncSetAttribute(permutationKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
               "permutation smem attribute");
-    permutationKernel<<<B, 256, smem, stream>>>(pivots, N, const_cast<int *>(pivots) + size_t(B) * N);
-    check(cudaGetLastError(), "permutation launch");
+    permutationKernel<<<B, 256, smem, stream>>>(pivots, N, pivots + size_t(B) * N);
+    diagonalInverseKernel<R><<<dim3((N + kSub - 1) / kSub, B, 2), 32, 0, stream>>>(LU, N, pivots, B);
+    check(cudaGetLastError(), "solve preparation launch");
 }
 
 }  // namespace
@@ -2047,12 +2015,12 @@ template <class R> void permutation(const int *pivots, uint32_t N, uint32_t B, c
 void luFactorBatch(double *LU, uint32_t N, uint32_t B, int *pivots, int *info, cudaStream_t stream,
                    KernelTimer *timer) {
     factor<double>(LU, N, B, pivots, info, stream, timer, nullptr);
-    permutation<double>(pivots, N, B, stream);
+    prepareSolves<double>(LU, pivots, N, B, stream);
 }
 void luFactorBatch(float *LU, uint32_t N, uint32_t B, int *pivots, int *info, cudaStream_t stream,
                    KernelTimer *timer, float *pack) {
     factor<float>(LU, N, B, pivots, info, stream, timer, pack);
-    permutation<float>(pivots, N, B, stream);
+    prepareSolves<float>(LU, pivots, N, B, stream);
 }
 void luSolveBatch(const double *LU, const int *pivots, uint32_t N, uint32_t B, uint32_t E, double *x,
                   void *scratch, cudaStream_t stream, KernelTimer *timer) {
@@ -2133,7 +2101,9 @@ void debugLuFactor(bool fp32, uint32_t N, uint32_t B, const double *matrices, do
     check(cudaStreamSynchronize(stream), "LU hook");
 }
 
-size_t luWorkspaceBytes(uint32_t N, uint32_t B) { return size_t(B) * (2 * size_t(N) + kMoves) * sizeof(int); }
+size_t luWorkspaceBytes(uint32_t N, uint32_t B) {
+    return inverseOffset(N, B) * sizeof(int) + size_t(B) * 2 * inverseEntries(N) * sizeof(double2);
+}
 size_t luPackBytes(uint32_t N, uint32_t B) { return size_t(B) * packFloats(N) * sizeof(float); }
 
 }  // namespace hsb

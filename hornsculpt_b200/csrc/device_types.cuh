@@ -200,7 +200,8 @@ void assembleNearField(const AssemblyGeometry &g, const double *k, const double 
 
 // Batched dense LU (partial pivoting) and solves, complex column-major. The
 // pivot buffer holds luWorkspaceBytes(N, B): the LAPACK-style interchanges
-// of each matrix, then their composition as a permutation. A solve needs
+// of each matrix, then their composition as a permutation, the moves of the
+// panel in work and the inverted 32 x 32 diagonal blocks. A solve needs
 // B * E * N complex elements of scratch.
 size_t luWorkspaceBytes(uint32_t N, uint32_t B);
 void luFactorBatch(double *LU, uint32_t N, uint32_t B, int *pivots, int *info, cudaStream_t stream,

@@ -352,7 +352,7 @@ void Session::preparePlan(const hs_numerics &o, double maxK, const volatile int3
 namespace {
 uint64_t perFrequencyBytes(uint64_t T, uint64_t N, uint32_t E, uint32_t O, bool mixed, uint32_t restart) {
     return assemblyWorkspaceBytes(uint32_t(T), uint32_t(N), E, 1, mixed) + 2 * N * N * 16 + 4 * E * N * 16 +
-           E * T * 16 + E * N * 16 + 8 * N + fieldPartialsBytes(uint32_t(T), E, O, 1) +
+           E * T * 16 + E * N * 16 + luWorkspaceBytes(uint32_t(N), 1) + fieldPartialsBytes(uint32_t(T), E, O, 1) +
            (mixed ? gmresWorkspaceBytes(uint32_t(N), E, restart) + luPackBytes(uint32_t(N), 1) : 0) + 64;
 }
 }  // namespace
