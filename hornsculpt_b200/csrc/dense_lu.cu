@@ -986,18 +986,20 @@ __global__ void __launch_bounds__(256) gemmKernel(R *LU, uint32_t N, uint32_t k0
 // C and 192 KB of operands, so the FP64 pipe (24.6 k cycles per tile on one SM)
 // leads the memory by more than a factor of two; at K = 32 they tie, which is why
 // the factorisation has two levels. A warp owns 4 x 4 (or 2 x 2) blocks of 8 x 8
-// outputs, real and imaginary accumulators in registers, starting from C
-// itself. Operands come in stages of 16 columns by cp.async into two buffers,
-// as complex pairs: one 16-byte load gives a fragment's real and imaginary part,
-// and 8 loads feed 64 matrix instructions. Leading dimensions of 2 (L) and 4 (U)
+// outputs, real and imaginary accumulators in registers. Operands come in stages
+// of 16 columns by cp.async into two buffers, as complex pairs: one 16-byte load
+// gives a fragment's real and imaginary part, and 8 loads feed 64 matrix
+// instructions. Leading dimensions of 2 (L) and 4 (U)
 // modulo 8 entries make both fragment reads free of bank conflicts. Three CTAs
-// per SM: a tile's loads of C and its stores overlap the others' products (two
-// left the matrix pipe at 51 %, waiting for C).
+// per SM: a tile's reads and writes of C overlap the others' products (two left
+// the matrix pipe at 51 %). The products are summed from zero and taken from C
+// at the end: accumulators that start from C round every product at C's size,
+// which raised the solve residual of the 12.8k horn from 5e-15 to 2.8e-14.
 //
 // Tile 64 x 64, or 32 x 32 where 64 x 64 tiles would leave SMs idle.
 // Measured, all updates of a factorisation, against one level of K = 32 updates
-// with FP64 fused multiply-adds: N = 6380 65.2 -> 25.3 ms (outer block 64: 28.0;
-// two CTAs per SM: 39.2), N = 2562 x 2 9.2 -> 4.0, N = 642 x 32 2.56 -> 1.11,
+// with FP64 fused multiply-adds: N = 6380 65.2 -> 24.5 ms (outer block 64: 28.0;
+// two CTAs per SM: 39.2), N = 2562 x 2 9.2 -> 3.9, N = 642 x 32 2.56 -> 1.04,
 // N = 258 0.137 -> 0.077
 // ---------------------------------------------------------------------------
 constexpr int kStageK = 16;
@@ -1044,20 +1046,15 @@ __global__ void __launch_bounds__(128, TILE == 64 ? 3 : 4) gemm64Kernel(double *
         asm volatile("cp.async.commit_group;");
     };
     stage(0, k0);
-    // accumulators: block (i, j) holds rows wr + 8i + lane / 4, columns wc + 8j + 2 (lane % 4) + {0, 1}
+    // sums of the products (from zero: started from C, which is larger, every product would be rounded at C's
+    // size). Block (i, j) holds rows wr + 8i + lane / 4, columns wc + 8j + 2 (lane % 4) + {0, 1}.
     double re[W][W][2], im[W][W][2];
     const uint32_t row = row0 + wr + lane / 4, col = col0 + wc + 2 * (lane % 4);
 #pragma unroll
     for (int i = 0; i < W; ++i)
 #pragma unroll
         for (int j = 0; j < W; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t r = row + 8 * i, c = col + 8 * j + h;
-                const double2 v = r < N && c < cEnd ? ld2(M + 2 * (size_t(c) * N + r)) : make_double2(0, 0);
-                re[i][j][h] = v.x;
-                im[i][j][h] = v.y;
-            }
+            re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0;
     const int stages = int(K) / kStageK;
     for (int s = 0; s < stages; ++s) {
         if (s + 1 < stages) {
@@ -1081,35 +1078,45 @@ __global__ void __launch_bounds__(128, TILE == 64 ? 3 : 4) gemm64Kernel(double *
             for (int i = 0; i < W; ++i)
 #pragma unroll
                 for (int j = 0; j < W; ++j)
-                    mma884(re[i][j], -a[i].x, b[j].x);
+                    mma884(re[i][j], a[i].x, b[j].x);
 #pragma unroll
             for (int i = 0; i < W; ++i)
 #pragma unroll
                 for (int j = 0; j < W; ++j)
-                    mma884(im[i][j], -a[i].x, b[j].y);
+                    mma884(im[i][j], a[i].x, b[j].y);
 #pragma unroll
             for (int i = 0; i < W; ++i)
 #pragma unroll
                 for (int j = 0; j < W; ++j)
-                    mma884(re[i][j], a[i].y, b[j].y);
+                    mma884(re[i][j], -a[i].y, b[j].y);
 #pragma unroll
             for (int i = 0; i < W; ++i)
 #pragma unroll
                 for (int j = 0; j < W; ++j)
-                    mma884(im[i][j], -a[i].y, b[j].x);
+                    mma884(im[i][j], a[i].y, b[j].x);
         }
         __syncthreads();
     }
+    // a column block's entries of C are read together, then written
 #pragma unroll
-    for (int i = 0; i < W; ++i)
+    for (int j = 0; j < W; ++j) {
+        double2 old[W][2];
 #pragma unroll
-        for (int j = 0; j < W; ++j)
+        for (int i = 0; i < W; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t r = row + 8 * i, c = col + 8 * j + h;
+                old[i][h] = r < N && c < cEnd ? ld2(M + 2 * (size_t(c) * N + r)) : make_double2(0, 0);
+            }
+#pragma unroll
+        for (int i = 0; i < W; ++i)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t r = row + 8 * i, c = col + 8 * j + h;
                 if (r < N && c < cEnd)
-                    st2(M + 2 * (size_t(c) * N + r), make_double2(re[i][j][h], im[i][j][h]));
+                    st2(M + 2 * (size_t(c) * N + r), make_double2(old[i][h].x - re[i][j][h], old[i][h].y - im[i][j][h]));
             }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1442,9 +1449,9 @@ __global__ void __launch_bounds__(kTrsmThreads, 1) trsmBlockKernel(R *LU, uint32
 // Blocked triangular solves. The row interchanges of a factorisation are
 // composed once into a permutation (permutationKernel, stored after the
 // interchanges), so a solve starts with a parallel gather of the right-hand
-// side into a work vector. The 32 x 32 diagonal blocks of both triangles are
-// inverted once per factorisation (diagonalInverseKernel, stored after the
-// permutations). Forward and backward substitution then run in blocks of
+// side into a work vector. In FP32 (a preconditioner) the 32 x 32 diagonal blocks
+// of both triangles are inverted once per factorisation (diagonalInverseKernel,
+// stored after the permutations); FP64 solves by substitution. Forward and backward substitution then run in blocks of
 // kTriBlock unknowns, one launch per block: CTA 0 brings the next block's rows
 // up to date with the block solved last and solves the next diagonal block; the
 // other CTAs apply the block solved last to every remaining row. The backward
@@ -1453,12 +1460,12 @@ __global__ void __launch_bounds__(kTrsmThreads, 1) trsmBlockKernel(R *LU, uint32
 // Bound: the chain of blocks. Everything CTA 0 needs is in flight from its
 // first instruction (the diagonal block by cp.async, 32 column loads per
 // thread), a 32 x 32 sub-block is one matrix-vector product with its inverse
-// instead of 32 dependent steps of shuffles (and divisions, backward), and
-// partial sums stay in the thread that owns their row and columns until their
+// (FP32) or 32 shuffled steps from shared memory with the reciprocal diagonal
+// (FP64), and partial sums stay in the thread that owns their row and columns until their
 // sub-block is next. Measured per solve against shuffled sub-blocks loaded when
 // their turn came (one CTA per system up to N = 1024): FP32 N = 6380 3.2 -> 1.0
 // ms, N = 4023 x 3 2.1 -> 0.65, N = 642 x 32 0.25 -> 0.125; FP64 N = 6380
-// 4.2 -> 1.5, N = 2562 x 2 1.7 -> 0.62, N = 258 0.117 -> 0.065.
+// 4.2 -> 1.7, N = 2562 x 2 1.7 -> 0.71, N = 258 0.117 -> 0.073.
 constexpr uint32_t kTriBlock = 128, kSub = 32;
 constexpr uint32_t kTriThreads = 512;                  // 128 rows x 4 column groups
 constexpr uint32_t kTriGroups = kTriThreads / kTriBlock;
@@ -1475,7 +1482,7 @@ template <class R> __host__ __device__ const C2<R> *inverses(const int *pivots, 
     return reinterpret_cast<const C2<R> *>(pivots + inverseOffset(N, B)) + (2 * size_t(f) + (lower ? 0 : 1)) * inverseEntries(N);
 }
 
-// Inverses of the 32 x 32 diagonal blocks (blockIdx.x) of both triangles
+// FP32: inverses of the 32 x 32 diagonal blocks (blockIdx.x) of both triangles
 // (blockIdx.z) of each matrix: lane c solves for column c of the inverse,
 // rows stored contiguously. Rows past N are those of the identity.
 template <class R>
@@ -1582,11 +1589,22 @@ __global__ void __launch_bounds__(kTriThreads) triStepKernel(const R *LU, const 
     };
     const auto subAt = [&](uint32_t s) { return Lower ? s : subs - 1 - s; };  // sub-block solved in step s
     if (solver) {
-        const C2<R> *inverse = inverses<R>(pivots, N, gridDim.z, f, Lower) + size_t(n0 / kSub) * kSub * kSub;
+        [[maybe_unused]] const C2<R> *inverse =
+            sizeof(R) == 4 ? inverses<R>(pivots, N, gridDim.z, f, Lower) + size_t(n0 / kSub) * kSub * kSub : nullptr;
         for (uint32_t a = 0; a < subs; ++a)
             for (uint32_t b = 0; b <= a; ++b) {
                 C2<R> *block = subBlock(a, b);
-                if (a == b) {  // [row][column]
+                if (a == b && sizeof(R) == 8) {  // the triangle itself; identity past the end
+                    for (uint32_t x = tid; x < kSub * kSub; x += kTriThreads) {
+                        const uint32_t row = kSub * subAt(a) + x % kSub, column = kSub * subAt(a) + x / kSub;
+                        if (row < nw && column < nw)
+                            copyAsync<R>(block + x, M + 2 * (size_t(n0 + column) * N + n0 + row));
+                        else
+                            block[x] = mk<R>(row == column ? 1 : 0, 0);
+                    }
+                    continue;
+                }
+                if (a == b) {  // the inverse, [row][column]
                     for (uint32_t x = tid; x < kSub * kSub; x += kTriThreads)
                         copyAsync<R>(block + x, reinterpret_cast<const R *>(inverse + size_t(subAt(a)) * kSub * kSub + x));
                     continue;
@@ -1646,30 +1664,58 @@ __global__ void __launch_bounds__(kTriThreads) triStepKernel(const R *LU, const 
         if (i / kSub == sub)
             part[g][i] = acc;
         __syncthreads();
-        // x = inverse * (y - partial sums): 16 threads per row, two columns each
-        const uint32_t row = tid / 16, c = 2 * (tid % 16);
-        const C2<R> *block = subBlock(s, s) + row * kSub + c;
-        C2<R> x = zero;
+        if constexpr (sizeof(R) == 8) {  // substitution, lane = row, by the first warp
+            if (tid < kSub) {
+                const uint32_t at = kSub * sub + tid;
+                C2<R> t = y[at];
 #pragma unroll
-        for (uint32_t h = 0; h < 2; ++h) {
-            const uint32_t at = kSub * sub + c + h;
-            C2<R> t = y[at];
-#pragma unroll
-            for (uint32_t q = 0; q < kTriGroups; ++q) {
-                t.x -= part[q][at].x;
-                t.y -= part[q][at].y;
+                for (uint32_t q = 0; q < kTriGroups; ++q) {
+                    t.x -= part[q][at].x;
+                    t.y -= part[q][at].y;
+                }
+                const C2<R> *column = subBlock(s, s) + tid;
+                const C2<R> d = Lower ? mk<R>(1, 0) : column[tid * kSub];
+                const R den = d.x * d.x + d.y * d.y;
+                const C2<R> reciprocal = mk<R>(d.x / den, -d.y / den);
+#pragma unroll 8
+                for (uint32_t q = 0; q < kSub; ++q) {
+                    const uint32_t m = Lower ? q : kSub - 1 - q;
+                    const C2<R> l = column[m * kSub];
+                    if (!Lower && tid == m)
+                        t = cmul<R>(t, reciprocal);
+                    const C2<R> x = mk<R>(__shfl_sync(0xffffffffu, t.x, m), __shfl_sync(0xffffffffu, t.y, m));
+                    if (Lower ? tid > m : tid < m)
+                        csub<R>(t, l, x);
+                }
+                y[at] = t;
             }
-            cadd<R>(x, block[h], t);
-        }
+            __syncthreads();
+        } else {
+            // x = inverse * (y - partial sums): 16 threads per row, two columns each
+            const uint32_t row = tid / 16, c = 2 * (tid % 16);
+            const C2<R> *block = subBlock(s, s) + row * kSub + c;
+            C2<R> x = zero;
 #pragma unroll
-        for (int h = 8; h >= 1; h >>= 1) {
-            x.x += __shfl_xor_sync(0xffffffffu, x.x, h);
-            x.y += __shfl_xor_sync(0xffffffffu, x.y, h);
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint32_t at = kSub * sub + c + h;
+                C2<R> t = y[at];
+#pragma unroll
+                for (uint32_t q = 0; q < kTriGroups; ++q) {
+                    t.x -= part[q][at].x;
+                    t.y -= part[q][at].y;
+                }
+                cadd<R>(x, block[h], t);
+            }
+#pragma unroll
+            for (int h = 8; h >= 1; h >>= 1) {
+                x.x += __shfl_xor_sync(0xffffffffu, x.x, h);
+                x.y += __shfl_xor_sync(0xffffffffu, x.y, h);
+            }
+            __syncthreads();  // y of this sub-block has been read
+            if (c == 0)
+                y[kSub * sub + row] = x;
+            __syncthreads();
         }
-        __syncthreads();  // y of this sub-block has been read
-        if (c == 0)
-            y[kSub * sub + row] = x;
-        __syncthreads();
         // its products into the rows still to be solved: 8 columns per thread
         const uint32_t ahead = Lower ? i / kSub : subs - 1 - i / kSub;  // this row's step
         if (i < kSub * subs && ahead > s) {
@@ -1998,7 +2044,7 @@ template <class R> void solve(const R *LU, const int *pivots, uint32_t N, uint32
     check(cudaGetLastError(), "triangular solve launch");
 }
 
-// What the solves need of a factorisation: the composed permutations and the inverted diagonal blocks.
+// What the solves need of a factorisation: the composed permutations and, in FP32, the inverted diagonal blocks.
 template <class R> void prepareSolves(const R *LU, int *pivots, uint32_t N, uint32_t B, cudaStream_t stream) {
     const size_t smem = 2 * size_t(N) * sizeof(int);
     static PerDeviceHighWater attr;
@@ -2006,7 +2052,8 @@ template <class R> void prepareSolves(const R *LU, int *pivots, uint32_t N, uint
         check(cudaFuncSetAttribute(permutationKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
               "permutation smem attribute");
     permutationKernel<<<B, 256, smem, stream>>>(pivots, N, pivots + size_t(B) * N);
-    diagonalInverseKernel<R><<<dim3((N + kSub - 1) / kSub, B, 2), 32, 0, stream>>>(LU, N, pivots, B);
+    if constexpr (sizeof(R) == 4)
+        diagonalInverseKernel<R><<<dim3((N + kSub - 1) / kSub, B, 2), 32, 0, stream>>>(LU, N, pivots, B);
     check(cudaGetLastError(), "solve preparation launch");
 }
 
@@ -2102,7 +2149,7 @@ void debugLuFactor(bool fp32, uint32_t N, uint32_t B, const double *matrices, do
 }
 
 size_t luWorkspaceBytes(uint32_t N, uint32_t B) {
-    return inverseOffset(N, B) * sizeof(int) + size_t(B) * 2 * inverseEntries(N) * sizeof(double2);
+    return inverseOffset(N, B) * sizeof(int) + size_t(B) * 2 * inverseEntries(N) * sizeof(float2);
 }
 size_t luPackBytes(uint32_t N, uint32_t B) { return size_t(B) * packFloats(N) * sizeof(float); }
 
