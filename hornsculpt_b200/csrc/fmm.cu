@@ -10,6 +10,7 @@
 // warp per quadrature point for expansion tables, the local expansion's
 // divergence formed once per leaf in coefficient space.
 #include "fmm.hpp"
+#include "device_once.hpp"
 #include "fmm_math.cuh"
 #include "kernel_timer.hpp"
 
@@ -274,6 +275,221 @@ __global__ void __launch_bounds__(256) p2mKernel(const FmmPanel *__restrict__ pa
             else
                 for (int ch = 0; ch < nch; ++ch)
                     out[size_t(ch) * nc + kk] = acc[ch];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Point tables. The regular solid harmonics R_n^m, m >= 0, of every quadrature
+// point about its leaf's centre depend on the wavenumber and the panel rule but
+// not on the vector the operator is applied to, and an apply met each of them
+// twice (emission and testing), evaluating Bessel, Theta and azimuth factors
+// again each time. They are tabulated once after prepare() or setPanelDegree()
+// (row of a point: entries triIndex(n, m), degree p + 1) and read by every
+// apply: P2M 2.0 -> 0.15 ms and L2P 2.25 -> 0.18 ms for the 8k-triangle horn
+// (leaf orders 10 to 17; the tables take 0.2 ms to build and 0.2 GB). A level whose table or shared memory does not fit evaluates the
+// points on the fly (p2mKernel, l2pKernel).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void decodeTri(int e, int &n, int &m) {
+    n = int((sqrtf(8.f * e + 1.f) - 1.f) * .5f);
+    while (n * (n + 1) / 2 > e)
+        --n;
+    while ((n + 1) * (n + 2) / 2 <= e)
+        ++n;
+    m = e - n * (n + 1) / 2;
+}
+
+// One thread per point: j_n in shared memory (one column per thread), Theta by
+// the recurrences of thetaColumn with their coefficients from a table.
+constexpr int kTableThreads = 64;
+__global__ void __launch_bounds__(kTableThreads) pointTableKernel(const FmmPanel *__restrict__ panels,
+                                                                  const uint32_t *__restrict__ itemLeaf,
+                                                                  const FmmItem *__restrict__ items, uint32_t points,
+                                                                  const double *__restrict__ centers, int degree, double k,
+                                                                  const double *__restrict__ rule, int rulePts,
+                                                                  double2 *__restrict__ table) {
+    extern __shared__ double smem[];
+    const int D = degree, entries = (D + 1) * (D + 2) / 2;
+    double *rec = smem;                     // [entries][2]: recurrence coefficients a, b of (n, m)
+    double *jn = rec + 2 * entries;         // [D + 1][threads]
+    for (int e = threadIdx.x; e < entries; e += kTableThreads) {
+        int n, m;
+        decodeTri(e, n, m);
+        if (n == m) {
+            rec[2 * e] = n ? -sqrt((2.0 * n + 1) / (2.0 * n)) : 0.0;  // Theta_n^n from Theta_(n-1)^(n-1) (times s)
+            rec[2 * e + 1] = 0;
+        } else if (n == m + 1) {
+            rec[2 * e] = sqrt(2.0 * m + 3);
+            rec[2 * e + 1] = 0;
+        } else {
+            rec[2 * e] = sqrt((4.0 * n * n - 1) / double(n * n - m * m));
+            rec[2 * e + 1] = sqrt(((n - 1.0) * (n - 1) - double(m) * m) / (4.0 * (n - 1) * (n - 1) - 1));
+        }
+    }
+    __syncthreads();
+    const uint32_t pt = blockIdx.x * kTableThreads + threadIdx.x;
+    if (pt >= points)
+        return;
+    const uint32_t item = pt / rulePts, q = pt % rulePts;
+    const FmmPanel &P = panels[items[item].panel];
+    const double *c = centers + 3 * size_t(itemLeaf[item]);
+    const double b1 = rule[4 * q + 1], b2 = rule[4 * q + 2];
+    double d[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        d[i] = (P.v0[i] + b1 * P.e1[i] + b2 * P.e2[i]) - c[i];
+    const double r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    const double ct = r > 0 ? d[2] / r : 1.0;
+    const double st = sqrt(fmax(0.0, 1.0 - ct * ct));
+    const double ph = atan2(d[1], d[0]);
+    double *j = jn + threadIdx.x;
+    {  // besselJ with strided storage
+        const double x = k * r;
+        if (!(x > 1e-300)) {
+            j[0] = 1;
+            for (int n = 1; n <= D; ++n)
+                j[n * kTableThreads] = 0;
+        } else {
+            const double sx = sin(x), cx = cos(x);
+            j[0] = sx / x;
+            int up = 0;
+            if (D >= 1 && x > 1.0) {
+                j[kTableThreads] = sx / (x * x) - cx / x;
+                up = 1;
+                while (up < D && up + 1 < x) {
+                    j[(up + 1) * kTableThreads] =
+                        (2 * up + 1) / x * j[up * kTableThreads] - j[(up - 1) * kTableThreads];
+                    ++up;
+                }
+            }
+            if (up < D) {
+                double rho = 0;
+                for (int n = D + 24 + int(x); n > up; --n) {
+                    rho = x / (2 * n + 1 - x * rho);
+                    if (n <= D)
+                        j[n * kTableThreads] = rho;
+                }
+                for (int n = up + 1; n <= D; ++n)
+                    j[n * kTableThreads] *= j[(n - 1) * kTableThreads];
+            }
+        }
+    }
+    double2 *out = table + size_t(pt) * entries;
+    double seed = 0.28209479177387814;  // 1 / sqrt(4 pi)
+    for (int m = 0; m <= D; ++m) {
+        double sn, cs;
+        sincos(m * ph, &sn, &cs);
+        if (m)
+            seed *= rec[2 * triIndex(m, m)] * st;
+        double a2 = 0, a1 = seed;
+        for (int n = m; n <= D; ++n) {
+            const int e = triIndex(n, m);
+            double v = a1;
+            if (n == m + 1)
+                v = rec[2 * e] * ct * a1;
+            else if (n > m + 1)
+                v = rec[2 * e] * (ct * a1 - rec[2 * e + 1] * a2);
+            a2 = n > m ? a1 : 0.0;
+            a1 = v;
+            const double a = j[n * kTableThreads] * v;
+            out[e] = make_double2(a * cs, a * sn);
+        }
+    }
+}
+
+// P2M from the point tables: two threads per (n, m >= 0), each over every second
+// point. The products of R's and the strength's parts give (n, m) and (n, -m)
+// together (R_n^-m = (-1)^m conj R_n^m).
+constexpr int kP2mPoints = 64;
+template <int NCH>
+__global__ void __launch_bounds__(256) p2mTableKernel(const FmmPanel *__restrict__ panels,
+                                                      const uint32_t *__restrict__ leaves,
+                                                      const uint32_t *__restrict__ itemStart,
+                                                      const FmmItem *__restrict__ items,
+                                                      const uint64_t *__restrict__ coefOffset, int p,
+                                                      const double2 *__restrict__ table, const double2 *__restrict__ pvec,
+                                                      int rhsMode, double2 *M, float2 *M32, const double *__restrict__ sigma,
+                                                      const double *__restrict__ rule, int rulePts) {
+    __shared__ double2 str[kP2mPoints][NCH];
+    __shared__ double part[128][4 * NCH + 1];
+    const uint32_t leaf = leaves[blockIdx.x];
+    const uint32_t i0 = itemStart[blockIdx.x], points = (itemStart[blockIdx.x + 1] - i0) * rulePts;
+    const int nc = (p + 1) * (p + 1), used = (p + 1) * (p + 2) / 2, entries = (p + 2) * (p + 3) / 2;
+    const int half = threadIdx.x >> 7, column = threadIdx.x & 127, firstChannel = blockIdx.y * NCH;
+    const double2 *rows = table + size_t(i0) * rulePts * entries;
+    for (int e0 = 0; e0 < used; e0 += 128) {
+        const int e = e0 + column;
+        double acc[NCH][4];  // sums of Rr sr, Ri si, Rr si, Ri sr
+#pragma unroll
+        for (int ch = 0; ch < NCH; ++ch)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                acc[ch][c] = 0;
+        for (uint32_t base = 0; base < points; base += kP2mPoints) {
+            const uint32_t count = min(uint32_t(kP2mPoints), points - base);
+            __syncthreads();
+            if (threadIdx.x < count) {
+                const uint32_t idx = base + threadIdx.x;
+                const FmmItem it = items[i0 + idx / rulePts];
+                double x[3];
+                double2 s[6];
+                if (rhsMode)
+                    fluxStrength(panels[it.panel], it.panel, it.mask, rule, idx % rulePts, pvec, x, s);
+                else
+                    pointStrengths(panels[it.panel], it.mask, rule, idx % rulePts, pvec, x, s);
+#pragma unroll
+                for (int ch = 0; ch < 6; ++ch)  // this CTA's channels
+                    if (ch >= firstChannel && ch < firstChannel + NCH)
+                        str[threadIdx.x][ch - firstChannel] = s[ch];
+            }
+            __syncthreads();
+            if (e < used) {
+                const double2 *row = rows + size_t(base) * entries + e;
+#pragma unroll 4
+                for (uint32_t j = half; j < count; j += 2) {
+                    const double2 R = row[size_t(j) * entries];
+#pragma unroll
+                    for (int ch = 0; ch < NCH; ++ch) {
+                        const double2 s = str[j][ch];
+                        acc[ch][0] = fma(R.x, s.x, acc[ch][0]);
+                        acc[ch][1] = fma(R.y, s.y, acc[ch][1]);
+                        acc[ch][2] = fma(R.x, s.y, acc[ch][2]);
+                        acc[ch][3] = fma(R.y, s.x, acc[ch][3]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (half == 1)
+#pragma unroll
+            for (int c = 0; c < 4 * NCH; ++c)
+                part[column][c] = acc[c / 4][c % 4];
+        __syncthreads();
+        if (half == 1 || e >= used)
+            continue;
+        int n, m;
+        decodeTri(e, n, m);
+        const double sign = m & 1 ? -1.0 : 1.0;
+        const int kk = coefIndex(n, m), ll = coefIndex(n, -m);
+        double2 *out = M + coefOffset[leaf];
+        float2 *out32 = M32 ? M32 + coefOffset[leaf] : nullptr;
+#pragma unroll
+        for (int ch = 0; ch < NCH; ++ch) {
+            double a[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                a[c] = acc[ch][c] + part[column][4 * ch + c];
+            const double2 plus = make_double2(a[0] + a[1], a[2] - a[3]);
+            const double2 minus = make_double2(sign * (a[0] - a[1]), sign * (a[2] + a[3]));
+            if (out32) {  // scaled FP32 moments, as in p2mKernel
+                out32[size_t(firstChannel + ch) * nc + kk] = make_float2(float(plus.x * sigma[n]), float(plus.y * sigma[n]));
+                if (m)
+                    out32[size_t(firstChannel + ch) * nc + ll] = make_float2(float(minus.x * sigma[n]), float(minus.y * sigma[n]));
+            } else {
+                out[size_t(firstChannel + ch) * nc + kk] = plus;
+                if (m)
+                    out[size_t(firstChannel + ch) * nc + ll] = minus;
+            }
         }
     }
 }
@@ -703,6 +919,31 @@ __device__ void loadLocals(const double2 *L64, const float2 *L32, const double *
     __syncthreads();
 }
 
+// Coefficient (n, m) of D = div V (times k): dx Vx + dy Vy + dz Vz = (d+ U- + d- U+) / 2 + dz Vz,
+// U-+ = Vx -+ i Vy, from the locals Ls of degree p (channels Vx, Vy, Vz first).
+__device__ double2 divergenceAt(const double2 *Ls, int p, int nc, int n, int m, double k) {
+    const double2 *Vx = Ls, *Vy = Ls + nc, *Vz = Ls + 2 * nc;
+    const auto U = [&](int nn, int mm, double sign) {  // Vx + sign i Vy
+        const double2 x = coefAt(Vx, p, nn, mm), y = coefAt(Vy, p, nn, mm);
+        return make_double2(x.x - sign * y.y, x.y + sign * y.x);
+    };
+    // dz: L_{n+1,m} A(n+1,m) - L_{n-1,m} A(n,m)
+    const double2 z1 = coefAt(Vz, p, n + 1, m), z0 = coefAt(Vz, p, n - 1, m);
+    const double a1 = coefA(n + 1, m), a0 = coefA(n, m);
+    double2 d = make_double2(z1.x * a1 - z0.x * a0, z1.y * a1 - z0.y * a0);
+    // d+ U-: U-_{n+1,m-1} Bm(n+1,m-1) + U-_{n-1,m-1} Bp(n-1,m-1)
+    const double2 u1 = U(n + 1, m - 1, -1), u0 = U(n - 1, m - 1, -1);
+    const double bm = coefBm(n + 1, m - 1), bp = coefBp(n - 1, m - 1);
+    d.x += 0.5 * (u1.x * bm + u0.x * bp);
+    d.y += 0.5 * (u1.y * bm + u0.y * bp);
+    // d- U+: -(U+_{n+1,m+1} Cm(n+1,m+1) + U+_{n-1,m+1} Cp(n-1,m+1))
+    const double2 v1 = U(n + 1, m + 1, 1), v0 = U(n - 1, m + 1, 1);
+    const double cm = coefCm(n + 1, m + 1), cp = coefCp(n - 1, m + 1);
+    d.x -= 0.5 * (v1.x * cm + v0.x * cp);
+    d.y -= 0.5 * (v1.y * cm + v0.y * cp);
+    return make_double2(k * d.x, k * d.y);
+}
+
 // L2P of the leaves of one level: forms D = div V (degree p + 1) in shared
 // memory, then one warp per item evaluates V, W, D at its quadrature points
 // and writes the item's incidence contributions
@@ -726,30 +967,10 @@ __global__ void __launch_bounds__(256) l2pKernel(const FmmPanel *__restrict__ pa
     const uint32_t leaf = leaves[blockIdx.x];
     loadLocals(Lcoef, L32, sigma, coefOffset[leaf], 6, nc, Ls);
     __syncthreads();
-    // D = dx Vx + dy Vy + dz Vz = (d+ U- + d- U+) / 2 + dz Vz, U-+ = Vx -+ i Vy (times k)
     for (int kk = threadIdx.x; kk < nd; kk += blockDim.x) {
         int n, m;
         decode(kk, n, m);
-        const double2 *Vx = Ls, *Vy = Ls + nc, *Vz = Ls + 2 * nc;
-        const auto U = [&](int nn, int mm, double sign) {  // Vx + sign i Vy
-            const double2 x = coefAt(Vx, p, nn, mm), y = coefAt(Vy, p, nn, mm);
-            return make_double2(x.x - sign * y.y, x.y + sign * y.x);
-        };
-        // dz: L_{n+1,m} A(n+1,m) - L_{n-1,m} A(n,m)
-        const double2 z1 = coefAt(Vz, p, n + 1, m), z0 = coefAt(Vz, p, n - 1, m);
-        const double a1 = coefA(n + 1, m), a0 = coefA(n, m);
-        double2 d = make_double2(z1.x * a1 - z0.x * a0, z1.y * a1 - z0.y * a0);
-        // d+ U-: U-_{n+1,m-1} Bm(n+1,m-1) + U-_{n-1,m-1} Bp(n-1,m-1)
-        const double2 u1 = U(n + 1, m - 1, -1), u0 = U(n - 1, m - 1, -1);
-        const double bm = coefBm(n + 1, m - 1), bp = coefBp(n - 1, m - 1);
-        d.x += 0.5 * (u1.x * bm + u0.x * bp);
-        d.y += 0.5 * (u1.y * bm + u0.y * bp);
-        // d- U+: -(U+_{n+1,m+1} Cm(n+1,m+1) + U+_{n-1,m+1} Cp(n-1,m+1))
-        const double2 v1 = U(n + 1, m + 1, 1), v0 = U(n - 1, m + 1, 1);
-        const double cm = coefCm(n + 1, m + 1), cp = coefCp(n - 1, m + 1);
-        d.x -= 0.5 * (v1.x * cm + v0.x * cp);
-        d.y -= 0.5 * (v1.y * cm + v0.y * cp);
-        Ld[kk] = make_double2(k * d.x, k * d.y);
+        Ld[kk] = divergenceAt(Ls, p, nc, n, m, k);
     }
     __syncthreads();
     const uint32_t i0 = itemStart[blockIdx.x], i1 = itemStart[blockIdx.x + 1];
@@ -813,6 +1034,104 @@ __global__ void __launch_bounds__(256) l2pKernel(const FmmPanel *__restrict__ pa
             for (int a = 0; a < 3; ++a)
                 if ((item.mask >> a) & 1)
                     far[item.inc[a]] = acc[a];
+    }
+}
+
+// L2P from the point tables. With L' = (-1)^m L_n^-m, L_n^m R + L_n^-m R_n^-m =
+// Re R (L + L') + Im R i (L - L'): both sums per (channel, n, m >= 0) are formed
+// once per leaf in shared memory. A warp takes an item; its lanes own the entries
+// of R, and since everything after is linear each lane forms its share of the
+// item's three contributions over all its points before one warp sum.
+HS_HD size_t l2pTableSmem(int p) {
+    return (6 * size_t(p + 1) * (p + 1) + 14 * size_t(p + 2) * (p + 3) / 2) * sizeof(double2);
+}
+__global__ void __launch_bounds__(256) l2pTableKernel(const FmmPanel *__restrict__ panels,
+                                                      const uint32_t *__restrict__ leaves,
+                                                      const uint32_t *__restrict__ itemStart,
+                                                      const FmmItem *__restrict__ items,
+                                                      const uint64_t *__restrict__ coefOffset, int p, double k,
+                                                      const double2 *__restrict__ table,
+                                                      const double2 *__restrict__ Lcoef, double2 *far,
+                                                      const float2 *__restrict__ L32, const double *__restrict__ sigma,
+                                                      const double *__restrict__ rule, int rulePts) {
+    extern __shared__ double smem[];
+    const int nc = (p + 1) * (p + 1), used = (p + 1) * (p + 2) / 2, entries = (p + 2) * (p + 3) / 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2 *Ls = reinterpret_cast<double2 *>(smem);  // [6][nc]
+    double2 *UV = Ls + 6 * nc;                        // [channel 0..6][entry][2]
+    loadLocals(Lcoef, L32, sigma, coefOffset[leaves[blockIdx.x]], 6, nc, Ls);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 7 * entries; i += blockDim.x) {
+        const int ch = i / entries, e = i - ch * entries;
+        int n, m;
+        decodeTri(e, n, m);
+        const auto value = [&](int mm) {
+            return ch < 6 ? coefAt(Ls + ch * nc, p, n, mm) : divergenceAt(Ls, p, nc, n, mm, k);
+        };
+        const double2 a = value(m);
+        double2 b = make_double2(0, 0);
+        if (m) {
+            b = value(-m);
+            if (m & 1)
+                b = make_double2(-b.x, -b.y);
+        }
+        UV[2 * i] = make_double2(a.x + b.x, a.y + b.y);
+        UV[2 * i + 1] = m ? make_double2(b.y - a.y, a.x - b.x) : make_double2(0, 0);
+    }
+    __syncthreads();
+    const uint32_t i0 = itemStart[blockIdx.x], i1 = itemStart[blockIdx.x + 1];
+    for (uint32_t it = i0 + blockIdx.y * kWarps + warp; it < i1; it += gridDim.y * kWarps) {
+        const FmmItem item = items[it];
+        const FmmPanel &Pn = panels[item.panel];
+        double acc[6] = {0, 0, 0, 0, 0, 0};
+        for (int q = 0; q < rulePts; ++q) {
+            const double2 *row = table + (size_t(it) * rulePts + q) * entries;
+            double2 f[7];
+#pragma unroll
+            for (int ch = 0; ch < 7; ++ch)
+                f[ch] = make_double2(0, 0);
+            for (int e = lane; e < entries; e += 32) {
+                const double2 R = row[e];
+#pragma unroll
+                for (int ch = 0; ch < 7; ++ch) {
+                    if (ch < 6 && e >= used)
+                        continue;
+                    const double2 U = UV[2 * (ch * entries + e)], V = UV[2 * (ch * entries + e) + 1];
+                    f[ch].x = fma(R.x, U.x, fma(R.y, V.x, f[ch].x));
+                    f[ch].y = fma(R.x, U.y, fma(R.y, V.y, f[ch].y));
+                }
+            }
+            // fields F = -i k f; D + i k n.V, and -(i / k) curl . W
+            const double w = rule[4 * q + 3] * Pn.area;
+            double nx = 0, ny = 0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                nx += Pn.n[d] * f[d].x;
+                ny += Pn.n[d] * f[d].y;
+            }
+            const double sx = k * f[6].y + k * k * nx, sy = -k * f[6].x + k * k * ny;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                double cx = 0, cy = 0;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    cx += Pn.curl[3 * a + d] * f[3 + d].x;
+                    cy += Pn.curl[3 * a + d] * f[3 + d].y;
+                }
+                const double wb = w * rule[4 * q + a];
+                acc[2 * a] += wb * sx - w * cx;
+                acc[2 * a + 1] += wb * sy - w * cy;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (lane == 0)
+            for (int a = 0; a < 3; ++a)
+                if ((item.mask >> a) & 1)
+                    far[item.inc[a]] = make_double2(acc[2 * a], acc[2 * a + 1]);
     }
 }
 
@@ -1399,6 +1718,14 @@ struct FmmOperator::Impl {
     double hfThreshold = 8.0;
     double tolerance = 1e-8;  // expansion tolerance of the last prepare()
     DevBuf rule, l2pScratch;
+    // Point tables of the prepared wavenumber and the current panel rule (pointTableKernel), built by the
+    // first apply after prepare() or setPanelDegree() (never inside a capture: both drop the graphs, and
+    // the first apply after that launches directly).
+    DevBuf itemLeaf, pointTable;
+    std::vector<uint64_t> tableStart;  // per level, entries
+    std::vector<bool> tableLevel;      // the level reads its table
+    bool tableStale = true;
+    const double2 *table(int l) const { return tableLevel[l] ? pointTable.as<double2>() + tableStart[l] : nullptr; }
     int rulePts = 0;
     unsigned panelDegree = 4;
     bool useGraphs = true;
@@ -1665,6 +1992,12 @@ FmmOperator::FmmOperator(const Space &space, const FmmTreeSettings &settings) : 
     uploadVec(I.centers, cen, s);
     uploadVec(I.incOff, I.incOffsets, s);
     uploadVec(I.dItems, I.items, s);
+    std::vector<uint32_t> itemLeaf(I.items.size());
+    for (int l = 0; l < levels; ++l)
+        for (size_t leaf = 0; leaf < I.leafNodes[l].size(); ++leaf)
+            for (uint32_t it = I.leafItemStart[l][leaf]; it < I.leafItemStart[l][leaf + 1]; ++it)
+                itemLeaf[I.itemBase[l] + it] = I.leafNodes[l][leaf];
+    uploadVec(I.itemLeaf, itemLeaf, s);
     I.dm2m.resize(levels);
     I.dm2l.resize(levels);
     I.dl2l.resize(levels);
@@ -1758,6 +2091,7 @@ void FmmOperator::setPanelDegree(unsigned degree, cudaStream_t stream) {
     fmmCheck(cudaStreamSynchronize(stream), "rule upload");
     I.rulePts = int(rule.size());
     I.panelDegree = degree;
+    I.tableStale = true;
     I.dropGraphs();
 }
 
@@ -1866,6 +2200,7 @@ void FmmOperator::setGraphs(bool enabled) {
 void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
     Impl &I = *impl_;
     I.dropGraphs();  // the tables and orders below change what a graph would replay
+    I.tableStale = true;
     k_ = k;
     levelInfo_.clear();
     if (tree_.ppFar.empty())
@@ -2089,6 +2424,47 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
     fmmCheck(cudaStreamSynchronize(stream), "prepare");
 }
 
+// Point tables of every level whose L2P tables fit shared memory, when all of them fit a quarter of the
+// free memory (24 GB at most); otherwise the leaves evaluate their points on the fly.
+void FmmOperator::buildPointTables(cudaStream_t stream) {
+    Impl &I = *impl_;
+    I.tableStale = false;
+    const int levels = int(tree_.levels.size());
+    I.tableStart.assign(levels, 0);
+    I.tableLevel.assign(levels, false);
+    size_t freeBytes = 0, totalBytes = 0, total = 0;
+    if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess)
+        freeBytes = 0;
+    const size_t cap = std::min<size_t>(size_t(24) << 30, freeBytes / 4 + I.pointTable.bytes);
+    for (int l = I.lmin; l < levels; ++l) {
+        const size_t points = size_t(I.itemBase[l + 1] - I.itemBase[l]) * I.rulePts;
+        if (!points || points > 0x7fffffffu || l2pTableSmem(I.order[l]) > kMaxShared)
+            continue;
+        I.tableLevel[l] = true;
+        I.tableStart[l] = total;
+        total += points * (size_t(I.order[l] + 2) * (I.order[l] + 3) / 2);
+    }
+    if (total * sizeof(double2) > cap) {
+        I.tableLevel.assign(levels, false);
+        return;
+    }
+    I.pointTable.ensure(total * sizeof(double2));
+    for (int l = I.lmin; l < levels; ++l) {
+        if (!I.tableLevel[l])
+            continue;
+        const int D = I.order[l] + 1;
+        const uint32_t points = (I.itemBase[l + 1] - I.itemBase[l]) * uint32_t(I.rulePts);
+        const size_t sm = (size_t(D + 1) * (D + 2) + size_t(D + 1) * kTableThreads) * sizeof(double);
+        fmmCheck(cudaFuncSetAttribute(pointTableKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
+                 "point table smem");
+        pointTableKernel<<<(points + kTableThreads - 1) / kTableThreads, kTableThreads, sm, stream>>>(
+            I.panels.as<FmmPanel>(), I.itemLeaf.as<uint32_t>() + I.itemBase[l], I.dItems.as<FmmItem>() + I.itemBase[l],
+            points, I.centers.as<double>(), D, k_, I.rule.as<double>(), I.rulePts,
+            I.pointTable.as<double2>() + I.tableStart[l]);
+        fmmCheck(cudaGetLastError(), "point table launch");
+    }
+}
+
 void FmmOperator::applyFar(const double *p, size_t stride, uint32_t S, double *y, cudaStream_t stream,
                            KernelTimer *timer) {
     for (uint32_t sys = 0; sys < S; ++sys)
@@ -2174,6 +2550,10 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
     }
     const int nch = rhs ? 1 : 6;
     const int levels = int(tree_.levels.size());
+    if (I.tableStale) {
+        TimedScope scope(timer, "fmm_point_tables", stream);
+        buildPointTables(stream);
+    }
     fmmCheck(cudaMemsetAsync(I.far.p, 0, 3 * size_t(I.T) * 16, stream), "zero contributions");
     if (I.fp32)
         fmmCheck(cudaMemsetAsync(I.Lc32.p, 0, I.coefTotal * 8, stream), "zero locals");
@@ -2241,6 +2621,18 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             if (!leaves)
                 continue;
             const int P = I.order[l];
+            if (const double2 *table = I.table(l)) {
+                // few leaves: a channel per CTA
+                const bool narrow = rhs || leaves < unsigned(smCount());
+                const auto kernel = narrow ? p2mTableKernel<1> : p2mTableKernel<6>;
+                kernel<<<dim3(leaves, narrow && !rhs ? 6 : 1), 256, 0, stream>>>(I.panels.as<FmmPanel>(), I.dLeaves[l].as<uint32_t>(),
+                                                   I.dLeafStart[l].as<uint32_t>(), I.dItems.as<FmmItem>() + I.itemBase[l],
+                                                   I.coefOffset.as<uint64_t>(), P, table, pv, rhs ? 1 : 0, I.Mc.as<double2>(),
+                                                   I.fp32 ? I.Mc32.as<float2>() : nullptr, I.levelSigma(l),
+                                                   I.rule.as<double>(), I.rulePts);
+                fmmCheck(cudaGetLastError(), "p2m launch");
+                continue;
+            }
             const size_t td = tableDoubles(P);
             const size_t sm = (kWarps * td) * 8 + kWarps * 6 * 16;
             if (sm > kMaxShared)
@@ -2325,6 +2717,20 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             if (!leaves)
                 continue;
             const int p = I.order[l], P = p + 1;
+            if (const double2 *table = rhs ? nullptr : I.table(l)) {
+                const size_t sm = l2pTableSmem(p);
+                fmmCheck(cudaFuncSetAttribute(l2pTableKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
+                         "l2p smem");
+                // few leaves: their items over several CTAs
+                const unsigned split = std::clamp(2u * unsigned(smCount()) / leaves, 1u, 8u);
+                l2pTableKernel<<<dim3(leaves, split), 256, sm, stream>>>(
+                    I.panels.as<FmmPanel>(), I.dLeaves[l].as<uint32_t>(), I.dLeafStart[l].as<uint32_t>(),
+                    I.dItems.as<FmmItem>() + I.itemBase[l], I.coefOffset.as<uint64_t>(), p, k_, table,
+                    I.Lc.as<double2>(), I.far.as<double2>(), I.fp32 ? I.Lc32.as<float2>() : nullptr, I.levelSigma(l),
+                    I.rule.as<double>(), I.rulePts);
+                fmmCheck(cudaGetLastError(), "l2p launch");
+                continue;
+            }
             const size_t td = tableDoubles(P);
             const size_t nc = size_t(p + 1) * (p + 1), nd = size_t(P + 1) * (P + 1);
             const size_t coefBytes = (rhs ? nc + 3 * nd : 6 * nc + nd) * 16, tableBytes = kWarps * td * 8;

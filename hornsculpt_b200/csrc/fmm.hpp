@@ -88,6 +88,7 @@ class FmmOperator {
     void run(const double *src, bool rhs, double *y, cudaStream_t stream, KernelTimer *timer);
     void launchApply(const double *src, bool rhs, double *y, cudaStream_t stream, KernelTimer *timer);
     void prepareHf(cudaStream_t stream);
+    void buildPointTables(cudaStream_t stream);
     void planeWaveM2L(int level, int nch, cudaStream_t stream);
 };
 

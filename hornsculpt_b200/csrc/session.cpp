@@ -368,10 +368,10 @@ size_t solveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t B, bo
 size_t fmmSolveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t restart) {
     // geometry and plan as for the dense form; near records and their pair
     // lists at about 700 near panel pairs per panel, near CSR values, GMRES
-    // basis and the expansion tables (a fixed allowance)
+    // basis, the expansion tables (a fixed allowance) and the point tables
     const size_t geometry = T * (200 + 48 + 112 + 16) + N * 24, plan = T * (T - 1) / 2 + T * 16 * 40 + T * 16 * 220;
     const size_t nearField = T * 700 * (kRecordDoubles * 8 + 4 + 8 + 8) + N * 500 * 20;
-    const size_t solve = size_t(E) * N * 16 * (restart + 12) + N * 6 * 1024 * 16 * 2;
+    const size_t solve = size_t(E) * N * 16 * (restart + 12) + N * 6 * 1024 * 16 * 2 + T * (size_t(24) << 10);
     const size_t fields = fieldPartialsBytes(uint32_t(T), E, O, 1) + size_t(E) * T * 16;
     return geometry + plan + nearField + solve + fields + (size_t(256) << 20);
 }
