@@ -859,6 +859,313 @@ __global__ void __launch_bounds__(256) m2lGroupKernel(const uint2 *__restrict__ 
     }
 }
 
+// Grouped M2L of the FP64 operator on the FP64 matrix instruction, for orders up
+// to kMatrixOrder. A chunk's columns (links x channels, real and imaginary parts
+// as two columns) form one real matrix X [coefficient][column] in shared memory;
+// each rotation is a product per degree with its Wigner block, the coaxial
+// translation a product per m with its complex table block (twice: with X and
+// with i X, whose columns are X's swapped in pairs). A warp takes (degree or m,
+// up to three tiles of 8 columns), keeps all output rows in accumulators and
+// writes them over its inputs, so one buffer holds the chunk and two CTAs fit an
+// SM. Items are handed out largest first.
+//
+// Bound: the FP64 pipe on the padded products (8 rows, 4 inner, 8 columns: 70 % of
+// the rotations' and 57 % of the coaxial work is useful at p = 12), which it keeps
+// 38 % busy beside the shared-memory traffic of staging and fragments (58 %). The
+// scalar form (m2lGroupKernel, kept for higher orders and FP32) read six shared
+// values and two table entries per 24 multiply-adds and kept the pipe at 23 %.
+// M2L of the 8k-triangle horn at 2 kHz (orders 10-17, 164 580 links): 5.3 -> 3.3 ms
+// (tables unpacked 4.1, packed 3.9, twelve warps a CTA 3.3).
+constexpr int kMatrixOrder = 23;
+// Row tiles of the largest degree, two instances: orders up to 15 (4 tiles) leave registers for twelve warps a
+// CTA, the rest run eight.
+constexpr int kMatrixRows = (2 * kMatrixOrder + 1 + 7) / 8, kSmallRows = 4, kSmallOrder = 15;
+constexpr int kSlab = 3;                                     // column tiles per item
+constexpr size_t kMatrixShared = 112 * 1024;                 // two CTAs per SM
+
+// columns (doubles) of X for C complex columns, and its row stride: 4 or 12 modulo 16 keeps the fragment
+// reads free of bank conflicts
+__host__ __device__ inline int matrixColumns(int C) { return (2 * C + 7) / 8 * 8; }
+__host__ __device__ inline int matrixStride(int C) {
+    const int n = matrixColumns(C);
+    return n + 4;  // n is 0 or 8 modulo 16
+}
+__host__ __device__ inline size_t matrixSmem(int p, int C, int g) {
+    return size_t(p + 1) * (p + 1) * matrixStride(C) * sizeof(double) + size_t(g) * (p + 1) * sizeof(double2);
+}
+
+__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// Table entries in fragment order: block (inner step kt, row tile mt) of a rows x
+// inner product is 32 consecutive entries, lane l the entry (8 mt + l / 4,
+// 4 kt + l % 4), zeros outside; so a warp reads one whole block per load.
+__host__ __device__ inline int packedBlocks(int rows, int inner) { return ((rows + 7) / 8) * ((inner + 3) / 4); }
+// Entries before degree n of a packed Wigner class, and before |m| = a of a packed coaxial class of order p.
+__host__ __device__ inline size_t packedWignerOffset(int n) {
+    size_t at = 0;
+    for (int j = 0; j < n; ++j)
+        at += size_t(packedBlocks(2 * j + 1, 2 * j + 1)) * 32;
+    return at;
+}
+__host__ __device__ inline size_t packedCoaxOffset(int p, int a) {
+    size_t at = 0;
+    for (int j = 0; j < a; ++j)
+        at += size_t(packedBlocks(p + 1 - j, p + 1 - j)) * 32;
+    return at;
+}
+
+// Packs the degrees n <= order[c] of every Wigner class: first d^n (back rotation), then its transpose
+// (forward). blockIdx.y: class, blockIdx.x: degree.
+__global__ void packWignerKernel(const double *__restrict__ wigner, const uint64_t *__restrict__ start,
+                                 const int *__restrict__ order, const uint64_t *__restrict__ packedStart,
+                                 double *__restrict__ packed) {
+    const uint32_t c = blockIdx.y;
+    const int n = blockIdx.x, top = min(order[c], kMatrixOrder);
+    if (n > top)
+        return;
+    const int w = 2 * n + 1, rowTiles = (w + 7) / 8, count = packedBlocks(w, w) * 32;
+    const double *d = wigner + start[c] + wignerOffset(n);
+    double *back = packed + packedStart[c] + packedWignerOffset(n);
+    double *forward = back + packedWignerOffset(top + 1);
+    for (int e = threadIdx.x; e < count; e += blockDim.x) {
+        const int block = e / 32, lane = e % 32;
+        const int row = 8 * (block % rowTiles) + lane / 4, k = 4 * (block / rowTiles) + lane % 4;
+        const bool inside = row < w && k < w;
+        back[e] = inside ? d[size_t(row) * w + k] : 0.0;
+        forward[e] = inside ? d[size_t(k) * w + row] : 0.0;
+    }
+}
+// Packs the square coaxial classes of order at most kMatrixOrder. blockIdx.y: class, blockIdx.x: |m|.
+__global__ void packCoaxKernel(const double2 *__restrict__ coax, const uint64_t *__restrict__ start,
+                               const int *__restrict__ pin, const int *__restrict__ pout,
+                               const uint64_t *__restrict__ packedStart, double2 *__restrict__ packed) {
+    const uint32_t c = blockIdx.y;
+    const int p = pin[c], a = blockIdx.x, wo = p + 1 - a;
+    if (pout[c] != p || p > kMatrixOrder || a > p)
+        return;
+    const int rowTiles = (wo + 7) / 8, count = packedBlocks(wo, wo) * 32;
+    const int big = p + 1;
+    const double2 *C = coax + start[c] + (big * (big + 1) * (2 * big + 1) - wo * (wo + 1) * (2 * wo + 1)) / 6;
+    double2 *out = packed + packedStart[c] + packedCoaxOffset(p, a);
+    for (int e = threadIdx.x; e < count; e += blockDim.x) {
+        const int block = e / 32, lane = e % 32;
+        const int row = 8 * (block % rowTiles) + lane / 4, k = 4 * (block / rowTiles) + lane % 4;
+        out[e] = row < wo && k < wo ? C[size_t(k) * wo + row] : make_double2(0, 0);
+    }
+}
+
+// X rows n^2 .. n^2 + 2n, column tiles [t0, t0 + tiles): X <- D X with D's packed blocks. The next inner
+// step's blocks are fetched while this step's products run.
+template <int ROWS>
+__device__ __forceinline__ void rotateMatrix(double *X, int ld, int n, int t0, int tiles, const double *packed) {
+    const int w = 2 * n + 1, lane = threadIdx.x & 31, row = lane >> 2, kl = lane & 3, rowTiles = (w + 7) / 8;
+    double acc[ROWS][kSlab][2], a[ROWS];
+    const double *d = packed + lane;
+#pragma unroll
+    for (int mt = 0; mt < ROWS; ++mt) {
+        a[mt] = mt < rowTiles ? __ldg(d + 32 * mt) : 0.0;
+#pragma unroll
+        for (int s = 0; s < kSlab; ++s)
+            acc[mt][s][0] = acc[mt][s][1] = 0;
+    }
+    double *base = X + size_t(n) * n * ld + 8 * t0;
+    for (int k0 = 0; k0 < w; k0 += 4) {
+        const int k = min(k0 + kl, w - 1);  // past the degree: its last row, times zero
+        double b[kSlab];
+#pragma unroll
+        for (int s = 0; s < kSlab; ++s)
+            b[s] = s < tiles ? base[size_t(k) * ld + 8 * s + row] : 0.0;
+        d += 32 * rowTiles;
+        const bool more = k0 + 4 < w;
+#pragma unroll
+        for (int mt = 0; mt < ROWS; ++mt) {
+            if (mt >= rowTiles)
+                break;
+            const double now = a[mt];
+            if (more)
+                a[mt] = __ldg(d + 32 * mt);
+#pragma unroll
+            for (int s = 0; s < kSlab; ++s)
+                if (s < tiles)
+                    mma884(acc[mt][s], now, b[s]);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int mt = 0; mt < ROWS; ++mt) {
+        if (mt >= rowTiles)
+            break;
+        if (8 * mt + row < w)
+#pragma unroll
+            for (int s = 0; s < kSlab; ++s)
+                if (s < tiles)
+                    *reinterpret_cast<double2 *>(base + size_t(8 * mt + row) * ld + 8 * s + 2 * kl) =
+                        make_double2(acc[mt][s][0], acc[mt][s][1]);
+    }
+    __syncwarp();
+}
+
+template <int ROWS>
+__global__ void __launch_bounds__(ROWS == kSmallRows ? 384 : 256, 2) m2lMatrixKernel(const uint2 *__restrict__ chunks,
+                                                          const uint32_t *__restrict__ sorted,
+                                                          const TransLink *__restrict__ links, int p, int nch, int gmax,
+                                                          const double2 *__restrict__ inCoef,
+                                                          const uint64_t *__restrict__ coefOffset,
+                                                          const double *__restrict__ wigner,
+                                                          const uint64_t *__restrict__ wignerStart,
+                                                          const int *__restrict__ wignerOrder,
+                                                          const double2 *__restrict__ coax,
+                                                          const uint64_t *__restrict__ coaxStart,
+                                                          double2 *__restrict__ u) {
+    extern __shared__ double smem[];
+    __shared__ int next[3];
+    const int nc = (p + 1) * (p + 1), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint2 chunk = chunks[blockIdx.x];
+    const int count = int(chunk.y), C = count * nch, ld = matrixStride(gmax * nch), columns = matrixColumns(C);
+    double *X = smem;
+    double2 *eph = reinterpret_cast<double2 *>(X + size_t(nc) * ld);  // [gmax][p + 1]
+    const TransLink L0 = links[sorted[chunk.x]];
+    const double *dtab = wigner + wignerStart[L0.wclass];  // packed: back rotations, then forward
+    const double2 *ctab = coax + coaxStart[L0.cclass];     // packed
+    // entries before degree n of the Wigner blocks (and their total), before |m| = a of the coaxial blocks
+    __shared__ int wignerAt[kMatrixOrder + 2], coaxAt[kMatrixOrder + 1];
+    if (threadIdx.x <= unsigned(kMatrixOrder) + 1)
+        wignerAt[threadIdx.x] = int(packedWignerOffset(threadIdx.x));
+    if (threadIdx.x >= 64 && int(threadIdx.x) - 64 <= p)
+        coaxAt[threadIdx.x - 64] = int(packedCoaxOffset(p, threadIdx.x - 64));
+    const int wignerTop = min(wignerOrder[L0.wclass], kMatrixOrder);
+    for (int e = threadIdx.x; e < count * (p + 1); e += blockDim.x) {
+        const int i = e / (p + 1), m = e - i * (p + 1);
+        double sn, cs;
+        sincos(m * links[sorted[chunk.x + i]].phi, &sn, &cs);
+        eph[e] = make_double2(cs, sn);
+    }
+    // zeros in the columns past the chunk
+    for (int e = threadIdx.x; e < nc * (columns - 2 * C); e += blockDim.x)
+        X[size_t(e / (columns - 2 * C)) * ld + 2 * C + e % (columns - 2 * C)] = 0;
+    if (threadIdx.x < 3)
+        next[threadIdx.x] = 0;
+    __syncthreads();
+    // staged inputs with the azimuth phase, a warp per (strip of 32 coefficients, channel)
+    const int strips = (nc + 31) / 32;
+    for (int item = warp; item < strips * nch; item += warps) {
+        const int ch = item / strips, kk = (item - ch * strips) * 32 + lane;
+        if (kk >= nc)
+            continue;
+        int n, m;
+        decode(kk, n, m);
+        const int am = m < 0 ? -m : m;
+        for (int i = 0; i < count; ++i) {
+            const double2 ph = eph[i * (p + 1) + am];
+            const double2 v = inCoef[coefOffset[links[sorted[chunk.x + i]].source] + size_t(ch) * nc + kk];
+            *reinterpret_cast<double2 *>(X + size_t(kk) * ld + 2 * (i * nch + ch)) =
+                cmul(v, m < 0 ? make_double2(ph.x, -ph.y) : ph);
+        }
+    }
+    __syncthreads();
+    const int tiles = columns / 8, slabs = (tiles + kSlab - 1) / kSlab;
+    const auto take = [&](int phase) {
+        int item = 0;
+        if (lane == 0)
+            item = atomicAdd(&next[phase], 1);
+        return __shfl_sync(0xffffffffu, item, 0);
+    };
+    // forward rotation: X[n, m'] = sum_m d^n[m, m'] X[n, m]
+    for (int item = take(0); item < (p + 1) * slabs; item = take(0)) {
+        const int n = p - item / slabs, t0 = (item % slabs) * kSlab;
+        rotateMatrix<ROWS>(X, ld, n, t0, min(kSlab, tiles - t0), dtab + wignerAt[wignerTop + 1] + wignerAt[n]);
+    }
+    __syncthreads();
+    // coaxial translation: X[n', m] = sum_n C_|m|[n][n'] X[n, m], rows n of one m
+    for (int item = take(1); item < (2 * p + 1) * slabs; item = take(1)) {
+        const int mi = item / slabs, t0 = (item % slabs) * kSlab, active = min(kSlab, tiles - t0);
+        const int a = (mi + 1) / 2, m = mi & 1 ? a : -a, wo = p + 1 - a;
+        const double2 *Ct = ctab + coaxAt[a] + lane;
+        const int rowTiles = (wo + 7) / 8;
+        const int row = lane >> 2, kl = lane & 3;
+        const double flip = row & 1 ? 1.0 : -1.0;  // i X: (-im, re)
+        constexpr int kTiles = ROWS / 2;  // of p + 1 rows
+        double acc[kTiles][kSlab][2];
+        double2 table[kTiles];
+#pragma unroll
+        for (int mt = 0; mt < kTiles; ++mt) {
+            table[mt] = mt < rowTiles ? __ldg(Ct + 32 * mt) : make_double2(0, 0);
+#pragma unroll
+            for (int s = 0; s < kSlab; ++s)
+                acc[mt][s][0] = acc[mt][s][1] = 0;
+        }
+        const auto rowOf = [&](int j) {  // X row of n = a + j
+            const int n = a + j;
+            return X + size_t(n * n + n + m) * ld + 8 * t0;
+        };
+        for (int k0 = 0; k0 < wo; k0 += 4) {
+            const double *x = rowOf(min(k0 + kl, wo - 1));
+            double b[kSlab], bi[kSlab];
+#pragma unroll
+            for (int s = 0; s < kSlab; ++s) {
+                b[s] = s < active ? x[8 * s + row] : 0.0;
+                bi[s] = s < active ? flip * x[8 * s + (row ^ 1)] : 0.0;
+            }
+            Ct += 32 * rowTiles;
+            const bool more = k0 + 4 < wo;
+#pragma unroll
+            for (int mt = 0; mt < kTiles; ++mt) {
+                if (mt >= rowTiles)
+                    break;
+                const double2 c = table[mt];
+                if (more)
+                    table[mt] = __ldg(Ct + 32 * mt);
+#pragma unroll
+                for (int s = 0; s < kSlab; ++s)
+                    if (s < active)
+                        mma884(acc[mt][s], c.x, b[s]);
+#pragma unroll
+                for (int s = 0; s < kSlab; ++s)
+                    if (s < active)
+                        mma884(acc[mt][s], c.y, bi[s]);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int mt = 0; mt < kTiles; ++mt) {
+            if (8 * mt >= wo)
+                break;
+            if (8 * mt + row < wo)
+#pragma unroll
+                for (int s = 0; s < kSlab; ++s)
+                    if (s < active)
+                        *reinterpret_cast<double2 *>(rowOf(8 * mt + row) + 8 * s + 2 * kl) =
+                            make_double2(acc[mt][s][0], acc[mt][s][1]);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    // back rotation: X[n, m1] = sum_m d^n[m1, m] X[n, m]
+    for (int item = take(2); item < (p + 1) * slabs; item = take(2)) {
+        const int n = p - item / slabs, t0 = (item % slabs) * kSlab;
+        rotateMatrix<ROWS>(X, ld, n, t0, min(kSlab, tiles - t0), dtab + wignerAt[n]);
+    }
+    __syncthreads();
+    // each link's contribution with the conjugate phase, into its own slot
+    for (int item = warp; item < strips * nch; item += warps) {
+        const int ch = item / strips, kk = (item - ch * strips) * 32 + lane;
+        if (kk >= nc)
+            continue;
+        int n, m;
+        decode(kk, n, m);
+        const int am = m < 0 ? -m : m;
+        for (int i = 0; i < count; ++i) {
+            const double2 ph = eph[i * (p + 1) + am];
+            const double2 v = *reinterpret_cast<const double2 *>(X + size_t(kk) * ld + 2 * (i * nch + ch));
+            u[(size_t(sorted[chunk.x + i]) * nch + ch) * nc + kk] = cmul(v, m < 0 ? ph : make_double2(ph.x, -ph.y));
+        }
+    }
+}
+
 // out[target] += sum over the target's links, in link order, of their slots.
 template <class R>
 __global__ void __launch_bounds__(256) m2lSumKernel(const uint32_t *__restrict__ outNodes,
@@ -1681,6 +1988,9 @@ struct FmmOperator::Impl {
     };
     std::vector<GroupPlan> gm2l;
     DevBuf slots;  // per-link M2L contributions (largest grouped level)
+    // tables of m2lMatrixKernel in fragment order (FP64 operator)
+    DevBuf wignerPacked, wignerPackedStart, wignerOrder, coaxPacked, coaxPackedStart;
+    bool wignerPackedValid = false;
     bool groupedM2l = true;
     std::vector<DevBuf> dLeaves, dLeafStart;
     std::vector<std::vector<uint32_t>> coaxClassOf;  // per kind*levels: local coax class index -> global
@@ -2260,6 +2570,7 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
         uploadVec(I.wignerStart, start, stream);
         I.hostWigner = std::move(tab);
         I.wigner32Valid = false;
+        I.wignerPackedValid = false;
     }
     // coaxial classes of this wavenumber
     int P = 0;
@@ -2316,6 +2627,38 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
         uint32_t(pin.size()), I.coaxPin.as<int>(), I.coaxPout.as<int>(), I.coaxStart.as<uint64_t>(),
         I.fl.as<double2>(), lmaxF, I.gaunt.as<double>(), I.gauntOff.as<uint32_t>(), P, I.coax.as<double2>());
     fmmCheck(cudaGetLastError(), "coaxial table launch");
+    if (!I.fp32) {  // the matrix form's tables
+        if (!I.wignerPackedValid) {
+            std::vector<uint64_t> packedStart;
+            uint64_t size = 0;
+            for (int order : I.wclassP) {
+                packedStart.push_back(size);
+                size += order < 0 ? 0 : 2 * packedWignerOffset(std::min(order, kMatrixOrder) + 1);
+            }
+            uploadVec(I.wignerPackedStart, packedStart, stream);
+            uploadVec(I.wignerOrder, I.wclassP, stream);
+            I.wignerPacked.ensure(std::max<uint64_t>(size, 1) * sizeof(double));
+            if (!I.wclassP.empty())
+                packWignerKernel<<<dim3(kMatrixOrder + 1, uint32_t(I.wclassP.size())), 128, 0, stream>>>(
+                    I.wigner.as<double>(), I.wignerStart.as<uint64_t>(), I.wignerOrder.as<int>(),
+                    I.wignerPackedStart.as<uint64_t>(), I.wignerPacked.as<double>());
+            fmmCheck(cudaGetLastError(), "packed Wigner table launch");
+            I.wignerPackedValid = true;
+        }
+        std::vector<uint64_t> packedStart;
+        uint64_t size = 0;
+        for (size_t c = 0; c < pin.size(); ++c) {
+            packedStart.push_back(size);
+            if (pin[c] == pout[c] && pin[c] <= kMatrixOrder)
+                size += packedCoaxOffset(pin[c], pin[c] + 1);
+        }
+        uploadVec(I.coaxPackedStart, packedStart, stream);
+        I.coaxPacked.ensure(std::max<uint64_t>(size, 1) * sizeof(double2));
+        packCoaxKernel<<<dim3(kMatrixOrder + 1, uint32_t(pin.size())), 128, 0, stream>>>(
+            I.coax.as<double2>(), I.coaxStart.as<uint64_t>(), I.coaxPin.as<int>(), I.coaxPout.as<int>(),
+            I.coaxPackedStart.as<uint64_t>(), I.coaxPacked.as<double2>());
+        fmmCheck(cudaGetLastError(), "packed coaxial table launch");
+    }
     prepareHf(stream);
     for (auto &info : levelInfo_)
         info.planeWave = I.hf[info.level].active ? 1 : 0;
@@ -2393,6 +2736,12 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
             for (int mode = 0; mode < 2; ++mode) {
                 const int nch = mode == 0 ? 6 : 1;
                 int g = 0, cpad = 0;
+                const bool matrix = !I.fp32 && p <= kMatrixOrder;
+                for (int cand = 16; matrix && cand >= 1 && !g; --cand)
+                    if (matrixSmem(p, cand * nch, cand) <= kMatrixShared)
+                        g = cand;
+                if (matrix && !g)
+                    g = 1;  // one CTA per SM
                 for (int cand = 16; cand >= 1 && !g; --cand)
                     if (groupSmemBytes(p, (cand * nch) | 1, cand, cb) <= 110 * 1024) {
                         g = cand;
@@ -2663,7 +3012,6 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
         constexpr bool f32 = std::is_same_v<RT, float>;
         const Impl::GroupPlan &gp = I.gm2l[l];
         const int mode = rhs ? 1 : 0, p = I.order[l], nc = (p + 1) * (p + 1);
-        const size_t sm = groupSmemBytes(p, gp.cpad[mode], gp.g[mode], sizeof(CT));
         const RT *wig;
         const CT *cx;
         if constexpr (f32) {
@@ -2673,12 +3021,30 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             wig = I.wigner.as<double>();
             cx = I.coax.as<double2>();
         }
-        fmmCheck(cudaFuncSetAttribute(m2lGroupKernel<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                 "grouped m2l smem");
-        m2lGroupKernel<RT><<<gp.chunkCount[mode], 256, sm, stream>>>(
-            gp.chunks[mode].as<uint2>(), gp.sorted.as<uint32_t>(), I.dm2l[l].links.as<TransLink>(), p, nch,
-            gp.cpad[mode], gp.g[mode], in, I.coefOffset.as<uint64_t>(), wig, I.wignerStart.as<uint64_t>(), cx,
-            I.coaxStart.as<uint64_t>(), I.slots.as<CT>());
+        bool matrix = false;
+        if constexpr (!f32) {
+            matrix = p <= kMatrixOrder;
+            if (matrix) {
+                const size_t sm = matrixSmem(p, gp.g[mode] * nch, gp.g[mode]);
+                const auto kernel = p <= kSmallOrder ? m2lMatrixKernel<kSmallRows> : m2lMatrixKernel<kMatrixRows>;
+                fmmCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
+                         "matrix m2l smem");
+                kernel<<<gp.chunkCount[mode], p <= kSmallOrder ? 384 : 256, sm, stream>>>(
+                    gp.chunks[mode].as<uint2>(), gp.sorted.as<uint32_t>(), I.dm2l[l].links.as<TransLink>(), p, nch,
+                    gp.g[mode], in, I.coefOffset.as<uint64_t>(), I.wignerPacked.as<double>(),
+                    I.wignerPackedStart.as<uint64_t>(), I.wignerOrder.as<int>(), I.coaxPacked.as<double2>(),
+                    I.coaxPackedStart.as<uint64_t>(), I.slots.as<CT>());
+            }
+        }
+        if (!matrix) {
+            const size_t sm = groupSmemBytes(p, gp.cpad[mode], gp.g[mode], sizeof(CT));
+            fmmCheck(cudaFuncSetAttribute(m2lGroupKernel<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
+                     "grouped m2l smem");
+            m2lGroupKernel<RT><<<gp.chunkCount[mode], 256, sm, stream>>>(
+                gp.chunks[mode].as<uint2>(), gp.sorted.as<uint32_t>(), I.dm2l[l].links.as<TransLink>(), p, nch,
+                gp.cpad[mode], gp.g[mode], in, I.coefOffset.as<uint64_t>(), wig, I.wignerStart.as<uint64_t>(), cx,
+                I.coaxStart.as<uint64_t>(), I.slots.as<CT>());
+        }
         fmmCheck(cudaGetLastError(), "grouped m2l launch");
         const dim3 grid(I.dm2l[l].count, unsigned((nch * nc + 255) / 256));
         TimedScope sums(timer, "fmm_m2l_sum", stream);  // nested in fmm_m2l
