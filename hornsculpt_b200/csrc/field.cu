@@ -6,6 +6,7 @@
 // in a fixed order.
 #include "device_once.hpp"
 #include "device_types.cuh"
+#include "green_math.cuh"
 #include "host_mesh.hpp"
 #include "kernel_timer.hpp"
 
@@ -23,6 +24,7 @@ constexpr int kTile = 256;
 // Field rules of degree 4, 6, 8, 12, 14: 6 + 12 + 16 + 49 + 64 points.
 constexpr int kFieldPoints = 147;
 __constant__ double cField[kFieldPoints * 4];
+__constant__ double cFieldWeighted[kFieldPoints * 2];  // w b1, w b2
 
 __device__ __forceinline__ void ruleOf(uint32_t degree, int &offset, int &count) {
     switch (degree) {
@@ -218,6 +220,139 @@ __global__ void __launch_bounds__(128) fieldKernel(FieldRequest req, const doubl
     }
 }
 
+// Far field of many directions (balloons): a thread owns a direction and runs
+// over a tile's panels, whose geometry and sources it reads from shared memory
+// (the same address for the whole warp). The phase k d.(y - origin) is affine in
+// the trial barycentrics and does not depend on the excitation, so a rule point
+// costs its sine and cosine and six accumulations into the moments sum w e^(i phase)
+// (1, b1, b2); the excitations' pressures and fluxes meet the moments once per
+// panel. One CTA per 64 directions, 256-panel tile and frequency, excitations in
+// groups of kFarExcitations. With one CTA per output (fieldKernel) every panel's
+// data were read and every phase was formed again for each output and excitation:
+// 2664 directions x 2 excitations x 8 frequencies x 1280 triangles 9.3 -> 2.9 ms.
+constexpr int kFarThreads = 64, kFarChunk = 32, kFarExcitations = 2;
+constexpr uint32_t kFarDirections = 32;  // from this many directions on
+
+struct FarPanel {
+    double o[3], e1[3], e2[3], n[3];  // o: first vertex minus the far-field origin
+};
+
+// Moments of one panel for rule points [RO, RO + RC): W = {1, b1, b2} sums, real and imaginary.
+template <int RO, int RC>
+__device__ __forceinline__ void farMoments(double phase, double p1, double p2, double (&W)[6]) {
+#pragma unroll(RC <= 16 ? RC / 2 : 4)
+    for (int s = 0; s < RC; ++s) {
+        const double *w = cField + 4 * (RO + s), *v = cFieldWeighted + 2 * (RO + s);
+        double sn, cs;
+        sinCos(fma(p2, w[2], fma(p1, w[1], phase)), sn, cs);
+        W[0] = fma(cs, w[3], W[0]);
+        W[1] = fma(sn, w[3], W[1]);
+        W[2] = fma(cs, v[0], W[2]);
+        W[3] = fma(sn, v[0], W[3]);
+        W[4] = fma(cs, v[1], W[4]);
+        W[5] = fma(sn, v[1], W[5]);
+    }
+}
+
+template <int RO, int RC>
+__device__ void farTile(const FieldRequest &req, uint32_t f, uint32_t e0, uint32_t count, uint32_t tile, double k,
+                        const double *pressure, const double *flux, const double (&x)[3], double (&v)[kFarExcitations][2],
+                        bool &bad, FarPanel *panels, double (*source)[kFarExcitations][8]) {
+    const uint32_t begin = tile * kTile, end = min(begin + uint32_t(kTile), req.T);
+    for (uint32_t base = begin; base < end; base += kFarChunk) {
+        const uint32_t n = min(uint32_t(kFarChunk), end - base);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += kFarThreads) {
+            const DPanel &pn = req.panels[base + i];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                panels[i].o[c] = pn.v0[c] - req.farOrigin[c];
+                panels[i].e1[c] = pn.e1[c];
+                panels[i].e2[c] = pn.e2[c];
+                panels[i].n[c] = pn.n[c];
+            }
+        }
+        // sources with the panel's Jacobian: p at the first vertex, its differences to the others, q
+        for (uint32_t i = threadIdx.x; i < n * count; i += kFarThreads) {
+            const uint32_t t = base + i / count, e = i % count;
+            const DPanel &pn = req.panels[t];
+            const double a = 2 * pn.area * kInvFourPi;
+            const double *p = pressure + (size_t(f) * req.E + e0 + e) * req.N * 2;
+            const double *q = flux + ((size_t(f) * req.E + e0 + e) * req.T + t) * 2;
+            double *s = source[i / count][e];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const double first = p[2 * pn.nodes[0] + c];
+                s[c] = a * first;
+                s[2 + c] = a * (p[2 * pn.nodes[1] + c] - first);
+                s[4 + c] = a * (p[2 * pn.nodes[2] + c] - first);
+                s[6 + c] = a * q[c];
+            }
+        }
+        __syncthreads();
+        for (uint32_t i = 0; i < n; ++i) {
+            const FarPanel &pn = panels[i];
+            const double phase = k * (x[0] * pn.o[0] + x[1] * pn.o[1] + x[2] * pn.o[2]);
+            const double p1 = k * (x[0] * pn.e1[0] + x[1] * pn.e1[1] + x[2] * pn.e1[2]);
+            const double p2 = k * (x[0] * pn.e2[0] + x[1] * pn.e2[1] + x[2] * pn.e2[2]);
+            const double nf = k * (x[0] * pn.n[0] + x[1] * pn.n[1] + x[2] * pn.n[2]);
+            bad |= !isfinite(phase + (p1 + p2));
+            double W[6] = {0, 0, 0, 0, 0, 0};
+            farMoments<RO, RC>(phase, p1, p2, W);
+#pragma unroll
+            for (int e = 0; e < kFarExcitations; ++e) {
+                if (uint32_t(e) >= count)
+                    break;
+                const double *s = source[i][e];
+                // U = sum w e^(i phase) p, W0 q
+                const double ur = s[0] * W[0] - s[1] * W[1] + s[2] * W[2] - s[3] * W[3] + s[4] * W[4] - s[5] * W[5];
+                const double ui = s[0] * W[1] + s[1] * W[0] + s[2] * W[3] + s[3] * W[2] + s[4] * W[5] + s[5] * W[4];
+                v[e][0] += -nf * ui - (s[6] * W[0] - s[7] * W[1]);
+                v[e][1] += nf * ur - (s[6] * W[1] + s[7] * W[0]);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kFarThreads) farFieldKernel(FieldRequest req, const double *ks, const double *pressure,
+                                                              const double *flux, const uint32_t *batchDegree,
+                                                              double *partials, int *error) {
+    __shared__ FarPanel panels[kFarChunk];
+    __shared__ double source[kFarChunk][kFarExcitations][8];
+    const uint32_t tiles = (req.T + kTile - 1) / kTile, groups = (req.E + kFarExcitations - 1) / kFarExcitations;
+    const uint32_t tile = blockIdx.y % tiles, f = blockIdx.y / tiles / groups;
+    const uint32_t e0 = (blockIdx.y / tiles % groups) * kFarExcitations;
+    const uint32_t count = min(uint32_t(kFarExcitations), req.E - e0);
+    const uint32_t o = blockIdx.x * kFarThreads + threadIdx.x;
+    const double k = ks[f];
+    double x[3], v[kFarExcitations][2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        x[c] = o < req.O ? req.observers[3 * o + c] : 0.0;
+#pragma unroll
+    for (int e = 0; e < kFarExcitations; ++e)
+        v[e][0] = v[e][1] = 0;
+    bool bad = false;
+    switch (batchDegree[f]) {
+    case 4: farTile<0, 6>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
+    case 6: farTile<6, 12>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
+    case 8: farTile<18, 16>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
+    case 12: farTile<34, 49>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
+    default: farTile<83, 64>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
+    }
+    if (bad)
+        atomicExch(error, kErrDistance);
+    if (o >= req.O)
+        return;
+    double sn, cs;
+    sincos(k * req.farDistance, &sn, &cs);
+    for (uint32_t e = 0; e < count; ++e) {
+        double *out = partials + 2 * (((size_t(f) * req.E + e0 + e) * req.O + o) * tiles + tile);
+        out[0] = (v[e][0] * cs + v[e][1] * sn) / req.farDistance;
+        out[1] = (v[e][1] * cs - v[e][0] * sn) / req.farDistance;
+    }
+}
+
 __global__ void finishKernel(const double *partials, uint32_t tiles, size_t outputs, double *out, int *error) {
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= outputs)
@@ -301,38 +436,44 @@ struct SamplePatch {
     uint32_t depth;
 };
 
-// D p - S q over one patch with one rule, and the magnitude sum |D p| + |S q|
-__device__ void patchIntegral(const DPanel &t, const SamplePatch &patch, V3 x, double k, const double (&p)[6],
-                              double qr, double qi, int offset, int count, double &re, double &im, double &mag) {
+// D p - S q over one patch with one rule, and the magnitude sum |D p| + |S q|.
+// (x - y).n is constant over the panel, and the magnitudes follow from the
+// moduli: |S q| = |q| / (4 pi r), |D p| = |p| |(x - y).n| sqrt(1 + (k r)^2) / (4 pi r^3).
+// With the short root and sine/cosine, 4096 points at 1280 triangles take 1.3 ms.
+struct SamplePanel {
+    double v0[3], e1[3], e2[3];  // observer minus first vertex, edges
+    double dn, scale;            // (x - y).n, 2 area / (4 pi)
+    double p[6];                 // pressure at the first vertex, differences to the others
+    double q[2], qAbs;
+};
+__device__ __forceinline__ void patchIntegral(const SamplePanel &t, const SamplePatch &patch, double k, int offset,
+                                              int count, double &re, double &im, double &mag) {
     re = im = mag = 0;
-    const V3 n = v3(t.n[0], t.n[1], t.n[2]);
     for (int r = 0; r < count; ++r) {
         const double *rule = cField + 4 * (offset + r);
-        double b[3];
-        for (int i = 0; i < 3; ++i)
-            b[i] = patch.b[i] * rule[0] + patch.b[3 + i] * rule[1] + patch.b[6 + i] * rule[2];
-        // y = v0 b0 + v1 b1 + v2 b2 with v1 = v0 + e1, v2 = v0 + e2
-        V3 y;
-        y.x = t.v0[0] * b[0] + (t.v0[0] + t.e1[0]) * b[1] + (t.v0[0] + t.e2[0]) * b[2];
-        y.y = t.v0[1] * b[0] + (t.v0[1] + t.e1[1]) * b[1] + (t.v0[1] + t.e2[1]) * b[2];
-        y.z = t.v0[2] * b[0] + (t.v0[2] + t.e1[2]) * b[1] + (t.v0[2] + t.e2[2]) * b[2];
-        const V3 d = x - y;
-        const double rr = sqrt(norm2(d));
+        const double b1 = patch.b[1] * rule[0] + patch.b[4] * rule[1] + patch.b[7] * rule[2];
+        const double b2 = patch.b[2] * rule[0] + patch.b[5] * rule[1] + patch.b[8] * rule[2];
+        const double dx = fma(-b2, t.e2[0], fma(-b1, t.e1[0], t.v0[0]));
+        const double dy = fma(-b2, t.e2[1], fma(-b1, t.e1[1], t.v0[1]));
+        const double dz = fma(-b2, t.e2[2], fma(-b1, t.e1[2], t.v0[2]));
+        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        const double rinv = reciprocalRoot(r2), rinv2 = rinv * rinv, kr = k * (r2 * rinv);
         double sn, cs;
-        sincos(k * rr, &sn, &cs);
-        const double gm = kInvFourPi / rr, gr = gm * cs, gi = -gm * sn;  // exp(-ikr) / (4 pi r)
-        const double bq = b[0] + b[1] + b[2];
-        const double sr = gr * qr * bq - gi * qi * bq, si = gr * qi * bq + gi * qr * bq;  // g (b . q)
-        const double pr = b[0] * p[0] + b[1] * p[2] + b[2] * p[4], pi = b[0] * p[1] + b[1] * p[3] + b[2] * p[5];
-        const double proj = dot(d, n) / rr;
-        // g (1/r + i k) proj (b . p)
-        const double hr = (gr / rr - gi * k) * proj, hi = (gi / rr + gr * k) * proj;
-        const double dr = hr * pr - hi * pi, di = hr * pi + hi * pr;
-        const double w = 2 * t.area * patch.fraction * rule[3];
-        re += w * (dr - sr);
-        im += w * (di - si);
-        mag += w * (sqrt(dr * dr + di * di) + sqrt(sr * sr + si * si));
+        sinCos(kr, sn, cs);
+        const double pr = fma(b2, t.p[4], fma(b1, t.p[2], t.p[0])), pi = fma(b2, t.p[5], fma(b1, t.p[3], t.p[1]));
+        // e^(-ikr) (1 + ikr) (x - y).n / r^2 p - e^(-ikr) q, over r
+        const double proj = t.dn * rinv2;
+        const double hr = fma(sn, kr, cs) * proj, hi = fma(cs, kr, -sn) * proj;
+        const double w = rule[3] * rinv;
+        re = fma(w, (hr * pr - hi * pi) - (cs * t.q[0] + sn * t.q[1]), re);
+        im = fma(w, (hr * pi + hi * pr) - (cs * t.q[1] - sn * t.q[0]), im);
+        const double square = fma(kr, kr, 1.0) * (pr * pr + pi * pi) * (proj * proj);
+        mag = fma(w, (square > 1e-290 ? square * reciprocalRoot(square) : 0.0) + t.qAbs, mag);
     }
+    const double s = t.scale * patch.fraction;
+    re *= s;
+    im *= s;
+    mag *= s;
 }
 
 __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPanel *__restrict__ panels, uint32_t T,
@@ -379,21 +520,37 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
     SamplePatch stack[kFieldStack];
     for (uint32_t t = tid; t < T && !failed; t += kFieldThreads) {
         const DPanel &panel = panels[t];
-        double p[6];
+        SamplePanel sample;
+        sample.scale = 2 * panel.area * kInvFourPi;
+        const double d0[3] = {x.x - panel.v0[0], x.y - panel.v0[1], x.z - panel.v0[2]};
+        sample.dn = d0[0] * panel.n[0] + d0[1] * panel.n[1] + d0[2] * panel.n[2];
+#pragma unroll
         for (int i = 0; i < 3; ++i) {
-            p[2 * i] = trace[2 * panel.nodes[i]];
-            p[2 * i + 1] = trace[2 * panel.nodes[i] + 1];
+            sample.v0[i] = d0[i];
+            sample.e1[i] = panel.e1[i];
+            sample.e2[i] = panel.e2[i];
         }
-        const double qr = flux[2 * t], qi = flux[2 * t + 1];
-        if (qr == 0 && qi == 0 && p[0] == 0 && p[1] == 0 && p[2] == 0 && p[3] == 0 && p[4] == 0 && p[5] == 0)
+        bool silent = true;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const double first = trace[2 * panel.nodes[0] + c], second = trace[2 * panel.nodes[1] + c],
+                         third = trace[2 * panel.nodes[2] + c];
+            sample.p[c] = first;
+            sample.p[2 + c] = second - first;
+            sample.p[4 + c] = third - first;
+            sample.q[c] = flux[2 * t + c];
+            silent = silent && first == 0 && second == 0 && third == 0 && sample.q[c] == 0;
+        }
+        if (silent)
             continue;
+        sample.qAbs = sqrt(sample.q[0] * sample.q[0] + sample.q[1] * sample.q[1]);
         int top = 0;
         stack[top++] = SamplePatch{{1, 0, 0, 0, 1, 0, 0, 0, 1}, 1.0, 0};
         while (top > 0) {
             const SamplePatch patch = stack[--top];
             double cr, ci, cm, fr, fi, fm;
-            patchIntegral(panel, patch, x, k, p, qr, qi, 0, 6, cr, ci, cm);    // degree 4
-            patchIntegral(panel, patch, x, k, p, qr, qi, 18, 16, fr, fi, fm);  // degree 8
+            patchIntegral(sample, patch, k, 0, 6, cr, ci, cm);    // degree 4
+            patchIntegral(sample, patch, k, 18, 16, fr, fi, fm);  // degree 8
             const double span = k * panel.maxEdge * sqrt(patch.fraction);
             const double diff = sqrt((fr - cr) * (fr - cr) + (fi - ci) * (fi - ci));
             if (span <= 3.14159265358979323846 && diff <= tolerance * fmax(fm, 1e-300)) {
@@ -461,7 +618,14 @@ void uploadFieldRules(cudaStream_t stream) {
                 table[4 * o + 3] = p.w;
                 ++o;
             }
+        double weighted[kFieldPoints * 2];
+        for (int i = 0; i < kFieldPoints; ++i) {
+            weighted[2 * i] = table[4 * i + 3] * table[4 * i + 1];
+            weighted[2 * i + 1] = table[4 * i + 3] * table[4 * i + 2];
+        }
         check(cudaMemcpyToSymbolAsync(cField, table, sizeof(table), 0, cudaMemcpyHostToDevice, stream),
+              "field rule upload");
+        check(cudaMemcpyToSymbolAsync(cFieldWeighted, weighted, sizeof(weighted), 0, cudaMemcpyHostToDevice, stream),
               "field rule upload");
         check(cudaStreamSynchronize(stream), "field rule upload");
     });
@@ -494,8 +658,13 @@ void evaluateFieldBatch(const FieldRequest &req, const double *ks, const double 
         return;
     {
         TimedScope s(timer, "field", stream);
-        fieldKernel<<<unsigned(outputs * tiles), 128, 0, stream>>>(req, ks, pressure, flux, batchDegree, partials,
-                                                                  error);
+        const uint64_t groups = uint64_t(req.B) * ((req.E + kFarExcitations - 1) / kFarExcitations) * tiles;
+        if (req.farField && req.O >= kFarDirections && groups <= 65535)
+            farFieldKernel<<<dim3((req.O + kFarThreads - 1) / kFarThreads, unsigned(groups)), kFarThreads, 0, stream>>>(
+                req, ks, pressure, flux, batchDegree, partials, error);
+        else
+            fieldKernel<<<unsigned(outputs * tiles), 128, 0, stream>>>(req, ks, pressure, flux, batchDegree, partials,
+                                                                      error);
     }
     {
         TimedScope s(timer, "field_finish", stream);
