@@ -381,8 +381,10 @@ class CudaBemSolver:
         _lib.check(self._lib.hs_bem_pressure_field(self._handle, frequency, medium.sound_speed, trace.ctypes.data,
                                                    deriv.ctypes.data, pts.ctypes.data, n, C.byref(st),
                                                    out.ctypes.data, status.ctypes.data))
-        return [PressureFieldSample(tuple(pts[i]), complex(out[2 * i], out[2 * i + 1]), FieldPointStatus(status[i]))
-                for i in range(n)]
+        # columns and lookups instead of a constructor chain per point: thousands of points a call
+        kinds = tuple(FieldPointStatus)
+        return list(map(PressureFieldSample, zip(pts[:, 0], pts[:, 1], pts[:, 2]),
+                        out.view(np.complex128)[:n].tolist(), (kinds[s] for s in status[:n].tolist())))
 
     # -- marshalling --------------------------------------------------------
     def _c_request(self, r: BemRequest):
