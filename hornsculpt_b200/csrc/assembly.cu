@@ -1179,37 +1179,23 @@ __device__ __forceinline__ void nearSample(float (&acc)[54], const DPanel &t, co
         }
 }
 
-// Green values (g, P, Q as re/im pairs) of one sample of a near pair in the
-// plain form, FP64.
-__device__ __forceinline__ void plainValues(double dx, double dy, double dz, double w, double k, const DPanel &t,
-                                            const DPanel &s, double (&val)[6], bool &bad) {
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    bad |= !(r2 > 0) || !isfinite(r2);
-    const double rinv = rsqrt(r2);
-    const double r = r2 * rinv, kr = k * r;
-    double sn, cs;
-    sincos(kr, &sn, &cs);
-    const double sc = w * rinv;
-    const double gr = cs * sc, gi = -sn * sc;
-    const double rr = gr - gi * kr, ri = gi + gr * kr;
-    const double rinv2 = rinv * rinv;
-    const double ps = (dx * s.n[0] + dy * s.n[1] + dz * s.n[2]) * rinv2;
-    const double qt = -(dx * t.n[0] + dy * t.n[1] + dz * t.n[2]) * rinv2;
-    val[0] = gr;
-    val[1] = gi;
-    val[2] = rr * ps;
-    val[3] = ri * ps;
-    val[4] = rr * qt;
-    val[5] = ri * qt;
-}
-
 // Near pairs whose patches are all tensor patches: one warp per unordered
 // pair. Lane (x, half) owns test point x of the patch rule and half of the
 // trial points; trial bases are contracted in registers, test bases through
 // shared memory by the 27 lanes that own a (kind, i, j) moment. Pairs with
 // projected patches go to nearKernel.
+//
+// The plain form accumulates the moments of regularPairsKernel with the short
+// root and sine/cosine; the mixed form keeps its sample and converts a patch
+// point's barycentrics to FP32 once. Jobs come with the most patches first (the
+// plan sorts them): patch counts range from one to hundreds, and in plan order
+// long pairs that started last left two thirds of the warps idle. Measured:
+// 8042 triangles x 3 frequencies (mixed) 16.8 -> 10.8 ms, 12 756 triangles plain
+// 11.7 -> 6.3, mixed 7.5 -> 5.0, 1280 x 32 plain 1.91 -> 1.39. Eight CTAs per SM
+// (mixed) and six (plain) are the most without spills. FP64 pipe 52 % (plain),
+// conversion pipe 49 % (mixed) active.
 template <bool Mixed>
-__global__ void __launch_bounds__(64, Mixed ? 10 : 1) nearWarpKernel(const DPanel *__restrict__ panels, uint32_t T,
+__global__ void __launch_bounds__(64, Mixed ? 8 : 6) nearWarpKernel(const DPanel *__restrict__ panels, uint32_t T,
                                                       const NearPairJob *__restrict__ jobs, uint32_t jobCount,
                                                       const Patch *__restrict__ patches, const double *__restrict__ ks,
                                                       std::conditional_t<Mixed, float, double> *__restrict__ records,
@@ -1217,8 +1203,9 @@ __global__ void __launch_bounds__(64, Mixed ? 10 : 1) nearWarpKernel(const DPane
     using Acc = std::conditional_t<Mixed, float, double>;
     __shared__ Acc sS[2][64][18];     // per warp: trial-contracted values S(x)
     __shared__ double sB[2][64][3];   // per warp: mapped test barycentrics
-    __shared__ double sY[2][64][3];   // per warp: mapped trial barycentrics
-    __shared__ double sE[2][64][3];   // per warp: trial points' offsets from the trial panel's first vertex
+    __shared__ __align__(16) double2 sE[2][64][2];  // per warp: trial points' offsets from the trial panel's first vertex
+    // per warp and trial point: mapped barycentrics (mixed: b0, b1, b2 in FP32; plain: b1, b2, b1^2, b1 b2, b2^2)
+    __shared__ __align__(16) std::conditional_t<Mixed, float4, double2> sY[2][64][Mixed ? 1 : 3];
     __shared__ double sM[2][54];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t pairIndex = blockIdx.x * 2 + warp;
@@ -1233,25 +1220,43 @@ __global__ void __launch_bounds__(64, Mixed ? 10 : 1) nearWarpKernel(const DPane
     bool bad = false;
     double own[2] = {0, 0};  // lanes 0..26: accumulated moment (kind, i, j) of this pair
     const double d0[3] = {t.v0[0] - s.v0[0], t.v0[1] - s.v0[1], t.v0[2] - s.v0[2]};
+    [[maybe_unused]] const float nsF[3] = {float(s.n[0]), float(s.n[1]), float(s.n[2])};
+    [[maybe_unused]] const float ntF[3] = {float(t.n[0]), float(t.n[1]), float(t.n[2])};
+    // plain: -(x - y).n_test = q0 + t1 b1 + t2 b2 of the trial barycentrics
+    [[maybe_unused]] double q0 = 0, t1 = 0, t2 = 0;
+    if constexpr (!Mixed) {
+        q0 = -(d0[0] * t.n[0] + d0[1] * t.n[1] + d0[2] * t.n[2]);
+        t1 = s.e1[0] * t.n[0] + s.e1[1] * t.n[1] + s.e1[2] * t.n[2];
+        t2 = s.e2[0] * t.n[0] + s.e2[1] * t.n[1] + s.e2[2] * t.n[2];
+    }
+    [[maybe_unused]] DistanceCheck distance;
     for (uint32_t q = 0; q < job.patchCount; ++q) {
         const Patch &patch = patches[job.firstPatch + q];
         const int n = patch.degree == 14 ? 64 : 16;
         const int ro = patch.degree == 14 ? 34 : 18;  // rule offsets of the 16- and 64-point bins
         // mapped rule points of this patch (test from patch.test, trial from patch.trial)
         for (int idx = lane; idx < n; idx += 32) {
-            double by[3];
+            double by[3], e[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 sB[warp][idx][i] = cRule[4 * (ro + idx)] * patch.test[i] + cRule[4 * (ro + idx) + 1] * patch.test[3 + i] +
                                    cRule[4 * (ro + idx) + 2] * patch.test[6 + i];
                 by[i] = cRule[4 * (ro + idx)] * patch.trial[i] + cRule[4 * (ro + idx) + 1] * patch.trial[3 + i] +
                         cRule[4 * (ro + idx) + 2] * patch.trial[6 + i];
-                sY[warp][idx][i] = by[i];
             }
             // the trial point's offset from the trial panel's first vertex, once per patch point
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                sE[warp][idx][c] = s.e1[c] * by[1] + s.e2[c] * by[2];
+                e[c] = s.e1[c] * by[1] + s.e2[c] * by[2];
+            sE[warp][idx][0] = make_double2(e[0], e[1]);
+            sE[warp][idx][1] = make_double2(e[2], 0);
+            if constexpr (Mixed)
+                sY[warp][idx][0] = make_float4(float(by[0]), float(by[1]), float(by[2]), 0.f);
+            else {
+                sY[warp][idx][0] = make_double2(by[1], by[2]);
+                sY[warp][idx][1] = make_double2(by[1] * by[1], by[1] * by[2]);
+                sY[warp][idx][2] = make_double2(by[2] * by[2], 0);
+            }
         }
         __syncwarp();
         const double wpatch = patch.areaFraction * w4;
@@ -1266,30 +1271,89 @@ __global__ void __launch_bounds__(64, Mixed ? 10 : 1) nearWarpKernel(const DPane
             const double Dz = d0[2] + (t.e1[2] * bt[1] + t.e2[2] * bt[2]);
             const double wx = cRule[4 * (ro + x) + 3] * wpatch;
             Acc S[18];
+            if constexpr (Mixed) {
 #pragma unroll
-            for (int c = 0; c < 18; ++c)
-                S[c] = 0;
-            for (int y = y0; y < y1; ++y) {
-                const double *bs = sY[warp][y], *ey = sE[warp][y];
-                const double dx = Dx - ey[0];
-                const double dy = Dy - ey[1];
-                const double dz = Dz - ey[2];
-                const double w = wx * cRule[4 * (ro + y) + 3];
-                Acc val[6];
-                if constexpr (Mixed) {
-                    const float ns[3] = {float(s.n[0]), float(s.n[1]), float(s.n[2])};
-                    const float nt[3] = {float(t.n[0]), float(t.n[1]), float(t.n[2])};
-                    mixedValues(dx, dy, dz, float(w), k, ns, nt, val, bad);
-                } else {
-                    plainValues(dx, dy, dz, w, k, t, s, val, bad);
+                for (int c = 0; c < 18; ++c)
+                    S[c] = 0;
+#pragma unroll 2
+                for (int y = y0; y < y1; ++y) {
+                    const float4 bs = sY[warp][y][0];
+                    const double2 e0 = sE[warp][y][0];
+                    const double dx = Dx - e0.x;
+                    const double dy = Dy - e0.y;
+                    const double dz = Dz - sE[warp][y][1].x;
+                    float val[6];
+                    mixedValues(dx, dy, dz, float(wx * cRule[4 * (ro + y) + 3]), k, nsF, ntF, val, bad);
+                    const float b[3] = {bs.x, bs.y, bs.z};
+#pragma unroll
+                    for (int kind = 0; kind < 3; ++kind)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            S[kind * 6 + 2 * j] += val[2 * kind] * b[j];
+                            S[kind * 6 + 2 * j + 1] += val[2 * kind + 1] * b[j];
+                        }
                 }
+            } else {
+                // moments of g against 1, b1, b2 and of u = g (1 + ikr) / r^2 up to second order, as in
+                // regularPairsKernel
+                double g[6], u[12];
 #pragma unroll
-                for (int kind = 0; kind < 3; ++kind)
+                for (int c = 0; c < 6; ++c)
+                    g[c] = 0;
 #pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        S[kind * 6 + 2 * j] += val[2 * kind] * Acc(bs[j]);
-                        S[kind * 6 + 2 * j + 1] += val[2 * kind + 1] * Acc(bs[j]);
-                    }
+                for (int c = 0; c < 12; ++c)
+                    u[c] = 0;
+#pragma unroll 2
+                for (int y = y0; y < y1; ++y) {
+                    const double2 e0 = sE[warp][y][0], b01 = sY[warp][y][0], b2nd = sY[warp][y][1];
+                    const double b1 = b01.x, b2 = b01.y, b22 = sY[warp][y][2].x;
+                    const double dx = Dx - e0.x, dy = Dy - e0.y, dz = Dz - sE[warp][y][1].x;
+                    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                    distance.add(r2);
+                    const double rinv = reciprocalRoot(r2);
+                    const double kr = k * (r2 * rinv);
+                    double sn, cs;
+                    sinCos(kr, sn, cs);
+                    const double sc = cRule[4 * (ro + y) + 3] * rinv;
+                    const double gr = cs * sc, gi = -sn * sc;
+                    const double rinv2 = rinv * rinv;
+                    const double ur = fma(-gi, kr, gr) * rinv2, ui = fma(gr, kr, gi) * rinv2;
+                    g[0] += gr;
+                    g[1] += gi;
+                    g[2] = fma(gr, b1, g[2]);
+                    g[3] = fma(gi, b1, g[3]);
+                    g[4] = fma(gr, b2, g[4]);
+                    g[5] = fma(gi, b2, g[5]);
+                    u[0] += ur;
+                    u[1] += ui;
+                    u[2] = fma(ur, b1, u[2]);
+                    u[3] = fma(ui, b1, u[3]);
+                    u[4] = fma(ur, b2, u[4]);
+                    u[5] = fma(ui, b2, u[5]);
+                    u[6] = fma(ur, b2nd.x, u[6]);
+                    u[7] = fma(ui, b2nd.x, u[7]);
+                    u[8] = fma(ur, b2nd.y, u[8]);
+                    u[9] = fma(ui, b2nd.y, u[9]);
+                    u[10] = fma(ur, b22, u[10]);
+                    u[11] = fma(ui, b22, u[11]);
+                }
+                // (x - y).n_trial is constant over the trial panel
+                const double ps = wx * (Dx * s.n[0] + Dy * s.n[1] + Dz * s.n[2]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    S[2 + c] = wx * g[2 + c];
+                    S[4 + c] = wx * g[4 + c];
+                    S[c] = wx * (g[c] - (g[2 + c] + g[4 + c]));
+                    S[8 + c] = ps * u[2 + c];
+                    S[10 + c] = ps * u[4 + c];
+                    S[6 + c] = ps * (u[c] - (u[2 + c] + u[4 + c]));
+                    const double m0 = fma(t2, u[4 + c], fma(t1, u[2 + c], q0 * u[c]));
+                    const double m1 = fma(t2, u[8 + c], fma(t1, u[6 + c], q0 * u[2 + c]));
+                    const double m2 = fma(t2, u[10 + c], fma(t1, u[8 + c], q0 * u[4 + c]));
+                    S[14 + c] = wx * m1;
+                    S[16 + c] = wx * m2;
+                    S[12 + c] = wx * (m0 - (m1 + m2));
+                }
             }
             if (n == 16) {
 #pragma unroll
@@ -1323,6 +1387,8 @@ __global__ void __launch_bounds__(64, Mixed ? 10 : 1) nearWarpKernel(const DPane
         sM[warp][kind * 18 + 2 * e] = own[0];
         sM[warp][kind * 18 + 2 * e + 1] = own[1];
     }
+    if constexpr (!Mixed)
+        bad = distance.bad();
     if (__any_sync(0xffffffffu, bad) && lane == 0)
         flagError(error, kErrDistance);
     __syncwarp();

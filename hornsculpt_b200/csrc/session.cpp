@@ -275,6 +275,26 @@ void Session::preparePlan(const hs_numerics &o, double maxK, const volatile int3
             projected = projected || plan_.patches[j.first + q].projection;
         (projected ? projectedPairs : nearPairs).push_back({j.test, j.trial, j.first, j.count});
     }
+    // Tensor pairs with the most patches first: a warp takes a pair, patch counts spread over three decades, and a
+    // long pair that starts last leaves the other SMs idle (a counting sort; equal counts keep the plan's order).
+    {
+        std::vector<uint32_t> start;
+        for (const auto &j : nearPairs) {
+            if (j.patchCount >= start.size())
+                start.resize(j.patchCount + 1, 0);
+            ++start[j.patchCount];
+        }
+        uint32_t at = 0;
+        for (size_t c = start.size(); c-- > 0;) {
+            const uint32_t n = start[c];
+            start[c] = at;
+            at += n;
+        }
+        std::vector<NearPairJob> sorted(nearPairs.size());
+        for (const auto &j : nearPairs)
+            sorted[start[j.patchCount]++] = j;
+        nearPairs = std::move(sorted);
+    }
     projectedPairCount_ = uint32_t(projectedPairs.size());
     nearPairs.insert(nearPairs.end(), projectedPairs.begin(), projectedPairs.end());
     if (!plan_.wholePanelDegrees.empty())
