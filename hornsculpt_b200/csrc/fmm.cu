@@ -2190,6 +2190,7 @@ FmmOperator::FmmOperator(const Space &space, const FmmTreeSettings &settings) : 
         }
         I.leafItemStart[l].push_back(uint32_t(I.items.size()) - I.itemBase[l]);
     }
+    I.itemBase[levels] = uint32_t(I.items.size());
     // translation plans with their polar and coaxial classes
     std::map<uint64_t, int> polar;
     const auto polarClass = [&](int64_t x, int64_t y, int64_t z) {
