@@ -1353,6 +1353,9 @@ __global__ void __launch_bounds__(256) l2pKernel(const FmmPanel *__restrict__ pa
 HS_HD size_t l2pTableSmem(int p) {
     return (6 * size_t(p + 1) * (p + 1) + 14 * size_t(p + 2) * (p + 3) / 2) * sizeof(double2);
 }
+HS_HD size_t l2pRhsTableSmem(int p) {
+    return (size_t(p + 1) * (p + 1) + 8 * size_t(p + 2) * (p + 3) / 2) * sizeof(double2);
+}
 __global__ void __launch_bounds__(256) l2pTableKernel(const FmmPanel *__restrict__ panels,
                                                       const uint32_t *__restrict__ leaves,
                                                       const uint32_t *__restrict__ itemStart,
@@ -1443,6 +1446,115 @@ __global__ void __launch_bounds__(256) l2pTableKernel(const FmmPanel *__restrict
     }
 }
 
+// Local coefficients (n, m) of the gradient of the field with coefficients Ls: d/dx, d/dy, d/dz.
+__device__ void gradientAt(const double2 *Ls, int p, int n, int m, double k, double2 (&grad)[3]) {
+    const double2 z1 = coefAt(Ls, p, n + 1, m), z0 = coefAt(Ls, p, n - 1, m);
+    const double a1 = coefA(n + 1, m), a0 = coefA(n, m);
+    const double2 dz = make_double2(z1.x * a1 - z0.x * a0, z1.y * a1 - z0.y * a0);
+    const double2 u1 = coefAt(Ls, p, n + 1, m - 1), u0 = coefAt(Ls, p, n - 1, m - 1);
+    const double bm = coefBm(n + 1, m - 1), bp = coefBp(n - 1, m - 1);
+    const double2 dp = make_double2(u1.x * bm + u0.x * bp, u1.y * bm + u0.y * bp);
+    const double2 v1 = coefAt(Ls, p, n + 1, m + 1), v0 = coefAt(Ls, p, n - 1, m + 1);
+    const double cm = coefCm(n + 1, m + 1), cp = coefCp(n - 1, m + 1);
+    const double2 dm = make_double2(-(v1.x * cm + v0.x * cp), -(v1.y * cm + v0.y * cp));
+    // dx = (d+ + d-) / 2, dy = -i (d+ - d-) / 2
+    grad[0] = make_double2(0.5 * k * (dp.x + dm.x), 0.5 * k * (dp.y + dm.y));
+    grad[1] = make_double2(0.5 * k * (dp.y - dm.y), -0.5 * k * (dp.x - dm.x));
+    grad[2] = make_double2(k * dz.x, k * dz.y);
+}
+
+// l2pRhsKernel from the point tables, in the form of l2pTableKernel: the sums
+// over +-m of S and its gradient once per leaf, a warp per item, one warp sum.
+// It was the one leaf pass left that evaluated its points. 8k-triangle horn at
+// 2 kHz: a right-hand side 5.4 -> 2.6 ms.
+__global__ void __launch_bounds__(256) l2pRhsTableKernel(const FmmPanel *__restrict__ panels,
+                                                         const uint32_t *__restrict__ leaves,
+                                                         const uint32_t *__restrict__ itemStart,
+                                                         const FmmItem *__restrict__ items,
+                                                         const uint64_t *__restrict__ coefOffset, int p, double k,
+                                                         const double2 *__restrict__ table,
+                                                         const double2 *__restrict__ Lcoef, double2 *far,
+                                                         const float2 *__restrict__ L32,
+                                                         const double *__restrict__ sigma,
+                                                         const double *__restrict__ rule, int rulePts) {
+    extern __shared__ double smem[];
+    const int nc = (p + 1) * (p + 1), used = (p + 1) * (p + 2) / 2, entries = (p + 2) * (p + 3) / 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2 *Ls = reinterpret_cast<double2 *>(smem);  // [nc]
+    double2 *UV = Ls + nc;                            // [S, d/dx, d/dy, d/dz][entry][2]
+    loadLocals(Lcoef, L32, sigma, coefOffset[leaves[blockIdx.x]], 1, nc, Ls);
+    __syncthreads();
+    for (int e = threadIdx.x; e < entries; e += blockDim.x) {
+        int n, m;
+        decodeTri(e, n, m);
+        const double sign = m & 1 ? -1.0 : 1.0;
+        double2 a[4], b[4], grad[3];
+        a[0] = coefAt(Ls, p, n, m);
+        b[0] = coefAt(Ls, p, n, -m);
+        gradientAt(Ls, p, n, m, k, grad);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            a[1 + d] = grad[d];
+        gradientAt(Ls, p, n, -m, k, grad);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            b[1 + d] = grad[d];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double2 v = m ? make_double2(sign * b[c].x, sign * b[c].y) : make_double2(0, 0);
+            UV[2 * (c * entries + e)] = make_double2(a[c].x + v.x, a[c].y + v.y);
+            UV[2 * (c * entries + e) + 1] = m ? make_double2(v.y - a[c].y, a[c].x - v.x) : make_double2(0, 0);
+        }
+    }
+    __syncthreads();
+    const uint32_t i0 = itemStart[blockIdx.x], i1 = itemStart[blockIdx.x + 1];
+    for (uint32_t it = i0 + blockIdx.y * kWarps + warp; it < i1; it += gridDim.y * kWarps) {
+        const FmmItem item = items[it];
+        const FmmPanel &Pn = panels[item.panel];
+        double acc[6] = {0, 0, 0, 0, 0, 0};
+        for (int q = 0; q < rulePts; ++q) {
+            const double2 *row = table + (size_t(it) * rulePts + q) * entries;
+            double2 f[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                f[c] = make_double2(0, 0);
+            for (int e = lane; e < entries; e += 32) {
+                const double2 R = row[e];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (c == 0 && e >= used)
+                        continue;
+                    const double2 U = UV[2 * (c * entries + e)], V = UV[2 * (c * entries + e) + 1];
+                    f[c].x = fma(R.x, U.x, fma(R.y, V.x, f[c].x));
+                    f[c].y = fma(R.x, U.y, fma(R.y, V.y, f[c].y));
+                }
+            }
+            // fields F = -i k f; -S + (i / k) n . grad S
+            double vx = -k * f[0].y, vy = k * f[0].x;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                vx += Pn.n[d] * f[1 + d].x;
+                vy += Pn.n[d] * f[1 + d].y;
+            }
+            const double w = rule[4 * q + 3] * Pn.area;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                acc[2 * a] += w * rule[4 * q + a] * vx;
+                acc[2 * a + 1] += w * rule[4 * q + a] * vy;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+                acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (lane == 0)
+            for (int a = 0; a < 3; ++a)
+                if ((item.mask >> a) & 1)
+                    far[item.inc[a]] = make_double2(acc[2 * a], acc[2 * a + 1]);
+    }
+}
+
 // L2P of the right-hand-side field S (channel 0): forms grad S (degree p + 1)
 // in shared memory, then one warp per item writes
 //   far[inc_a] = sum_q w phi_a (-S + (i / k) n . grad S)
@@ -1468,19 +1580,11 @@ __global__ void __launch_bounds__(256) l2pRhsKernel(const FmmPanel *__restrict__
     for (int kk = threadIdx.x; kk < nd; kk += blockDim.x) {
         int n, m;
         decode(kk, n, m);
-        const double2 z1 = coefAt(Ls, p, n + 1, m), z0 = coefAt(Ls, p, n - 1, m);
-        const double a1 = coefA(n + 1, m), a0 = coefA(n, m);
-        const double2 dz = make_double2(z1.x * a1 - z0.x * a0, z1.y * a1 - z0.y * a0);
-        const double2 u1 = coefAt(Ls, p, n + 1, m - 1), u0 = coefAt(Ls, p, n - 1, m - 1);
-        const double bm = coefBm(n + 1, m - 1), bp = coefBp(n - 1, m - 1);
-        const double2 dp = make_double2(u1.x * bm + u0.x * bp, u1.y * bm + u0.y * bp);
-        const double2 v1 = coefAt(Ls, p, n + 1, m + 1), v0 = coefAt(Ls, p, n - 1, m + 1);
-        const double cm = coefCm(n + 1, m + 1), cp = coefCp(n - 1, m + 1);
-        const double2 dm = make_double2(-(v1.x * cm + v0.x * cp), -(v1.y * cm + v0.y * cp));
-        // dx = (d+ + d-) / 2, dy = -i (d+ - d-) / 2
-        Lg[kk] = make_double2(0.5 * k * (dp.x + dm.x), 0.5 * k * (dp.y + dm.y));
-        Lg[nd + kk] = make_double2(0.5 * k * (dp.y - dm.y), -0.5 * k * (dp.x - dm.x));
-        Lg[2 * nd + kk] = make_double2(k * dz.x, k * dz.y);
+        double2 grad[3];
+        gradientAt(Ls, p, n, m, k, grad);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            Lg[d * nd + kk] = grad[d];
     }
     __syncthreads();
     const uint32_t i0 = itemStart[blockIdx.x], i1 = itemStart[blockIdx.x + 1];
@@ -3085,13 +3189,13 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             if (!leaves)
                 continue;
             const int p = I.order[l], P = p + 1;
-            if (const double2 *table = rhs ? nullptr : I.table(l)) {
-                const size_t sm = l2pTableSmem(p);
-                fmmCheck(cudaFuncSetAttribute(l2pTableKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                         "l2p smem");
+            if (const double2 *table = I.table(l)) {
+                const auto kernel = rhs ? l2pRhsTableKernel : l2pTableKernel;
+                const size_t sm = rhs ? l2pRhsTableSmem(p) : l2pTableSmem(p);
+                fmmCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)), "l2p smem");
                 // few leaves: their items over several CTAs
                 const unsigned split = std::clamp(2u * unsigned(smCount()) / leaves, 1u, 8u);
-                l2pTableKernel<<<dim3(leaves, split), 256, sm, stream>>>(
+                kernel<<<dim3(leaves, split), 256, sm, stream>>>(
                     I.panels.as<FmmPanel>(), I.dLeaves[l].as<uint32_t>(), I.dLeafStart[l].as<uint32_t>(),
                     I.dItems.as<FmmItem>() + I.itemBase[l], I.coefOffset.as<uint64_t>(), p, k_, table,
                     I.Lc.as<double2>(), I.far.as<double2>(), I.fp32 ? I.Lc32.as<float2>() : nullptr, I.levelSigma(l),
