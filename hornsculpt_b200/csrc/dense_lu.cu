@@ -4,10 +4,11 @@
 // (the reference factors in FP32 with cuSOLVER getrf/getrs).
 //
 // Matrices are column-major N x N complex (interleaved reals), one per
-// frequency of the batch (blockIdx.y / blockIdx.z). Right-looking blocked LU
-// with panel width 32: a single-CTA panel factorisation per matrix, row
-// interchanges outside the panel, a unit-lower triangular solve for the U
-// block row and a shared-memory tiled complex GEMM for the trailing update.
+// frequency of the batch (blockIdx.y / blockIdx.z). Right-looking blocked LU in
+// two levels: 32-wide panels in the registers of a thread-block cluster update
+// the rest of their outer block, whose U rows are then solved at once and the
+// trailing matrix updated once, in FP64 by the FP64 matrix instruction, in FP32
+// by the tensor cores (3xTF32).
 #include "device_once.hpp"
 #include "device_types.cuh"
 #include "kernel_timer.hpp"
@@ -1465,7 +1466,8 @@ __global__ void __launch_bounds__(kTrsmThreads, 1) trsmBlockKernel(R *LU, uint32
 // sub-block is next. Measured per solve against shuffled sub-blocks loaded when
 // their turn came (one CTA per system up to N = 1024): FP32 N = 6380 3.2 -> 1.0
 // ms, N = 4023 x 3 2.1 -> 0.65, N = 642 x 32 0.25 -> 0.125; FP64 N = 6380
-// 4.2 -> 1.7, N = 2562 x 2 1.7 -> 0.71, N = 258 0.117 -> 0.073.
+// 4.2 -> 1.7, N = 2562 x 2 1.7 -> 0.71, N = 258 0.117 -> 0.073 (before the
+// steps overlapped, see triStepKernel).
 constexpr uint32_t kTriBlock = 128, kSub = 32;
 constexpr uint32_t kTriThreads = 512;                  // 128 rows x 4 column groups
 constexpr uint32_t kTriGroups = kTriThreads / kTriBlock;

@@ -3,7 +3,8 @@
 // adaptive quartering of panels within two edge lengths of the observer,
 // or the asymptotic far field F(d) exp(-ikR)/R. FP64 throughout; one CTA
 // per (frequency, excitation, observer, 256-panel tile), reduced over tiles
-// in a fixed order.
+// in a fixed order. Requests of 32 directions and more share each panel's data
+// among a CTA's directions (farFieldKernel).
 #include "device_once.hpp"
 #include "device_types.cuh"
 #include "green_math.cuh"
