@@ -2079,10 +2079,8 @@ template <class R> void solve(const R *LU, const int *pivots, uint32_t N, uint32
 // What the solves need of a factorisation: the composed permutations and, in FP32, the inverted diagonal blocks.
 template <class R> void prepareSolves(const R *LU, int *pivots, uint32_t N, uint32_t B, cudaStream_t stream) {
     const size_t smem = 2 * size_t(N) * sizeof(int);
-    static PerDeviceHighWater attr;
-    if (smem > 48 * 1024 && attr.raise(smem))
-        check(cudaFuncSetAttribute(permutationKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)),
-              "permutation smem attribute");
+    if (smem > 48 * 1024)  // one kernel for both precisions, so one limit
+        allowSharedMemory(reinterpret_cast<const void *>(permutationKernel));
     permutationKernel<<<B, 256, smem, stream>>>(pivots, N, pivots + size_t(B) * N);
     if constexpr (sizeof(R) == 4)
         diagonalInverseKernel<R><<<dim3((N + kSub - 1) / kSub, B, 2), 32, 0, stream>>>(LU, N, pivots, B);

@@ -7,8 +7,10 @@
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 namespace hsb {
 
@@ -61,24 +63,29 @@ template <class V> class PerDeviceValue {
     V value_[256] = {};
 };
 
-// Largest dynamic shared-memory opt-in already applied to one kernel on each
-// device: raise() returns true when `bytes` exceeds it (the caller then sets
-// the kernel attribute) and records the new value.
-class PerDeviceHighWater {
-  public:
-    bool raise(size_t bytes) {
-        const int device = currentDevice();
-        std::lock_guard<std::mutex> lock(mutex_);
-        if (bytes <= level_[device])
-            return false;
-        level_[device] = bytes;
-        return true;
-    }
-
-  private:
-    std::mutex mutex_;
-    size_t level_[256] = {};
-};
+// Lets `kernel` take the dynamic shared memory the device offers beyond the
+// default 48 KB. The limit belongs to the kernel function, so every session,
+// thread and launch size shares it: it is raised once per device, to all the
+// device can give, and never set to the need of one launch, which another
+// launch may exceed.
+inline void allowSharedMemory(const void *kernel) {
+    static std::mutex mutex;
+    static std::set<std::pair<int, const void *>> allowed;
+    const int device = currentDevice();
+    std::lock_guard<std::mutex> lock(mutex);
+    if (allowed.count({device, kernel}))
+        return;
+    cudaFuncAttributes own{};
+    int most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&own, kernel);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(own.sharedSizeBytes));
+    if (e != cudaSuccess)
+        throw std::runtime_error(std::string("CUDA shared memory limit: ") + cudaGetErrorString(e));
+    allowed.emplace(device, kernel);
+}
 
 // Multiprocessors of the current device.
 inline int smCount() {
