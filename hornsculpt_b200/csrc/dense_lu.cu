@@ -2080,7 +2080,7 @@ template <class R> void solve(const R *LU, const int *pivots, uint32_t N, uint32
 template <class R> void prepareSolves(const R *LU, int *pivots, uint32_t N, uint32_t B, cudaStream_t stream) {
     const size_t smem = 2 * size_t(N) * sizeof(int);
     if (smem > 48 * 1024)  // one kernel for both precisions, so one limit
-        allowSharedMemory(reinterpret_cast<const void *>(permutationKernel));
+        allowSharedMemory(permutationKernel);
     permutationKernel<<<B, 256, smem, stream>>>(pivots, N, pivots + size_t(B) * N);
     if constexpr (sizeof(R) == 4)
         diagonalInverseKernel<R><<<dim3((N + kSub - 1) / kSub, B, 2), 32, 0, stream>>>(LU, N, pivots, B);

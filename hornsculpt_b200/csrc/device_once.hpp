@@ -86,6 +86,9 @@ inline void allowSharedMemory(const void *kernel) {
         throw std::runtime_error(std::string("CUDA shared memory limit: ") + cudaGetErrorString(e));
     allowed.emplace(device, kernel);
 }
+template <class... P> void allowSharedMemory(void (*kernel)(P...)) {
+    allowSharedMemory(reinterpret_cast<const void *>(kernel));
+}
 
 // Multiprocessors of the current device.
 inline int smCount() {

@@ -2910,8 +2910,7 @@ void FmmOperator::buildPointTables(cudaStream_t stream) {
         const int D = I.order[l] + 1;
         const uint32_t points = (I.itemBase[l + 1] - I.itemBase[l]) * uint32_t(I.rulePts);
         const size_t sm = (size_t(D + 1) * (D + 2) + size_t(D + 1) * kTableThreads) * sizeof(double);
-        fmmCheck(cudaFuncSetAttribute(pointTableKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                 "point table smem");
+        allowSharedMemory(pointTableKernel);
         pointTableKernel<<<(points + kTableThreads - 1) / kTableThreads, kTableThreads, sm, stream>>>(
             I.panels.as<FmmPanel>(), I.itemLeaf.as<uint32_t>() + I.itemBase[l], I.dItems.as<FmmItem>() + I.itemBase[l],
             points, I.centers.as<double>(), D, k_, I.rule.as<double>(), I.rulePts,
@@ -2979,8 +2978,8 @@ void FmmOperator::planeWaveM2L(int l, int nch, cudaStream_t stream) {
     const size_t sm = (size_t(nc) + size_t(mw) * kHfRows + h.nph) * 16;
     if (sm > kMaxShared)
         throw Unsupported("Fast-multipole plane-wave order exceeds the shared-memory tables; refine the tree.");
-    fmmCheck(cudaFuncSetAttribute(signatureKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)), "signature smem");
-    fmmCheck(cudaFuncSetAttribute(projectKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)), "project smem");
+    allowSharedMemory(signatureKernel);
+    allowSharedMemory(projectKernel);
     const uint32_t nodes = uint32_t(I.levelNodes[l].size()), outs = I.dm2l[l].count;
     signatureKernel<<<dim3(nodes, nch), 256, sm, stream>>>(I.Mc.as<double2>(), I.coefOffset.as<uint64_t>(),
                                                            h.ids.as<uint32_t>(), p, h.theta.as<double>(), h.nth, h.nph,
@@ -3047,8 +3046,7 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
         }
         const dim3 grid(d.count * K, groups);
         const auto launch = [&](auto kernel) {
-            fmmCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                     "translate smem");
+            allowSharedMemory(kernel);
             kernel<<<grid, 256, sm, stream>>>(d.out.as<uint32_t>(), d.start.as<uint32_t>(), d.links.as<TransLink>(),
                                               pin, pout, in, out, I.coefOffset.as<uint64_t>(), wig,
                                               I.wignerStart.as<uint64_t>(), cx, I.coaxStart.as<uint64_t>(),
@@ -3092,8 +3090,7 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             const size_t sm = (kWarps * td) * 8 + kWarps * 6 * 16;
             if (sm > kMaxShared)
                 throw Unsupported("Fast-multipole leaf order exceeds the shared-memory tables; refine the tree.");
-            fmmCheck(cudaFuncSetAttribute(p2mKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                     "p2m smem");
+            allowSharedMemory(p2mKernel);
             p2mKernel<<<leaves, 256, sm, stream>>>(I.panels.as<FmmPanel>(), I.dLeaves[l].as<uint32_t>(),
                                                    I.dLeafStart[l].as<uint32_t>(), I.dItems.as<FmmItem>() + I.itemBase[l],
                                                    I.centers.as<double>(), I.coefOffset.as<uint64_t>(), P, k_, pv,
@@ -3133,8 +3130,7 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             if (matrix) {
                 const size_t sm = matrixSmem(p, gp.g[mode] * nch, gp.g[mode]);
                 const auto kernel = p <= kSmallOrder ? m2lMatrixKernel<kSmallRows> : m2lMatrixKernel<kMatrixRows>;
-                fmmCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                         "matrix m2l smem");
+                allowSharedMemory(kernel);
                 kernel<<<gp.chunkCount[mode], p <= kSmallOrder ? 384 : 256, sm, stream>>>(
                     gp.chunks[mode].as<uint2>(), gp.sorted.as<uint32_t>(), I.dm2l[l].links.as<TransLink>(), p, nch,
                     gp.g[mode], in, I.coefOffset.as<uint64_t>(), I.wignerPacked.as<double>(),
@@ -3144,8 +3140,7 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
         }
         if (!matrix) {
             const size_t sm = groupSmemBytes(p, gp.cpad[mode], gp.g[mode], sizeof(CT));
-            fmmCheck(cudaFuncSetAttribute(m2lGroupKernel<RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                     "grouped m2l smem");
+            allowSharedMemory(m2lGroupKernel<RT>);
             m2lGroupKernel<RT><<<gp.chunkCount[mode], 256, sm, stream>>>(
                 gp.chunks[mode].as<uint2>(), gp.sorted.as<uint32_t>(), I.dm2l[l].links.as<TransLink>(), p, nch,
                 gp.cpad[mode], gp.g[mode], in, I.coefOffset.as<uint64_t>(), wig, I.wignerStart.as<uint64_t>(), cx,
@@ -3192,7 +3187,7 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
             if (const double2 *table = I.table(l)) {
                 const auto kernel = rhs ? l2pRhsTableKernel : l2pTableKernel;
                 const size_t sm = rhs ? l2pRhsTableSmem(p) : l2pTableSmem(p);
-                fmmCheck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)), "l2p smem");
+                allowSharedMemory(kernel);
                 // few leaves: their items over several CTAs
                 const unsigned split = std::clamp(2u * unsigned(smCount()) / leaves, 1u, 8u);
                 kernel<<<dim3(leaves, split), 256, sm, stream>>>(
@@ -3215,16 +3210,14 @@ void FmmOperator::launchApply(const double *src, bool rhs, double *y, cudaStream
                 I.l2pScratch.ensure(size_t(leaves) * coefBytes);
             double2 *scratch = spill ? I.l2pScratch.as<double2>() : nullptr;
             if (rhs) {
-                fmmCheck(cudaFuncSetAttribute(l2pRhsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                         "l2p smem");
+                allowSharedMemory(l2pRhsKernel);
                 l2pRhsKernel<<<leaves, 256, sm, stream>>>(
                     I.panels.as<FmmPanel>(), I.dLeaves[l].as<uint32_t>(), I.dLeafStart[l].as<uint32_t>(),
                     I.dItems.as<FmmItem>() + I.itemBase[l], I.centers.as<double>(), I.coefOffset.as<uint64_t>(), p, k_,
                     I.Lc.as<double2>(), I.far.as<double2>(), I.fp32 ? I.Lc32.as<float2>() : nullptr,
                     I.levelSigma(l), I.rule.as<double>(), I.rulePts, scratch);
             } else {
-                fmmCheck(cudaFuncSetAttribute(l2pKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-                         "l2p smem");
+                allowSharedMemory(l2pKernel);
                 l2pKernel<<<leaves, 256, sm, stream>>>(I.panels.as<FmmPanel>(), I.dLeaves[l].as<uint32_t>(),
                                                        I.dLeafStart[l].as<uint32_t>(),
                                                        I.dItems.as<FmmItem>() + I.itemBase[l], I.centers.as<double>(),

@@ -3,6 +3,7 @@
 // cuda/support_fmm_solve.cu:401-525, without the finer-seed audit).
 #include "device_types.cuh"
 #include "fmm.hpp"
+#include "device_once.hpp"
 #include "kernel_timer.hpp"
 
 #include <algorithm>
@@ -374,8 +375,7 @@ void FmmSystem::factorBlocks(cudaStream_t stream, KernelTimer *timer) {
     TimedScope scope(timer, "fmm_block_jacobi", stream);
     sysCheck(cudaMemsetAsync(I.flag.p, 0, sizeof(int), stream), "flag reset");
     const size_t sm = size_t(kMaxBlock) * 2 * kMaxBlock * 16;
-    sysCheck(cudaFuncSetAttribute(blockInverseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)),
-             "block smem");
+    allowSharedMemory(blockInverseKernel);
     blockInverseKernel<<<I.blocks, 256, sm, stream>>>(I.blockStart.as<uint32_t>(), I.blockVerts.as<uint32_t>(),
                                                      I.rowStart.as<uint32_t>(), I.cols.as<uint32_t>(),
                                                      I.vals.as<double2>(), I.invStart.as<uint64_t>(),
