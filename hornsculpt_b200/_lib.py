@@ -140,6 +140,7 @@ def load():
         "hs_bem_debug_fmm_far": (C.c_int, [_P, C.POINTER(hs_numerics), C.c_double, C.c_double, _P, _P, _P, _P,
                                            C.c_size_t, C.POINTER(C.c_size_t), _P, C.c_size_t,
                                            C.POINTER(C.c_size_t)]),
+        "hs_bem_debug_fmm_tables": (C.c_int, [_P, C.c_uint64, C.c_int]),
         "hs_bem_debug_fmm_selftest": (C.c_int, [C.POINTER(C.c_double)]),
         "hs_bem_session_set_plane_wave_threshold": (C.c_int, [_P, C.c_double]),
         "hs_bem_session_set_fmm_grouped_m2l": (C.c_int, [_P, C.c_int]),

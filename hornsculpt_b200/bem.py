@@ -478,6 +478,12 @@ class CudaBemSolver:
                                                    b.ctypes.data))
         return _cplx(A).reshape(N, N).T, _cplx(b)  # column-major -> [row, col]
 
+    def debug_fmm_tables(self, limit: int | None = None, refused: bool = False) -> None:
+        """Device bytes of a fast-multipole operator's point tables (None: the default, 0: points on the
+        fly), or tables whose allocation fails."""
+        _lib.check(self._lib.hs_bem_debug_fmm_tables(self._handle, 2 ** 64 - 1 if limit is None else limit,
+                                                     1 if refused else 0))
+
     def debug_fmm_far(self, numerics: BemNumerics, k: float, tolerance: float, pressure: np.ndarray):
         """Far part of the fast-multipole operator applied to a P1 vector (row-equilibrated
         like debug_assemble), the near support-pair pattern as CSR (row_start, cols) and

@@ -668,6 +668,15 @@ hs_status hs_bem_session_fmm_audit_counts(const hs_bem_session *s, uint64_t *dir
     return HS_OK;
 }
 
+hs_status hs_bem_debug_fmm_tables(hs_bem_session *s, uint64_t bytes, int refused) {
+    if (!s)
+        return fail(HS_E_INVALID, "Session handle is null.");
+    return guarded([&]() {
+        std::lock_guard<std::mutex> lock(s->impl->mutex);
+        s->impl->setPointTables(size_t(bytes), refused != 0);
+    });
+}
+
 hs_status hs_bem_debug_fmm_selftest(double *error) {
     if (!error)
         return fail(HS_E_INVALID, "Self-test error pointer must be non-null.");

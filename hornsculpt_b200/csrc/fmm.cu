@@ -57,17 +57,24 @@ struct DevBuf {
             fmmCheck(cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, s), "upload");
     }
     void ensure(size_t n) {
+        if (!tryEnsure(n))
+            throw OutOfMemory("CUDA fast multipole workspace allocation failed.");
+    }
+    // The same without an exception: false, and an empty buffer, where the device has no room.
+    bool tryEnsure(size_t n) {
         if (n <= bytes)
-            return;
+            return true;
         if (p)
             fmmCheck(cudaFree(p), "free");
         p = nullptr;
         bytes = 0;
         if (cudaMalloc(&p, n) != cudaSuccess) {
+            cudaGetLastError();  // not the next launch's error
             p = nullptr;
-            throw OutOfMemory("CUDA fast multipole workspace allocation failed.");
+            return false;
         }
         bytes = n;
+        return true;
     }
 };
 template <class T> void uploadVec(DevBuf &b, const std::vector<T> &v, cudaStream_t s) {
@@ -2134,12 +2141,14 @@ struct FmmOperator::Impl {
     double tolerance = 1e-8;  // expansion tolerance of the last prepare()
     DevBuf rule, l2pScratch;
     // Point tables of the prepared wavenumber and the current panel rule (pointTableKernel), built by the
-    // first apply after prepare() or setPanelDegree() (never inside a capture: both drop the graphs, and
-    // the first apply after that launches directly).
+    // first apply after prepare() or setPanelDegree() (never inside a capture: run() launches directly
+    // while they are stale).
     DevBuf itemLeaf, pointTable;
     std::vector<uint64_t> tableStart;  // per level, entries
     std::vector<bool> tableLevel;      // the level reads its table
     bool tableStale = true;
+    size_t tableBytes = SIZE_MAX;  // setPointTables
+    bool tableRefused = false;
     const double2 *table(int l) const { return tableLevel[l] ? pointTable.as<double2>() + tableStart[l] : nullptr; }
     int rulePts = 0;
     unsigned panelDegree = 4;
@@ -2511,6 +2520,13 @@ void FmmOperator::setPanelDegree(unsigned degree, cudaStream_t stream) {
     I.dropGraphs();
 }
 
+void FmmOperator::setPointTables(size_t bytes, bool refused) {
+    impl_->tableBytes = bytes;
+    impl_->tableRefused = refused;
+    impl_->tableStale = true;
+    impl_->dropGraphs();
+}
+
 unsigned FmmOperator::panelDegree() const { return impl_->panelDegree; }
 
 void FmmOperator::setFp32(bool enabled) {
@@ -2880,17 +2896,17 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
 }
 
 // Point tables of every level whose L2P tables fit shared memory, when all of them fit a quarter of the
-// free memory (24 GB at most); otherwise the leaves evaluate their points on the fly.
+// free memory (24 GB at most); otherwise, or where the device has no room after all, the leaves evaluate their
+// points on the fly.
 void FmmOperator::buildPointTables(cudaStream_t stream) {
     Impl &I = *impl_;
-    I.tableStale = false;
     const int levels = int(tree_.levels.size());
     I.tableStart.assign(levels, 0);
     I.tableLevel.assign(levels, false);
     size_t freeBytes = 0, totalBytes = 0, total = 0;
     if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess)
         freeBytes = 0;
-    const size_t cap = std::min<size_t>(size_t(24) << 30, freeBytes / 4 + I.pointTable.bytes);
+    const size_t cap = std::min({I.tableBytes, size_t(24) << 30, freeBytes / 4 + I.pointTable.bytes});
     for (int l = I.lmin; l < levels; ++l) {
         const size_t points = size_t(I.itemBase[l + 1] - I.itemBase[l]) * I.rulePts;
         if (!points || points > 0x7fffffffu || l2pTableSmem(I.order[l]) > kMaxShared)
@@ -2899,11 +2915,11 @@ void FmmOperator::buildPointTables(cudaStream_t stream) {
         I.tableStart[l] = total;
         total += points * (size_t(I.order[l] + 2) * (I.order[l] + 3) / 2);
     }
-    if (total * sizeof(double2) > cap) {
+    if (total * sizeof(double2) > cap || I.tableRefused || !I.pointTable.tryEnsure(total * sizeof(double2))) {
         I.tableLevel.assign(levels, false);
+        I.tableStale = false;
         return;
     }
-    I.pointTable.ensure(total * sizeof(double2));
     for (int l = I.lmin; l < levels; ++l) {
         if (!I.tableLevel[l])
             continue;
@@ -2917,6 +2933,7 @@ void FmmOperator::buildPointTables(cudaStream_t stream) {
             I.pointTable.as<double2>() + I.tableStart[l]);
         fmmCheck(cudaGetLastError(), "point table launch");
     }
+    I.tableStale = false;  // only now: an exception above leaves them to the next apply
 }
 
 void FmmOperator::applyFar(const double *p, size_t stride, uint32_t S, double *y, cudaStream_t stream,
@@ -2936,9 +2953,11 @@ void FmmOperator::run(const double *src, bool rhs, double *y, cudaStream_t strea
     const bool capturable = stream != nullptr && stream != cudaStreamLegacy && stream != cudaStreamPerThread;
     // with kernel profiling on, plain launches keep every family's time
     const bool profiling = timer && timer->enabled();
-    if (!I.useGraphs || !capturable || profiling || tree_.ppFar.empty() ||
-        (!I.graph[mode] && I.applies[mode]++ == 0)) {
+    const bool graphs = I.useGraphs && capturable && !profiling && !tree_.ppFar.empty();
+    if (!graphs || (!I.graph[mode] && (I.applies[mode] == 0 || I.tableStale))) {
         launchApply(src, rhs, y, stream, timer);
+        if (graphs)
+            ++I.applies[mode];  // an apply that failed may have left buffers unsized: it does not count
         return;
     }
     const size_t inBytes = size_t(rhs ? I.T : I.N) * 16, outBytes = size_t(I.N) * 16;

@@ -75,6 +75,10 @@ class FmmOperator {
     // 4 -> 6 -> 8 -> 12 like the reference's compareQuadrature).
     void setPanelDegree(unsigned degree, cudaStream_t stream);
     unsigned panelDegree() const;
+    // Limit on the device bytes of the point tables (leaf levels without a table
+    // evaluate their points on the fly). `refused`: their allocation fails as on a
+    // full device (tests).
+    void setPointTables(size_t bytes, bool refused);
 
   private:
     struct Impl;

@@ -1408,6 +1408,15 @@ void Session::setPlanner(uint32_t planner) {
     planner_ = planner;
 }
 
+void Session::setPointTables(size_t bytes, bool refused) {
+    pointTableBytes_ = bytes;
+    pointTablesRefused_ = refused;
+    if (fmm_)
+        fmm_->setPointTables(bytes, refused);
+    if (fmmInner_)
+        fmmInner_->setPointTables(bytes, refused);
+}
+
 void Session::setGroupedM2l(bool enabled) {
     groupedM2l_ = enabled;
     if (fmm_)
@@ -1516,6 +1525,7 @@ FmmOperator &Session::fmmOperator(const hs_numerics &o, double tuneK, double tun
         fmm_->setGraphs(graphs_);
         fmm_->setHfThreshold(planeWaveThreshold_);
         fmm_->setGroupedM2l(groupedM2l_);
+        fmm_->setPointTables(pointTableBytes_, pointTablesRefused_);
         fmmSettings_ = st;
     }
     return *fmm_;
@@ -1584,6 +1594,7 @@ FmmOperator &Session::fmmInnerOperator(const hs_numerics &o) {
         fmmInner_->setFp32(true);
         fmmInner_->setGraphs(graphs_);
         fmmInner_->setGroupedM2l(groupedM2l_);
+        fmmInner_->setPointTables(pointTableBytes_, pointTablesRefused_);
         fmmInnerSettings_ = fmmSettings_;
     }
     (void)o;

@@ -94,6 +94,7 @@ class Session {
     void setGraphs(bool enabled);
     void setPlaneWaveThreshold(double threshold);
     void setGroupedM2l(bool enabled);
+    void setPointTables(size_t bytes, bool refused);
     // Interaction planner: on the device (default) or the host's threads;
     // both give the same plan bit for bit. The statistics are the last device
     // plan's.
@@ -148,6 +149,8 @@ class Session {
     bool graphs_ = true;
     double planeWaveThreshold_ = 8.0;
     bool groupedM2l_ = true;
+    size_t pointTableBytes_ = SIZE_MAX;
+    bool pointTablesRefused_ = false;
 
     MeshInput mesh_;
     V3 origin_{};

@@ -330,6 +330,12 @@ hs_status hs_bem_debug_fmm_far(hs_bem_session *session, const hs_numerics *numer
                                size_t near_capacity, size_t *near_count, uint32_t *level_info, size_t level_capacity,
                                size_t *level_count);
 hs_status hs_bem_debug_fmm_selftest(double *error);
+/* Point tables of the session's fast-multipole operators (the solid harmonics
+ * of the panels' quadrature points, one table per operator): at most `bytes` of
+ * device memory each; 0 evaluates every point on the fly, UINT64_MAX is the
+ * default. refused != 0 lets their allocation fail as on a full device. The
+ * operator is the same to rounding. */
+hs_status hs_bem_debug_fmm_tables(hs_bem_session *session, uint64_t bytes, int refused);
 /* Interaction planner of a session (makeInteractionPlan,
  * interaction_plan.cpp:156): HS_PLANNER_DEVICE (default) classifies the
  * panel pairs and runs the adaptive near-pair refinement on the session's
