@@ -60,14 +60,17 @@ struct DevBuf {
         if (!tryEnsure(n))
             throw OutOfMemory("CUDA fast multipole workspace allocation failed.");
     }
-    // The same without an exception: false, and an empty buffer, where the device has no room.
-    bool tryEnsure(size_t n) {
-        if (n <= bytes)
-            return true;
+    void release() {
         if (p)
             fmmCheck(cudaFree(p), "free");
         p = nullptr;
         bytes = 0;
+    }
+    // The same without an exception: false, and an empty buffer, where the device has no room.
+    bool tryEnsure(size_t n) {
+        if (n <= bytes)
+            return true;
+        release();
         if (cudaMalloc(&p, n) != cudaSuccess) {
             cudaGetLastError();  // not the next launch's error
             p = nullptr;
@@ -2525,7 +2528,11 @@ void FmmOperator::setPointTables(size_t bytes, bool refused) {
     impl_->tableRefused = refused;
     impl_->tableStale = true;
     impl_->dropGraphs();
+    if (impl_->pointTable.bytes > bytes)
+        impl_->pointTable.release();
 }
+
+size_t FmmOperator::pointTableBytes() const { return impl_->pointTable.bytes; }
 
 unsigned FmmOperator::panelDegree() const { return impl_->panelDegree; }
 
@@ -2895,31 +2902,27 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
     fmmCheck(cudaStreamSynchronize(stream), "prepare");
 }
 
-// Point tables of every level whose L2P tables fit shared memory, when all of them fit a quarter of the
-// free memory (24 GB at most); otherwise, or where the device has no room after all, the leaves evaluate their
-// points on the fly.
+// Point tables of the levels whose L2P tables fit shared memory, the deepest (with most of the leaves)
+// first, up to the limit on their bytes; the leaves of the other levels, or all where the device has no
+// room after all, evaluate their points on the fly.
 void FmmOperator::buildPointTables(cudaStream_t stream) {
     Impl &I = *impl_;
     const int levels = int(tree_.levels.size());
     I.tableStart.assign(levels, 0);
     I.tableLevel.assign(levels, false);
-    size_t freeBytes = 0, totalBytes = 0, total = 0;
-    if (cudaMemGetInfo(&freeBytes, &totalBytes) != cudaSuccess)
-        freeBytes = 0;
-    const size_t cap = std::min({I.tableBytes, size_t(24) << 30, freeBytes / 4 + I.pointTable.bytes});
-    for (int l = I.lmin; l < levels; ++l) {
+    const size_t limit = std::min(I.tableBytes, pointTableLimit(I.T)) / sizeof(double2);
+    size_t total = 0;
+    for (int l = levels - 1; l >= I.lmin; --l) {
         const size_t points = size_t(I.itemBase[l + 1] - I.itemBase[l]) * I.rulePts;
-        if (!points || points > 0x7fffffffu || l2pTableSmem(I.order[l]) > kMaxShared)
+        const size_t entries = points * (size_t(I.order[l] + 2) * (I.order[l] + 3) / 2);
+        if (!points || points > 0x7fffffffu || l2pTableSmem(I.order[l]) > kMaxShared || total + entries > limit)
             continue;
         I.tableLevel[l] = true;
         I.tableStart[l] = total;
-        total += points * (size_t(I.order[l] + 2) * (I.order[l] + 3) / 2);
+        total += entries;
     }
-    if (total * sizeof(double2) > cap || I.tableRefused || !I.pointTable.tryEnsure(total * sizeof(double2))) {
+    if (I.tableRefused || !I.pointTable.tryEnsure(total * sizeof(double2)))
         I.tableLevel.assign(levels, false);
-        I.tableStale = false;
-        return;
-    }
     for (int l = I.lmin; l < levels; ++l) {
         if (!I.tableLevel[l])
             continue;

@@ -15,6 +15,7 @@
 #include "host_mesh.hpp"
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <memory>
 #include <utility>
 #include <vector>
@@ -28,6 +29,16 @@ struct FmmLevelInfo {
     double radius;
     uint32_t planeWave;  // 1: M2L in the plane-wave (diagonal) form at this level
 };
+
+// Device bytes the point tables of one operator may take: a choice from the
+// mesh size alone, so that a solve's arithmetic does not depend on what else the
+// device holds. Leaf orders of 10 to 19 take 15 to 23 KB a triangle by the
+// six-point panel rule, twice that by the audit's twelve points and 125 KB by the
+// largest promoted rule; 8 GB leave room for the near field and the plan of the
+// largest meshes.
+inline size_t pointTableLimit(size_t triangles) {
+    return std::min(triangles * (size_t(128) << 10), size_t(8) << 30);
+}
 
 class FmmOperator {
   public:
@@ -75,10 +86,11 @@ class FmmOperator {
     // 4 -> 6 -> 8 -> 12 like the reference's compareQuadrature).
     void setPanelDegree(unsigned degree, cudaStream_t stream);
     unsigned panelDegree() const;
-    // Limit on the device bytes of the point tables (leaf levels without a table
-    // evaluate their points on the fly). `refused`: their allocation fails as on a
-    // full device (tests).
+    // Limit on the device bytes of the point tables, beside pointTableLimit (leaf
+    // levels without a table evaluate their points on the fly). `refused`: their
+    // allocation fails as on a full device (tests).
     void setPointTables(size_t bytes, bool refused);
+    size_t pointTableBytes() const;  // held now
 
   private:
     struct Impl;

@@ -151,8 +151,10 @@ std::unique_ptr<Result> Server::wait(uint64_t ticket, hs_serve_timing &timing) {
 }
 
 // Under the lock: the oldest queued request whose mesh is idle, with the
-// compatible queued requests on the same mesh, if its footprint fits.
-std::vector<std::shared_ptr<Server::Job>> Server::takeGroup(size_t &footprint) {
+// compatible queued requests on the same mesh, if its footprint fits. pointTables:
+// whether the footprint includes a fast-multipole solve's point tables, which it
+// does without where the budget has no room for them.
+std::vector<std::shared_ptr<Server::Job>> Server::takeGroup(size_t &footprint, bool &pointTables) {
     for (auto it = queue_.begin(); it != queue_.end(); ++it) {
         const auto &head = *it;
         auto s = sessions_.find(head->meshKey);
@@ -183,6 +185,10 @@ std::vector<std::shared_ptr<Server::Job>> Server::takeGroup(size_t &footprint) {
             B = (B + 1) / 2;
             need = solveFootprint(T, N, E, O, B, mixed, o.fmm_restart_length);
         }
+        const size_t tables = fmm ? fmmTableFootprint(T, mixed) : 0;
+        pointTables = tables && need + tables <= budget_;
+        if (pointTables)
+            need += tables;
         if (need > budget_) {
             // cannot run even alone: fail it here
             for (auto &job : group) {
@@ -194,7 +200,7 @@ std::vector<std::shared_ptr<Server::Job>> Server::takeGroup(size_t &footprint) {
             for (auto &job : group)
                 queue_.erase(std::find(queue_.begin(), queue_.end(), job));
             done_.notify_all();
-            return takeGroup(footprint);
+            return takeGroup(footprint, pointTables);
         }
         // other idle resident sessions hold memory too; the head's own session is covered by `need`
         if (reserved_ + idleBytes(head->meshKey) + need > budget_) {
@@ -258,12 +264,13 @@ void Server::worker(int index) {
     for (;;) {
         std::vector<std::shared_ptr<Job>> group;
         size_t footprint = 0;
+        bool pointTables = false;
         {
             std::unique_lock<std::mutex> lock(mutex_);
             work_.wait(lock, [&] {
                 if (stop_)
                     return true;
-                group = takeGroup(footprint);
+                group = takeGroup(footprint, pointTables);
                 return !group.empty();
             });
             if (stop_ && group.empty())
@@ -377,6 +384,8 @@ void Server::worker(int index) {
                     done_.notify_all();
             };
             std::lock_guard<std::mutex> solveLock(session->mutex);
+            if (head.request.base.numerics.acceleration == HS_FAST_MULTIPOLE)
+                session->setPointTables(pointTables ? SIZE_MAX : 0, false);
             merged = session->solve(r, nullptr, nullptr, nullptr, &hooks);
         } catch (...) {
             error = std::current_exception();

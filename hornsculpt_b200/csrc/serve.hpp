@@ -66,7 +66,7 @@ class Server {
         uint64_t lastUse = 0;
     };
     void worker(int index);
-    std::vector<std::shared_ptr<Job>> takeGroup(size_t &footprint);
+    std::vector<std::shared_ptr<Job>> takeGroup(size_t &footprint, bool &pointTables);
     size_t idleBytes(uint64_t keep) const;
     void evictIdle(size_t needed, uint64_t keep);
     bool evictOldestIdle(uint64_t keep);

@@ -388,16 +388,20 @@ size_t solveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t B, bo
 size_t fmmSolveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t restart) {
     // geometry and plan as for the dense form; near records and their pair
     // lists at about 700 near panel pairs per panel, near CSR values, GMRES
-    // basis, the expansion tables (a fixed allowance) and the point tables
+    // basis and the expansion tables (a fixed allowance)
     const size_t geometry = T * (200 + 48 + 112 + 16) + N * 24, plan = T * (T - 1) / 2 + T * 16 * 40 + T * 16 * 220;
     const size_t nearField = T * 700 * (kRecordDoubles * 8 + 4 + 8 + 8) + N * 500 * 20;
-    const size_t solve = size_t(E) * N * 16 * (restart + 12) + N * 6 * 1024 * 16 * 2 + T * (size_t(24) << 10);
+    const size_t solve = size_t(E) * N * 16 * (restart + 12) + N * 6 * 1024 * 16 * 2;
     const size_t fields = fieldPartialsBytes(uint32_t(T), E, O, 1) + size_t(E) * T * 16;
     return geometry + plan + nearField + solve + fields + (size_t(256) << 20);
 }
 
+size_t fmmTableFootprint(size_t T, bool mixed) {
+    return pointTableLimit(T) * (mixed ? 2 : 1);  // the mixed form's inner operator has its own
+}
+
 size_t Session::residentBytes() const {
-    size_t bytes = 0;
+    size_t bytes = (fmm_ ? fmm_->pointTableBytes() : 0) + (fmmInner_ ? fmmInner_->pointTableBytes() : 0);
     for (const DeviceBuffer *b : {&dPanels_, &dBounds_, &dMixedPanels_, &dIncOffsets_, &dIncPanel_, &dIncLocal_,
                                   &dRowScale_, &dMass_, &dPairCode_, &dTouching_, &dNearPairs_, &dPatches_, &dSingularTuples_,
                                   &dSingularTable_, &dRecords_, &dColumns_, &dPanelRhs_, &dBins_, &dBinCounts_, &dBinOffsets_, &dA_,
@@ -1409,6 +1413,8 @@ void Session::setPlanner(uint32_t planner) {
 }
 
 void Session::setPointTables(size_t bytes, bool refused) {
+    if (bytes == pointTableBytes_ && refused == pointTablesRefused_)
+        return;
     pointTableBytes_ = bytes;
     pointTablesRefused_ = refused;
     if (fmm_)

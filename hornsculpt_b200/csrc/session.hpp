@@ -222,5 +222,7 @@ private:
 size_t solveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t B, bool mixed, uint32_t restart);
 // The same for the fast-multipole form (one frequency at a time, sparse near field).
 size_t fmmSolveFootprint(size_t T, size_t N, uint32_t E, uint32_t O, uint32_t restart);
+// What its point tables may take on top (Session::setPointTables(0, false) does without).
+size_t fmmTableFootprint(size_t T, bool mixed);
 
 }  // namespace hsb
