@@ -18,6 +18,7 @@
 #include "green_math.cuh"
 #include "host_mesh.hpp"
 #include "kernel_timer.hpp"
+#include "near_tiles.cuh"
 
 #include <algorithm>
 #include <stdexcept>
@@ -2223,6 +2224,7 @@ __global__ void __launch_bounds__(kNearThreads) nearValuesKernel(
     for (uint32_t base = 0; base == 0 || base < length; base += kNearTile) {
         const uint32_t count = min(kNearTile, length - base);
         const bool last = base + count >= length;
+        const uint32_t previous = base ? map.col[list + base - 1] : 0;
         for (uint32_t p = threadIdx.x; p < count; p += kNearThreads) {
             const uint32_t s = map.col[list + base + p];
             double2 acc[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
@@ -2254,21 +2256,14 @@ __global__ void __launch_bounds__(kNearThreads) nearValuesKernel(
             double2 v = base ? vals[e] : make_double2(0, 0);
             for (uint32_t os = incOffsets[j]; os < incOffsets[j + 1]; ++os) {
                 const uint32_t s = incPanel[os];
-                uint32_t lo = 0, hi = count;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) / 2;
-                    if (trial[mid] < s)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                if (lo < count && trial[lo] == s) {
-                    escaped |= missing[lo] != 0;
-                    const double2 r = sums[incLocal[os] * kNearTile + lo];
+                const uint32_t at = nearTilePlace(trial, count, s);
+                if (at < count && trial[at] == s) {
+                    escaped |= missing[at] != 0;
+                    const double2 r = sums[incLocal[os] * kNearTile + at];
                     v.x += r.x;
                     v.y += r.y;
                 } else  // in another tile, or in none
-                    escaped |= (lo == 0 && base == 0) || (lo == count && last) || (lo > 0 && lo < count);
+                    escaped |= nearTileMisses(at, count, base == 0, last, previous, s);
             }
             if (last) {
                 for (uint32_t oa = o0; oa < o1; ++oa) {
