@@ -748,6 +748,7 @@ __global__ void __launch_bounds__(kClassifyThreads)
                 if (lane == unsigned(b))
                     mine = unsigned(__popc(m));
             }
+            __syncwarp();  // the warp's other lanes have read the places of the frequency before
             if (lane < kBins)
                 starts[warp * kBins + lane] = mine;
             __syncthreads();
