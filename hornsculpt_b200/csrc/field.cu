@@ -222,17 +222,40 @@ __global__ void __launch_bounds__(128) fieldKernel(FieldRequest req, const doubl
 }
 
 // Far field of many directions (balloons): a thread owns a direction and runs
-// over a tile's panels, whose geometry and sources it reads from shared memory
+// over a span of panels, whose geometry and sources it reads from shared memory
 // (the same address for the whole warp). The phase k d.(y - origin) is affine in
 // the trial barycentrics and does not depend on the excitation, so a rule point
 // costs its sine and cosine and six accumulations into the moments sum w e^(i phase)
 // (1, b1, b2); the excitations' pressures and fluxes meet the moments once per
-// panel. One CTA per 64 directions, 256-panel tile and frequency, excitations in
-// groups of kFarExcitations. With one CTA per output (fieldKernel) every panel's
-// data were read and every phase was formed again for each output and excitation:
-// 2664 directions x 2 excitations x 8 frequencies x 1280 triangles 9.3 -> 2.9 ms.
+// panel. One CTA per 64 directions, span and frequency, excitations in groups of
+// kFarExcitations. With one CTA per output (fieldKernel) every panel's
+// data were read and every phase was formed again for each output and excitation.
+//
+// A span is 256 panels, halved down to 8 until the CTAs of one frequency fill the
+// device: a thread's walk over 256 panels takes 0.5 to 1.6 ms (6 to 49 rule points)
+// however few directions there are. The batch does not count, here and in the
+// choice of the kernel: a result must not depend on what it is solved with.
+// Below 32 directions, or 384 outputs and tiles a frequency, fieldKernel is the
+// faster one (1280 triangles, one frequency, 37 directions of two excitations,
+// 370: 0.049 against 0.053 ms; 180 of one, 900: 0.084 against 0.059).
+// Field and sum, fieldKernel, always 256 panels, now:
+//   1280 triangles, 1 frequency,   180 directions x 1 excitation   0.084, 0.78, 0.059 ms
+//   1280 triangles, 8 frequencies, 180 directions x 1 excitation    0.32, 0.79, 0.15
+//   1280 triangles, 8 frequencies, 2664 directions x 2 excitations   7.9, 1.97, 1.60
+//   5120 triangles, 1 frequency,  2664 directions x 1 excitation    1.86, 0.81, 0.74
 constexpr int kFarThreads = 64, kFarChunk = 32, kFarExcitations = 2;
-constexpr uint32_t kFarDirections = 32;  // from this many directions on
+constexpr uint32_t kFarDirections = 32, kFarOutputTiles = 384, kFarSpanLeast = 8, kFarCtas = 8 * 148;
+// Whether a far field of one frequency goes to farFieldKernel, and its panels a span.
+bool sharesDirections(uint32_t T, uint32_t E, uint32_t O) {
+    return O >= kFarDirections && uint64_t(E) * O * ((T + kTile - 1) / kTile) >= kFarOutputTiles;
+}
+uint32_t farSpan(uint32_t T, uint32_t E, uint32_t O) {
+    const uint64_t columns = uint64_t((O + kFarThreads - 1) / kFarThreads) * ((E + kFarExcitations - 1) / kFarExcitations);
+    uint32_t span = kTile;
+    while (span > kFarSpanLeast && columns * ((T + span - 1) / span) < kFarCtas)
+        span /= 2;
+    return span;
+}
 
 struct FarPanel {
     double o[3], e1[3], e2[3], n[3];  // o: first vertex minus the far-field origin
@@ -256,10 +279,9 @@ __device__ __forceinline__ void farMoments(double phase, double p1, double p2, d
 }
 
 template <int RO, int RC>
-__device__ void farTile(const FieldRequest &req, uint32_t f, uint32_t e0, uint32_t count, uint32_t tile, double k,
+__device__ void farTile(const FieldRequest &req, uint32_t f, uint32_t e0, uint32_t count, uint32_t begin, uint32_t end, double k,
                         const double *pressure, const double *flux, const double (&x)[3], double (&v)[kFarExcitations][2],
                         bool &bad, FarPanel *panels, double (*source)[kFarExcitations][8]) {
-    const uint32_t begin = tile * kTile, end = min(begin + uint32_t(kTile), req.T);
     for (uint32_t base = begin; base < end; base += kFarChunk) {
         const uint32_t n = min(uint32_t(kFarChunk), end - base);
         __syncthreads();
@@ -317,14 +339,15 @@ __device__ void farTile(const FieldRequest &req, uint32_t f, uint32_t e0, uint32
 
 __global__ void __launch_bounds__(kFarThreads) farFieldKernel(FieldRequest req, const double *ks, const double *pressure,
                                                               const double *flux, const uint32_t *batchDegree,
-                                                              double *partials, int *error) {
+                                                              uint32_t span, double *partials, int *error) {
     __shared__ FarPanel panels[kFarChunk];
     __shared__ double source[kFarChunk][kFarExcitations][8];
-    const uint32_t tiles = (req.T + kTile - 1) / kTile, groups = (req.E + kFarExcitations - 1) / kFarExcitations;
-    const uint32_t tile = blockIdx.y % tiles, f = blockIdx.y / tiles / groups;
-    const uint32_t e0 = (blockIdx.y / tiles % groups) * kFarExcitations;
+    const uint32_t tiles = (req.T + span - 1) / span, groups = (req.E + kFarExcitations - 1) / kFarExcitations;
+    const uint32_t columns = (req.O + kFarThreads - 1) / kFarThreads, rest = blockIdx.x / columns;
+    const uint32_t tile = rest % tiles, begin = tile * span, end = min(begin + span, req.T), f = rest / tiles / groups;
+    const uint32_t e0 = (rest / tiles % groups) * kFarExcitations;
     const uint32_t count = min(uint32_t(kFarExcitations), req.E - e0);
-    const uint32_t o = blockIdx.x * kFarThreads + threadIdx.x;
+    const uint32_t o = blockIdx.x % columns * kFarThreads + threadIdx.x;
     const double k = ks[f];
     double x[3], v[kFarExcitations][2];
 #pragma unroll
@@ -335,11 +358,11 @@ __global__ void __launch_bounds__(kFarThreads) farFieldKernel(FieldRequest req, 
         v[e][0] = v[e][1] = 0;
     bool bad = false;
     switch (batchDegree[f]) {
-    case 4: farTile<0, 6>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
-    case 6: farTile<6, 12>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
-    case 8: farTile<18, 16>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
-    case 12: farTile<34, 49>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
-    default: farTile<83, 64>(req, f, e0, count, tile, k, pressure, flux, x, v, bad, panels, source); break;
+    case 4: farTile<0, 6>(req, f, e0, count, begin, end, k, pressure, flux, x, v, bad, panels, source); break;
+    case 6: farTile<6, 12>(req, f, e0, count, begin, end, k, pressure, flux, x, v, bad, panels, source); break;
+    case 8: farTile<18, 16>(req, f, e0, count, begin, end, k, pressure, flux, x, v, bad, panels, source); break;
+    case 12: farTile<34, 49>(req, f, e0, count, begin, end, k, pressure, flux, x, v, bad, panels, source); break;
+    default: farTile<83, 64>(req, f, e0, count, begin, end, k, pressure, flux, x, v, bad, panels, source); break;
     }
     if (bad)
         atomicExch(error, kErrDistance);
@@ -352,6 +375,32 @@ __global__ void __launch_bounds__(kFarThreads) farFieldKernel(FieldRequest req, 
         out[0] = (v[e][0] * cs + v[e][1] * sn) / req.farDistance;
         out[1] = (v[e][1] * cs - v[e][0] * sn) / req.farDistance;
     }
+}
+
+// The same for the spans of farFieldKernel, which can be hundreds: a warp per output.
+__global__ void finishSpansKernel(const double *partials, uint32_t spans, size_t outputs, double *out, int *error) {
+    const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    if (i >= outputs)
+        return;
+    const double2 *row = reinterpret_cast<const double2 *>(partials) + i * spans;
+    double r = 0, im = 0;
+#pragma unroll 4
+    for (uint32_t t = lane; t < spans; t += 32) {
+        const double2 v = row[t];
+        r += v.x;
+        im += v.y;
+    }
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+        r += __shfl_xor_sync(0xffffffffu, r, h);
+        im += __shfl_xor_sync(0xffffffffu, im, h);
+    }
+    if (lane != 0)
+        return;
+    if (!isfinite(r) || !isfinite(im))
+        atomicExch(error, kErrNonFinite);
+    reinterpret_cast<double2 *>(out)[i] = make_double2(r, im);
 }
 
 __global__ void finishKernel(const double *partials, uint32_t tiles, size_t outputs, double *out, int *error) {
@@ -646,30 +695,38 @@ void samplePressureField(const DPanel *panels, uint32_t T, const double *trace, 
 }
 
 size_t fieldPartialsBytes(uint32_t T, uint32_t E, uint32_t O, uint32_t B) {
-    return size_t(B) * E * O * ((T + kTile - 1) / kTile) * 2 * sizeof(double);
+    const uint32_t panels = sharesDirections(T, E, O) ? farSpan(T, E, O) : uint32_t(kTile);
+    return size_t(B) * E * O * ((T + panels - 1) / panels) * 2 * sizeof(double);
 }
 
 void evaluateFieldBatch(const FieldRequest &req, const double *ks, const double *pressure, const double *flux,
                         const uint32_t *batchDegree, double *partials, double *out, int *error, cudaStream_t stream,
                         KernelTimer *timer) {
     uploadFieldRules(stream);
-    const uint32_t tiles = (req.T + kTile - 1) / kTile;
+    uint32_t tiles = (req.T + kTile - 1) / kTile;
     const size_t outputs = size_t(req.B) * req.E * req.O;
     if (!outputs)
         return;
+    const bool shared = req.farField && sharesDirections(req.T, req.E, req.O);
     {
         TimedScope s(timer, "field", stream);
-        const uint64_t groups = uint64_t(req.B) * ((req.E + kFarExcitations - 1) / kFarExcitations) * tiles;
-        if (req.farField && req.O >= kFarDirections && groups <= 65535)
-            farFieldKernel<<<dim3((req.O + kFarThreads - 1) / kFarThreads, unsigned(groups)), kFarThreads, 0, stream>>>(
-                req, ks, pressure, flux, batchDegree, partials, error);
-        else
+        if (shared) {
+            const uint32_t span = farSpan(req.T, req.E, req.O);
+            tiles = (req.T + span - 1) / span;
+            const size_t ctas = size_t(req.B) * ((req.E + kFarExcitations - 1) / kFarExcitations) * tiles *
+                                ((req.O + kFarThreads - 1) / kFarThreads);
+            farFieldKernel<<<unsigned(ctas), kFarThreads, 0, stream>>>(req, ks, pressure, flux, batchDegree, span,
+                                                                       partials, error);
+        } else
             fieldKernel<<<unsigned(outputs * tiles), 128, 0, stream>>>(req, ks, pressure, flux, batchDegree, partials,
                                                                       error);
     }
     {
         TimedScope s(timer, "field_finish", stream);
-        finishKernel<<<unsigned((outputs + 127) / 128), 128, 0, stream>>>(partials, tiles, outputs, out, error);
+        if (shared)
+            finishSpansKernel<<<unsigned((outputs + 3) / 4), 128, 0, stream>>>(partials, tiles, outputs, out, error);
+        else
+            finishKernel<<<unsigned((outputs + 127) / 128), 128, 0, stream>>>(partials, tiles, outputs, out, error);
     }
     check(cudaGetLastError(), "field launch");
 }
