@@ -278,6 +278,21 @@ __device__ __forceinline__ void farMoments(double phase, double p1, double p2, d
     }
 }
 
+// The same for phases beyond sinCos: a far-field origin may lie anywhere.
+__device__ __noinline__ void farMomentsWide(int ro, int rc, double phase, double p1, double p2, double (&W)[6]) {
+    for (int s = 0; s < rc; ++s) {
+        const double *w = cField + 4 * (ro + s), *v = cFieldWeighted + 2 * (ro + s);
+        double sn, cs;
+        sincos(fma(p2, w[2], fma(p1, w[1], phase)), &sn, &cs);
+        W[0] = fma(cs, w[3], W[0]);
+        W[1] = fma(sn, w[3], W[1]);
+        W[2] = fma(cs, v[0], W[2]);
+        W[3] = fma(sn, v[0], W[3]);
+        W[4] = fma(cs, v[1], W[4]);
+        W[5] = fma(sn, v[1], W[5]);
+    }
+}
+
 template <int RO, int RC>
 __device__ void farTile(const FieldRequest &req, uint32_t f, uint32_t e0, uint32_t count, uint32_t begin, uint32_t end, double k,
                         const double *pressure, const double *flux, const double (&x)[3], double (&v)[kFarExcitations][2],
@@ -321,7 +336,10 @@ __device__ void farTile(const FieldRequest &req, uint32_t f, uint32_t e0, uint32
             const double nf = k * (x[0] * pn.n[0] + x[1] * pn.n[1] + x[2] * pn.n[2]);
             bad |= !isfinite(phase + (p1 + p2));
             double W[6] = {0, 0, 0, 0, 0, 0};
-            farMoments<RO, RC>(phase, p1, p2, W);
+            if (fabs(phase) + fabs(p1) + fabs(p2) < kSinCosLimit)
+                farMoments<RO, RC>(phase, p1, p2, W);
+            else
+                farMomentsWide(RO, RC, phase, p1, p2, W);
 #pragma unroll
             for (int e = 0; e < kFarExcitations; ++e) {
                 if (uint32_t(e) >= count)

@@ -3,8 +3,9 @@
 //
 // A sample spends most of its FP64 instructions here. The library's rsqrt and
 // sincos carry branches for denormal, infinite and very large arguments that
-// no sample meets (distances are checked by the caller, k*r stays far below
-// 2^31), and those branches keep the compiler from interleaving the samples of
+// no sample meets (distances are checked by the caller; k*r stays far below
+// kSinCosLimit between panels, whose areas are at least 1e-14 of the mesh's
+// extent squared, and pressure samples so far away do not converge), and those branches keep the compiler from interleaving the samples of
 // an unrolled loop. Both functions are within 1.5 units in the last place
 // (measured: root 0.99, sine 1.44, cosine 1.45 over 1e-12 .. 1e7), like the
 // library's.
@@ -24,11 +25,12 @@ __device__ __forceinline__ double reciprocalRoot(double x) {
     return fma(fma(e, 0.375, 0.5), e * y, y);
 }
 
-// sin(x) and cos(x) for |x| < 2^31: Cody-Waite reduction by pi/2 in two parts
+// sin(x) and cos(x) for |x| < kSinCosLimit: Cody-Waite reduction by pi/2 in two parts
 // (the first product is exact inside its fma, because the difference has no bit
 // below 2^-52 and is smaller than one), then minimax polynomials on
 // [-pi/4, pi/4] fitted with the Remez exchange in 60 digits: relative error
 // 3.5e-18 of sin(r)/r, absolute 4.7e-20 of cos(r).
+constexpr double kSinCosLimit = 0x1p31;
 __device__ __forceinline__ void sinCos(double x, double &sine, double &cosine) {
     constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
     const double shifted = fma(x, 0x1.45f306dc9c883p-1, kRound);
