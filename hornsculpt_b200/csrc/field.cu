@@ -513,7 +513,9 @@ struct SamplePanel {
     double dn, scale;            // (x - y).n, 2 area / (4 pi)
     double p[6];                 // pressure at the first vertex, differences to the others
     double q[2], qAbs;
+    bool wide;                   // k r may leave sinCos's range (Wide only)
 };
+template <bool Wide>
 __device__ __forceinline__ void patchIntegral(const SamplePanel &t, const SamplePatch &patch, double k, int offset,
                                               int count, double &re, double &im, double &mag) {
     re = im = mag = 0;
@@ -527,7 +529,10 @@ __device__ __forceinline__ void patchIntegral(const SamplePanel &t, const Sample
         const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
         const double rinv = reciprocalRoot(r2), rinv2 = rinv * rinv, kr = k * (r2 * rinv);
         double sn, cs;
-        sinCos(kr, sn, cs);
+        if (Wide && t.wide)
+            sincos(kr, &sn, &cs);
+        else
+            sinCos(kr, sn, cs);
         const double pr = fma(b2, t.p[4], fma(b1, t.p[2], t.p[0])), pi = fma(b2, t.p[5], fma(b1, t.p[3], t.p[1]));
         // e^(-ikr) (1 + ikr) (x - y).n / r^2 p - e^(-ikr) q, over r
         const double proj = t.dn * rinv2;
@@ -544,6 +549,9 @@ __device__ __forceinline__ void patchIntegral(const SamplePanel &t, const Sample
     mag *= s;
 }
 
+// Wide: some point is so far away that k r leaves sinCos's range; the panels that
+// are take the library's functions (the others the same as without).
+template <bool Wide>
 __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPanel *__restrict__ panels, uint32_t T,
                                                                      const double *__restrict__ trace,
                                                                      const double *__restrict__ flux,
@@ -591,6 +599,7 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
         SamplePanel sample;
         sample.scale = 2 * panel.area * kInvFourPi;
         const double d0[3] = {x.x - panel.v0[0], x.y - panel.v0[1], x.z - panel.v0[2]};
+        sample.wide = Wide && !(k * (fabs(d0[0]) + fabs(d0[1]) + fabs(d0[2]) + 2 * panel.maxEdge) < kSinCosLimit);
         sample.dn = d0[0] * panel.n[0] + d0[1] * panel.n[1] + d0[2] * panel.n[2];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -617,8 +626,8 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
         while (top > 0) {
             const SamplePatch patch = stack[--top];
             double cr, ci, cm, fr, fi, fm;
-            patchIntegral(sample, patch, k, 0, 6, cr, ci, cm);    // degree 4
-            patchIntegral(sample, patch, k, 18, 16, fr, fi, fm);  // degree 8
+            patchIntegral<Wide>(sample, patch, k, 0, 6, cr, ci, cm);    // degree 4
+            patchIntegral<Wide>(sample, patch, k, 18, 16, fr, fi, fm);  // degree 8
             const double span = k * panel.maxEdge * sqrt(patch.fraction);
             const double diff = sqrt((fr - cr) * (fr - cr) + (fi - ci) * (fi - ci));
             if (span <= 3.14159265358979323846 && diff <= tolerance * fmax(fm, 1e-300)) {
@@ -700,15 +709,16 @@ void uploadFieldRules(cudaStream_t stream) {
 }
 
 void samplePressureField(const DPanel *panels, uint32_t T, const double *trace, const double *flux,
-                         const double *points, uint32_t count, double k, double minDistance, double tolerance,
-                         uint32_t maxDepth, double *pressure, int32_t *status, cudaStream_t stream) {
+                         const double *points, uint32_t count, double farthest, double k, double minDistance,
+                         double tolerance, uint32_t maxDepth, double *pressure, int32_t *status, cudaStream_t stream) {
     if (maxDepth > 12)
         throw std::invalid_argument("Invalid pressure field settings.");
     uploadFieldRules(stream);
     if (!count)
         return;
-    pressureFieldKernel<<<count, kFieldThreads, 0, stream>>>(panels, T, trace, flux, points, k, minDistance, tolerance,
-                                                           maxDepth, pressure, status);
+    const auto kernel = k * farthest < kSinCosLimit ? pressureFieldKernel<false> : pressureFieldKernel<true>;
+    kernel<<<count, kFieldThreads, 0, stream>>>(panels, T, trace, flux, points, k, minDistance, tolerance, maxDepth,
+                                                pressure, status);
     check(cudaGetLastError(), "pressure field launch");
 }
 

@@ -3,9 +3,9 @@
 //
 // A sample spends most of its FP64 instructions here. The library's rsqrt and
 // sincos carry branches for denormal, infinite and very large arguments that
-// no sample meets (distances are checked by the caller; k*r stays far below
+// no sample meets (distances are checked by the caller, and k*r stays far below
 // kSinCosLimit between panels, whose areas are at least 1e-14 of the mesh's
-// extent squared, and pressure samples so far away do not converge), and those branches keep the compiler from interleaving the samples of
+// extent squared; observers may lie anywhere, so the fields check it), and those branches keep the compiler from interleaving the samples of
 // an unrolled loop. Both functions are within 1.5 units in the last place
 // (measured: root 0.99, sine 1.44, cosine 1.45 over 1e-12 .. 1e7), like the
 // library's.

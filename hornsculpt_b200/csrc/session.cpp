@@ -493,15 +493,19 @@ void Session::pressureField(double frequency, double soundSpeed, const double *t
     if (count > 0x7fffffffu)
         throw InvalidArgument("Too many pressure field points.");
     std::vector<double> local(3 * count);
+    double reach = 0, extent = 0;
     for (size_t i = 0; i < count; ++i) {
         if (!std::isfinite(points[3 * i]) || !std::isfinite(points[3 * i + 1]) || !std::isfinite(points[3 * i + 2]))
             throw InvalidArgument("Invalid pressure field point.");
         local[3 * i] = points[3 * i] - origin_.x;  // session coordinates are centred on vertex 0
         local[3 * i + 1] = points[3 * i + 1] - origin_.y;
         local[3 * i + 2] = points[3 * i + 2] - origin_.z;
+        reach = std::max(reach, std::fabs(local[3 * i]) + std::fabs(local[3 * i + 1]) + std::fabs(local[3 * i + 2]));
     }
     if (!count)
         return;
+    for (const V3 &v : space_.vertices)
+        extent = std::max(extent, std::fabs(v.x) + std::fabs(v.y) + std::fabs(v.z));
     const cudaStream_t s = stream();
     dSamplePoints_.ensure(local.size() * 8);
     dSampleTrace_.ensure(N * 16);
@@ -515,8 +519,8 @@ void Session::pressureField(double frequency, double soundSpeed, const double *t
          "derivative upload");
     const double k = 2 * M_PI * frequency / soundSpeed;
     samplePressureField(dPanels_.as<DPanel>(), uint32_t(T), dSampleTrace_.as<double>(), dSampleFlux_.as<double>(),
-                        dSamplePoints_.as<double>(), uint32_t(count), k, st.minimum_boundary_distance,
-                        st.relative_quadrature_tolerance, st.maximum_quadrature_depth, dSampleOut_.as<double>(),
+                        dSamplePoints_.as<double>(), uint32_t(count), reach + 5 * extent, k,
+                        st.minimum_boundary_distance, st.relative_quadrature_tolerance, st.maximum_quadrature_depth, dSampleOut_.as<double>(),
                         dSampleStatus_.as<int32_t>(), s);
     cuda(cudaMemcpyAsync(pressure, dSampleOut_.as<void>(), count * 16, cudaMemcpyDeviceToHost, s), "field download");
     cuda(cudaMemcpyAsync(status, dSampleStatus_.as<void>(), count * 4, cudaMemcpyDeviceToHost, s), "field download");
