@@ -507,10 +507,13 @@ struct SamplePatch {
 // D p - S q over one patch with one rule, and the magnitude sum |D p| + |S q|.
 // (x - y).n is constant over the panel, and the magnitudes follow from the
 // moduli: |S q| = |q| / (4 pi r), |D p| = |p| |(x - y).n| sqrt(1 + (k r)^2) / (4 pi r^3).
+// A panel's sources are taken in units of a power of two near their largest, so
+// that no square over- or underflows whatever the amplitude is.
 // With the short root and sine/cosine, 4096 points at 1280 triangles take 1.3 ms.
 struct SamplePanel {
     double v0[3], e1[3], e2[3];  // observer minus first vertex, edges
     double dn, scale;            // (x - y).n, 2 area / (4 pi)
+    double unit;                 // of p, q and the panel's integrals
     double p[6];                 // pressure at the first vertex, differences to the others
     double q[2], qAbs;
     bool wide;                   // k r may leave sinCos's range (Wide only)
@@ -607,19 +610,31 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
             sample.e1[i] = panel.e1[i];
             sample.e2[i] = panel.e2[i];
         }
-        bool silent = true;
+        double source[4][2], largest = 0;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            const double first = trace[2 * panel.nodes[0] + c], second = trace[2 * panel.nodes[1] + c],
-                         third = trace[2 * panel.nodes[2] + c];
-            sample.p[c] = first;
-            sample.p[2 + c] = second - first;
-            sample.p[4 + c] = third - first;
-            sample.q[c] = flux[2 * t + c];
-            silent = silent && first == 0 && second == 0 && third == 0 && sample.q[c] == 0;
+#pragma unroll
+            for (int v = 0; v < 3; ++v)
+                source[v][c] = trace[2 * panel.nodes[v] + c];
+            source[3][c] = flux[2 * t + c];
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                largest = fmax(largest, fabs(source[v][c]));
         }
-        if (silent)
+        if (largest == 0)
             continue;
+        // the largest's power of two, within what has a reciprocal
+        const int exponent = min(max(__double2hiint(largest) & 0x7ff00000, 0x00100000), 0x7fd00000);
+        const double inverse = __hiloint2double(0x7fe00000 - exponent, 0);
+        sample.unit = __hiloint2double(exponent, 0);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const double first = source[0][c] * inverse;
+            sample.p[c] = first;
+            sample.p[2 + c] = source[1][c] * inverse - first;
+            sample.p[4 + c] = source[2][c] * inverse - first;
+            sample.q[c] = source[3][c] * inverse;
+        }
         sample.qAbs = sqrt(sample.q[0] * sample.q[0] + sample.q[1] * sample.q[1]);
         int top = 0;
         stack[top++] = SamplePatch{{1, 0, 0, 0, 1, 0, 0, 0, 1}, 1.0, 0};
@@ -631,8 +646,8 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
             const double span = k * panel.maxEdge * sqrt(patch.fraction);
             const double diff = sqrt((fr - cr) * (fr - cr) + (fi - ci) * (fi - ci));
             if (span <= 3.14159265358979323846 && diff <= tolerance * fmax(fm, 1e-300)) {
-                re += fr;
-                im += fi;
+                re = fma(fr, sample.unit, re);
+                im = fma(fi, sample.unit, im);
                 continue;
             }
             if (patch.depth >= maxDepth) {
