@@ -896,14 +896,15 @@ constexpr size_t kMatrixShared = 112 * 1024;                 // two CTAs per SM
 
 // columns (doubles) of X for C complex columns, and its row stride: 4 or 12 modulo 16 keeps the fragment
 // reads free of bank conflicts
-__host__ __device__ inline int matrixColumns(int C) { return (2 * C + 7) / 8 * 8; }
-__host__ __device__ inline int matrixStride(int C) {
+__host__ __device__ constexpr int matrixColumns(int C) { return (2 * C + 7) / 8 * 8; }
+__host__ __device__ constexpr int matrixStride(int C) {
     const int n = matrixColumns(C);
     return n + 4;  // n is 0 or 8 modulo 16
 }
-__host__ __device__ inline size_t matrixSmem(int p, int C, int g) {
+__host__ __device__ constexpr size_t matrixSmem(int p, int C, int g) {
     return size_t(p + 1) * (p + 1) * matrixStride(C) * sizeof(double) + size_t(g) * (p + 1) * sizeof(double2);
 }
+static_assert(matrixSmem(kMatrixOrder, 6, 1) <= kMatrixShared, "a link of the largest order must fit");
 
 __device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -2869,8 +2870,6 @@ void FmmOperator::prepare(double k, double tolerance, cudaStream_t stream) {
                 for (int cand = 16; matrix && cand >= 1 && !g; --cand)
                     if (matrixSmem(p, cand * nch, cand) <= kMatrixShared)
                         g = cand;
-                if (matrix && !g)
-                    g = 1;  // one CTA per SM
                 for (int cand = 16; cand >= 1 && !g; --cand)
                     if (groupSmemBytes(p, (cand * nch) | 1, cand, cb) <= 110 * 1024) {
                         g = cand;
