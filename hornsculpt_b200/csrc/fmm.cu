@@ -296,10 +296,10 @@ __global__ void __launch_bounds__(256) p2mKernel(const FmmPanel *__restrict__ pa
 // twice (emission and testing), evaluating Bessel, Theta and azimuth factors
 // again each time. They are tabulated once after prepare() or setPanelDegree()
 // (row of a point: entries triIndex(n, m), degree p + 1) and read by every
-// apply: P2M 2.0 -> 0.23 ms and L2P 2.25 -> 0.45 ms for the 8k-triangle horn
-// (leaf orders 10 to 17; the tables take about 0.4 ms to build). A level whose
-// table or shared memory does not fit evaluates the points on the fly
-// (p2mKernel, l2pKernel).
+// apply: P2M 2.0 -> 0.23 ms and L2P 2.25 -> 0.33 ms for the 8k-triangle horn
+// (leaf orders 10 to 17; the tables take about 0.4 ms to build). A level beyond
+// the limit on the tables' bytes (pointTableLimit), or whose order does not fit
+// shared memory, evaluates the points on the fly (p2mKernel, l2pKernel).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void decodeTri(int e, int &n, int &m) {
     n = int((sqrtf(8.f * e + 1.f) - 1.f) * .5f);
