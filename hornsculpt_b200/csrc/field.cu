@@ -610,7 +610,8 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
             sample.e1[i] = panel.e1[i];
             sample.e2[i] = panel.e2[i];
         }
-        double source[4][2], largest = 0;
+        double source[4][2];
+        unsigned largest = 0, bits = 0;  // the largest's high word; whether anything is not zero
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
 #pragma unroll
@@ -618,13 +619,16 @@ __global__ void __launch_bounds__(kFieldThreads) pressureFieldKernel(const DPane
                 source[v][c] = trace[2 * panel.nodes[v] + c];
             source[3][c] = flux[2 * t + c];
 #pragma unroll
-            for (int v = 0; v < 4; ++v)
-                largest = fmax(largest, fabs(source[v][c]));
+            for (int v = 0; v < 4; ++v) {
+                const unsigned high = unsigned(__double2hiint(source[v][c])) & 0x7fffffffu;
+                largest = max(largest, high);
+                bits |= high | unsigned(__double2loint(source[v][c]));
+            }
         }
-        if (largest == 0)
+        if (bits == 0)
             continue;
         // the largest's power of two, within what has a reciprocal
-        const int exponent = min(max(__double2hiint(largest) & 0x7ff00000, 0x00100000), 0x7fd00000);
+        const int exponent = min(max(int(largest & 0x7ff00000u), 0x00100000), 0x7fd00000);
         const double inverse = __hiloint2double(0x7fe00000 - exponent, 0);
         sample.unit = __hiloint2double(exponent, 0);
 #pragma unroll
